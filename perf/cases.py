@@ -109,17 +109,16 @@ def _keep(case, make):
     return _kept[key]
 
 
-# Room for mesh vertices: a n + b n^(2/3), a volume (loose particles) and a
-# surface part; a program of this kind allots twice as many triangles.
-_ROOM = {"ball": (8, 60), "slab": (12, 30), "mixed": (2.5, 300), "dam": (3, 80), "sheets": (4, 200), "spray": (8, 40),
-         "two_radius": (1, 60)}
+# Room for mesh vertices of n particles: at most 60 a particle (loose ones),
+# else a surface part and one that grows with n; a program of this kind allots
+# twice as many triangles.
+_ROOM = {"ball": 6, "slab": 13, "mixed": 3, "dam": 4, "sheets": 6, "spray": 9, "two_radius": 3}
 
 
 def _room(shape, n):
     """Pinned host buffers for the mesh of n particles, filled up to the
     counts a pass returns."""
-    a, b = _ROOM[shape]
-    nv = int(a * n + b * n ** (2 / 3)) + 4096
+    nv = min(60 * n, 600000 + _ROOM[shape] * n)
     return {"verts": torch.zeros((nv, 3), dtype=torch.float32).pin_memory(),
             "tris": torch.zeros((int(2.1 * nv), 3), dtype=torch.int32).pin_memory()}
 
