@@ -441,7 +441,6 @@ int pi_ctx_create(int device, size_t budget_bytes, pi_ctx** out) {
   PI_CUDA(cudaEventCreateWithFlags(&c->ev_topo_read, cudaEventDisableTiming));
   PI_CUDA(cudaEventCreateWithFlags(&c->ev_qef_in, cudaEventDisableTiming));
   PI_CUDA(cudaEventCreateWithFlags(&c->ev_qef_done, cudaEventDisableTiming));
-  c->coop_blocks = top_levels_grid(device, c->smCount);
   PI_CUDA(cudaEventCreateWithFlags(&c->ev_tris_ready, cudaEventDisableTiming));
   PI_CUDA(cudaEventCreateWithFlags(&c->ev_tris_copied, cudaEventDisableTiming));
   PI_CUDA(cudaEventCreateWithFlags(&c->ev_read, cudaEventDisableTiming));

@@ -102,9 +102,6 @@ struct pi_ctx {
   // no budget (its device buffers and events carry over); freed with the
   // context
   pi_frame* recon = nullptr;
-  // grid of the cooperative coarse-level octree kernel (0: no cooperative
-  // launch on this device)
-  int coop_blocks = 0;
   // a second stream for device-to-host copies that overlap the compute
   // stream (pi_reconstruct's triangle download), and its two events
   cudaStream_t copy_stream = nullptr;
@@ -232,7 +229,7 @@ namespace pisurf {
 constexpr int kPinAniso = 0, kPinOctree = 1, kPinExtract = 2, kPinSlots = 3;
 constexpr int kPinValid = kPinSlots;  // bit of pin_pending for the valid-key count
 // after the slots: word 0 the valid-key count, word 1 the octree level's
-// INTERNAL count; then the coarse-level kernel's level starts and depth
+// INTERNAL count; then the coarse levels' starts and INTERNAL count
 constexpr int kPinTopOffset = kPinSlots * kCounterWords + 8;
 constexpr int kPinTopWords = 32;
 // one word for the extraction's split count reads, one for the topology's
@@ -278,9 +275,6 @@ void stage_extract(pi_frame* f);
 // after the anisotropy pass; the icosahedra at vertex v0 and triangle t0.
 void stage_splash_list(pi_frame* f);
 void splash_mesh(pi_frame* f, long long v0, long long t0);
-// Grid (blocks) of the cooperative coarse-level octree kernel on `device`,
-// 0 where cooperative launches are not available.
-int top_levels_grid(int device, int sm_count);
 // QEF vertices of the leaves of level [lb, le); scratch holds at least
 // le - lb + 1 ints (device memory the caller no longer needs).
 void qef_level(pi_frame* f, long long lb, long long le, int depth, const int8_t* npart = nullptr, int part = 0);

@@ -32,8 +32,6 @@
 #include <algorithm>
 #include <cmath>
 
-#include <cooperative_groups.h>
-
 #include "chunk.cuh"
 #include "device.cuh"
 #include "internal.h"
@@ -98,6 +96,22 @@ __device__ __forceinline__ bool inside(const GrownBox& b, float4 p) {
   return p.x > b.lox && p.x < b.hix && p.y > b.loy && p.y < b.hiy && p.z > b.loz && p.z < b.hiz && p.w == 0.f;
 }
 
+// Whether a particle of the sorted range [s, e) lies in the grown box: eight
+// at a time, so that their loads are in flight together (the range of a coarse
+// node's row beside the fluid holds a hundred and more that do not).
+__device__ __forceinline__ bool any_inside(const GrownBox& b, const float4* __restrict__ pos, int s, int e) {
+  for (; s < e; s += 8) {
+    float4 p[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p[k] = __ldg(pos + min(s + k, e - 1));
+    bool hit = false;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) hit |= inside(b, p[k]);
+    if (hit) return true;
+  }
+  return false;
+}
+
 // Particle range of cell c (linear index over the block) of a grown box.
 __device__ __forceinline__ void block_cell(const GridView& g, const GrownBox& b, int c, int* s, int* e) {
   const int nxb = b.x1 - b.x0 + 1, nyb = b.y1 - b.y0 + 1;
@@ -131,11 +145,7 @@ __global__ void k_empty(LevelArgs a, const float4* __restrict__ nd_c, float4* __
         const int z = b.z0 + r / nyb, y = b.y0 + r % nyb;
         const long long base = ((long long)z * a.g.ny + y) * a.g.nx;
         const int s = __ldg(a.g.off + base + b.x0), e = __ldg(a.g.off + base + b.x1 + 1);
-        for (int j = s; j < e; ++j)
-          if (inside(b, __ldg(a.pos + j))) {
-            hit = true;
-            break;
-          }
+        hit = any_inside(b, a.pos, s, e);
       }
       found = __any_sync(0xffffffffu, hit);
     }
@@ -901,24 +911,39 @@ __global__ void __launch_bounds__(32 * kSpawnWarps, CURV ? 16 : 24) k_spawn_scan
   }
 }
 
-// The coarse levels (depth < D_min - 1) in one cooperative launch: their
-// nodes are INTERNAL exactly when their grown box holds a particle, so a
-// level is an emptiness test per node, a scan of the INTERNAL flags and the
-// spawn of 8 children per INTERNAL node, the same steps (and results) as
-// k_empty, k_internal_flag, the scan and k_spawn, with grid-wide barriers
-// in place of launches and of the host's read of each level's size.  The
-// levels are small (at most kTopLevelNodes nodes; the loop stops before a
-// larger one), so block 0 scans the flags alone.  Node data written in the
-// launch is read through the L2 (ld.global.cg), never the read-only path.
-constexpr int kTopLevelNodes = 4096;
+// The coarse levels 0 .. D (D = D_min - 1, at most kTopDepth), in two
+// launches.  A coarse node is INTERNAL exactly when its grown box holds a
+// particle, and the nodes a level can hold are known beforehand: the 8^d
+// paths from the root, whose centres follow from the path alone.  So
+// k_top_test tests the paths of every level side by side (k_empty's test),
+// and k_top_nodes writes the nodes that exist: creation order within a level
+// is path order, so a node's place is eight times the number of INTERNAL
+// nodes before its parent, plus its octant.
+// What bounds it is latency: a coarse node spans thousands of cell rows, and a
+// level-by-level pass (one cooperative launch with a grid barrier between the
+// levels, a warp per node) waits for the longest scan of each level in turn.
+// It took 27 us on a 2k-particle frame, 207 us at 1M (dam break) and 596 us
+// at 1.7M; the two kernels take 5 + 6, 28 + 10 and 48 + 14 us.
+constexpr int kTopDepth = 5;         // 8^5 paths: testing the next level's 2^18 would cost more than a launch per level
+constexpr int kTopBlockDepth = 2;    // levels tested by a block per node (the others by a warp)
 constexpr int kTopThreads = 256;
 
+// Paths of the levels above d, and of the levels up to d.
+__host__ __device__ constexpr int top_base(int d) { return ((1 << (3 * d)) - 1) / 7; }
+// First word of level d's flags (each level starts a word).
+__host__ __device__ constexpr int top_word(int d) { return d == 0 ? 0 : d == 1 ? 1 : 2 + ((1 << (3 * d)) - 64) / 7 / 32; }
+constexpr int kTopWords = top_word(kTopDepth + 1);
+static_assert(kTopDepth + 5 <= kPinTopWords, "the level starts fit their pinned words");
+
 struct TopArgs {
-  LevelArgs la;  // grid, particles, expand, iso (lb / le / big set per level)
-  int dstop;     // levels 0 .. dstop - 1 at most
-  long long* lv;     // level starts: level d is [lv[d], lv[d + 1])
-  int* flag;         // kTopLevelNodes + 1
-  int* depth_out;    // levels done
+  LevelArgs la;  // grid, particles, expand, iso
+  int D;         // deepest level
+  int spawn;     // k_top_nodes also writes the children of level D's INTERNAL nodes
+  float cx, cy, cz, half;  // root
+  int size;                // the root's edge in lattice units
+  unsigned* flags;         // kTopWords: non-empty paths, a bit each
+  long long* lv;           // kPinTopWords: level starts, then the INTERNAL count of level D, then levels done
+  int* rank;               // level D: INTERNAL nodes before each node
   float4* nd_c;
   float4* nd_v;
   uint64_t* nd_id;
@@ -931,141 +956,169 @@ struct TopArgs {
   int4* nd_org;
 };
 
-__global__ void __launch_bounds__(kTopThreads) k_top_levels(TopArgs t) {
-  namespace cg = cooperative_groups;
-  cg::grid_group grid = cg::this_grid();
-  __shared__ int s_warp[kTopThreads / 32];
-  __shared__ int s_carry;
-  const int lane = threadIdx.x & 31;
-  const long long gwarp = ((long long)blockIdx.x * kTopThreads + threadIdx.x) >> 5;
-  const long long nwarps = (long long)gridDim.x * kTopThreads / 32;
-  const long long gthread = (long long)blockIdx.x * kTopThreads + threadIdx.x;
-  const long long nthreads = (long long)gridDim.x * kTopThreads;
-  int depth = 0;
-  for (;;) {
-    const long long lb = __ldcg(t.lv + depth), le = __ldcg(t.lv + depth + 1);
-    const long long n = le - lb;
-    LevelArgs a = t.la;
-    // emptiness: one warp per node (k_empty's test), INTERNAL if non-empty
-    for (long long w = gwarp; w < n; w += nwarps) {
-      const long long node = lb + w;
-      const GrownBox b = grown_box(a.g, __ldcg(t.nd_c + node), a.expand);
-      bool found = false;
-      if (b.x0 <= b.x1 && b.y0 <= b.y1 && b.z0 <= b.z1) {
-        const int nyb = b.y1 - b.y0 + 1;
-        const int rows = (b.z1 - b.z0 + 1) * nyb;
-        for (int r0 = 0; r0 < rows && !found; r0 += 32) {
-          const int r = r0 + lane;
-          bool hit = false;
-          if (r < rows) {
-            const int z = b.z0 + r / nyb, y = b.y0 + r % nyb;
-            const long long base = ((long long)z * a.g.ny + y) * a.g.nx;
-            const int s = __ldg(a.g.off + base + b.x0), e = __ldg(a.g.off + base + b.x1 + 1);
-            for (int j = s; j < e; ++j)
-              if (inside(b, __ldg(a.pos + j))) {
-                hit = true;
-                break;
-              }
-          }
-          found = __any_sync(0xffffffffu, hit);
-        }
-      }
-      if (lane == 0) {
-        if (!found) {
-          t.nd_type[node] = T_EMPTY;
-          t.nd_curv[node] = 1.0f;  // area == 0
-          float4 v = __ldcg(t.nd_v + node);
-          v.w = a.iso;
-          t.nd_v[node] = v;
-        } else {
-          t.nd_type[node] = T_INTERNAL;
-          t.nd_curv[node] = -1.0f;
-        }
-        t.flag[w] = found ? 1 : 0;
-      }
-    }
-    grid.sync();
-    // exclusive scan of the flags by block 0; the next level's end
-    if (blockIdx.x == 0) {
-      if (threadIdx.x == 0) s_carry = 0;
-      __syncthreads();
-      for (long long b0 = 0; b0 < n; b0 += kTopThreads) {
-        const long long i = b0 + threadIdx.x;
-        const int v = i < n ? __ldcg(t.flag + i) : 0;
-        int inc = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, inc, o);
-          if (lane >= o) inc += u;
-        }
-        if (lane == 31) s_warp[threadIdx.x >> 5] = inc;
-        __syncthreads();
-        int wbase = 0, total = 0;
-        for (int k = 0; k < kTopThreads / 32; ++k) {
-          if (k < (int)(threadIdx.x >> 5)) wbase += s_warp[k];
-          total += s_warp[k];
-        }
-        if (i < n) t.flag[i] = s_carry + wbase + inc - v;
-        __syncthreads();
-        if (threadIdx.x == 0) s_carry += total;
-        __syncthreads();
-      }
-      if (threadIdx.x == 0) t.lv[depth + 2] = le + 8LL * s_carry;
-    }
-    grid.sync();
-    // spawn (k_spawn): children of the INTERNAL nodes from the level's end on
-    for (long long w = gthread; w < n; w += nthreads) {
-      const long long i = lb + w;
-      if (__ldcg(t.nd_type + i) != T_INTERNAL) {
-        t.nd_child[i] = -1;
-        continue;
-      }
-      const long long b = le + 8LL * __ldcg(t.flag + w);
-      t.nd_child[i] = (int)b;
-      const float4 pc = __ldcg(t.nd_c + i);
-      const float hc = pc.w / 2;
-      const uint64_t pid = __ldcg(reinterpret_cast<const unsigned long long*>(t.nd_id) + i);
-      const int4 po = __ldcg(t.nd_org + i);
-      const int hs = po.w >> 1;
-      for (int k = 0; k < 8; ++k) {
-        const float sx = (k & 1) ? hc : -hc, sy = (k & 2) ? hc : -hc, sz = (k & 4) ? hc : -hc;
-        const float4 cc = make_float4(__fadd_rn(pc.x, sx), __fadd_rn(pc.y, sy), __fadd_rn(pc.z, sz), hc);
-        t.nd_c[b + k] = cc;
-        t.nd_v[b + k] = make_float4(cc.x, cc.y, cc.z, 0.f);
-        t.nd_id[b + k] = pid * 8ull + (uint64_t)k;
-        t.nd_parent[b + k] = (int)i;
-        t.nd_child[b + k] = -1;
-        t.nd_type[b + k] = T_UNCERTAIN;
-        t.nd_depth[b + k] = (int8_t)(depth + 1);
-        t.nd_sc[b + k] = 0;
-        t.nd_curv[b + k] = 0.f;
-        t.nd_org[b + k] =
-            make_int4(po.x + ((k & 1) ? hs : 0), po.y + ((k & 2) ? hs : 0), po.z + ((k & 4) ? hs : 0), hs);
-      }
-    }
-    const long long next = __ldcg(t.lv + depth + 2) - le;  // written before the last barrier
-    ++depth;
-    if (next == 0 || depth >= t.dstop || next > kTopLevelNodes) break;  // the same for every thread
-    grid.sync();
+// Centre and half size of path `id` of level d: the children's centres in
+// turn, as k_spawn computes them, and its integer origin.
+__device__ __forceinline__ float4 top_centre(const TopArgs& t, int d, int id, int4* org) {
+  float4 c = make_float4(t.cx, t.cy, t.cz, t.half);
+  int4 o = make_int4(0, 0, 0, t.size);
+  for (int l = d - 1; l >= 0; --l) {
+    const int k = (id >> (3 * l)) & 7;
+    const float hc = c.w / 2;
+    c = make_float4(__fadd_rn(c.x, (k & 1) ? hc : -hc), __fadd_rn(c.y, (k & 2) ? hc : -hc),
+                    __fadd_rn(c.z, (k & 4) ? hc : -hc), hc);
+    const int hs = o.w >> 1;
+    o = make_int4(o.x + ((k & 1) ? hs : 0), o.y + ((k & 2) ? hs : 0), o.z + ((k & 4) ? hs : 0), hs);
   }
-  if (gthread == 0) *t.depth_out = depth;
+  *org = o;
+  return c;
 }
 
-int top_levels_grid(int device, int sm_count) {
-  int coop = 0;
-  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device) != cudaSuccess || !coop) {
-    (void)cudaGetLastError();
-    return 0;
+__global__ void __launch_bounds__(kTopThreads) k_top_test(TopArgs t) {
+  __shared__ int s_found;
+  constexpr int warps = kTopThreads / 32;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // blocks [0, wide): a block per node of the first levels; then a warp per node
+  const int wide = top_base(min(t.D, kTopBlockDepth) + 1);
+  const bool whole = (int)blockIdx.x < wide;  // block-uniform
+  const int n = whole ? (int)blockIdx.x : wide + ((int)blockIdx.x - wide) * warps + warp;
+  if (whole) {
+    if (threadIdx.x == 0) s_found = 0;
+    __syncthreads();
   }
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_top_levels, kTopThreads, 0) != cudaSuccess ||
-      per_sm < 1) {
-    (void)cudaGetLastError();
-    return 0;
+  if (n >= top_base(t.D + 1)) return;  // a warp past the last node (never in a block-per-node block)
+  int d = 0;
+  while (n >= top_base(d + 1)) ++d;
+  const int id = n - top_base(d);
+  int4 org;
+  const LevelArgs& a = t.la;
+  const GrownBox b = grown_box(a.g, top_centre(t, d, id, &org), a.expand);
+  bool found = false;
+  if (b.x0 <= b.x1 && b.y0 <= b.y1 && b.z0 <= b.z1) {
+    const int nyb = b.y1 - b.y0 + 1;
+    const int rows = (b.z1 - b.z0 + 1) * nyb;
+    const int step = whole ? kTopThreads : 32;
+    for (int r0 = whole ? warp * 32 : 0; r0 < rows && !found; r0 += step) {
+      const int r = r0 + lane;
+      bool hit = false;
+      if (r < rows) {
+        const int z = b.z0 + r / nyb, y = b.y0 + r % nyb;
+        const long long base = ((long long)z * a.g.ny + y) * a.g.nx;
+        const int s = __ldg(a.g.off + base + b.x0), e = __ldg(a.g.off + base + b.x1 + 1);
+        hit = any_inside(b, a.pos, s, e);
+      }
+      // another warp of the node may have found a particle meanwhile
+      if (whole && *(volatile int*)&s_found) hit = true;
+      found = __any_sync(0xffffffffu, hit);
+    }
   }
-  // the coarse levels hold at most a few thousand nodes: half the SMs, one
-  // block each, leave room for other contexts' kernels
-  return std::max(1, std::min(per_sm * sm_count, sm_count / 2));
+  if (lane == 0 && found) {
+    if (whole) s_found = 1;
+    atomicOr(t.flags + top_word(d) + (id >> 5), 1u << (id & 31));
+  }
+}
+
+__global__ void __launch_bounds__(kTopThreads) k_top_nodes(TopArgs t) {
+  __shared__ unsigned s_flag[kTopWords];
+  __shared__ int s_pre[kTopWords];  // INTERNAL nodes of the word's level before the word
+  __shared__ int s_warp[kTopThreads / 32];
+  __shared__ int s_count[kTopDepth + 1];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // INTERNAL nodes: non-empty paths whose parent is INTERNAL (every block
+  // works this out for itself: at most 1172 words)
+  for (int d = 0; d <= t.D; ++d) {
+    const int words = max(1, (1 << (3 * d)) >> 5), w0 = top_word(d);
+    int carry = 0;
+    for (int i0 = 0; i0 < words; i0 += kTopThreads) {
+      const int i = i0 + threadIdx.x;
+      unsigned f = 0u;
+      if (i < words) {
+        f = t.flags[w0 + i];
+        if (d > 0) {
+          // the word's 32 nodes have 4 parents (one bit each) in one word
+          const unsigned pw = s_flag[top_word(d - 1) + (i >> 3)] >> ((i & 7) * 4);
+          unsigned keep = 0u;
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if ((pw >> k) & 1u) keep |= 0xffu << (8 * k);
+          f &= keep;
+        }
+        s_flag[w0 + i] = f;
+      }
+      const int c = __popc(f);
+      int inc = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
+      }
+      if (lane == 31) s_warp[warp] = inc;
+      __syncthreads();
+      int before = 0, total = 0;
+#pragma unroll
+      for (int k = 0; k < kTopThreads / 32; ++k) {
+        if (k < warp) before += s_warp[k];
+        total += s_warp[k];
+      }
+      if (i < words) s_pre[w0 + i] = carry + before + inc - c;
+      carry += total;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) s_count[d] = carry;
+  }
+  __syncthreads();
+  auto internal = [&](int d, int id) { return (s_flag[top_word(d) + (id >> 5)] >> (id & 31)) & 1u; };
+  auto rank = [&](int d, int id) {
+    return s_pre[top_word(d) + (id >> 5)] + __popc(s_flag[top_word(d) + (id >> 5)] & ((1u << (id & 31)) - 1u));
+  };
+  long long begin[kTopDepth + 3];
+  begin[0] = 0;
+  begin[1] = 1;
+  for (int d = 0; d <= t.D; ++d) begin[d + 2] = begin[d + 1] + 8LL * s_count[d];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    for (int d = 0; d <= t.D + 2; ++d) t.lv[d] = begin[d];
+    t.lv[t.D + 3] = s_count[t.D];
+  }
+  const int n = (int)(blockIdx.x * kTopThreads + threadIdx.x);
+  if (n >= top_base(t.D + 1)) return;
+  int d = 0;
+  while (n >= top_base(d + 1)) ++d;
+  const int id = n - top_base(d);
+  if (d > 0 && !internal(d - 1, id >> 3)) return;  // no such node
+  const long long at = d == 0 ? 0 : begin[d] + 8LL * rank(d - 1, id >> 3) + (id & 7);
+  const bool in = internal(d, id);
+  const long long kids = begin[d + 1] + 8LL * rank(d, id);
+  int4 org;
+  const float4 c = top_centre(t, d, id, &org);
+  t.nd_c[at] = c;
+  t.nd_v[at] = make_float4(c.x, c.y, c.z, in ? 0.f : t.la.iso);
+  t.nd_id[at] = (uint64_t)id;
+  t.nd_parent[at] = d == 0 ? -1 : d == 1 ? 0 : (int)(begin[d - 1] + 8LL * rank(d - 2, id >> 6) + ((id >> 3) & 7));
+  t.nd_child[at] = in ? (int)kids : -1;
+  t.nd_type[at] = in ? T_INTERNAL : T_EMPTY;
+  t.nd_depth[at] = (int8_t)d;
+  t.nd_sc[at] = 0;
+  t.nd_curv[at] = in ? -1.0f : 1.0f;  // area == 0 where empty; not needed where INTERNAL
+  t.nd_org[at] = org;
+  if (d < t.D) return;
+  t.rank[at - begin[d]] = rank(d, id);
+  if (!t.spawn || !in) return;
+  const float hc = c.w / 2;
+  const int hs = org.w >> 1;
+  for (int k = 0; k < 8; ++k) {
+    const float4 cc = make_float4(__fadd_rn(c.x, (k & 1) ? hc : -hc), __fadd_rn(c.y, (k & 2) ? hc : -hc),
+                                  __fadd_rn(c.z, (k & 4) ? hc : -hc), hc);
+    t.nd_c[kids + k] = cc;
+    t.nd_v[kids + k] = make_float4(cc.x, cc.y, cc.z, 0.f);
+    t.nd_id[kids + k] = (uint64_t)id * 8ull + (uint64_t)k;
+    t.nd_parent[kids + k] = (int)at;
+    t.nd_child[kids + k] = -1;
+    t.nd_type[kids + k] = T_UNCERTAIN;
+    t.nd_depth[kids + k] = (int8_t)(d + 1);
+    t.nd_sc[kids + k] = 0;
+    t.nd_curv[kids + k] = 0.f;
+    t.nd_org[kids + k] =
+        make_int4(org.x + ((k & 1) ? hs : 0), org.y + ((k & 2) ? hs : 0), org.z + ((k & 4) ? hs : 0), hs);
+  }
 }
 
 __global__ void k_root(float cx, float cy, float cz, float h, int size, float4* nd_c, float4* nd_v,
@@ -1440,12 +1493,12 @@ void stage_octree(pi_frame* f) {
   }
   f->nNodes = 0;
   f->levelBegin.clear();
-  ensure_nodes(f, 1 << 16);
+  // coarse levels written by k_top_nodes: 0 .. D, and the children of level D
+  // when it is not the last one above D_min
+  const int D = std::min(f->dmin - 1, kTopDepth);
+  const bool top_spawn = D < f->dmin - 1;
+  ensure_nodes(f, std::max(1 << 16, D >= 0 ? top_base(D + 1 + (top_spawn ? 1 : 0)) : 0));
   if (!f->ev[kLevelEvent]) PI_CUDA(cudaEventCreateWithFlags(&f->ev[kLevelEvent], cudaEventDisableTiming));
-  PI_LAUNCH(k_root, 1, 1, 0, s, f->rootC[0], f->rootC[1], f->rootC[2], f->rootH, 1 << f->dmax, f->nd_c.p,
-            f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p,
-            f->nd_curv.p, f->nd_org.p);
-  f->nNodes = 1;
   const GridHost& gh = f->g;
   GridView g{gh.bounding[0], gh.bounding[2], gh.bounding[4], gh.cell, gh.nx, gh.ny, gh.nz, f->off.p};
   PartView P{f->pos.p, f->xm.p, f->ga.p, f->gb.p, f->xlo.p};
@@ -1461,24 +1514,41 @@ void stage_octree(pi_frame* f) {
   ucum.alloc(ctx, s, ek + 1);  // exclusive scan of ucnt (sparse levels)
   long long lb = 0, le = 1;
   bool known = false;  // emptiness and curvature of this level settled by the parents' scan
+  // Spawns the children of level `depth` (INTERNAL ranks given), the children's
+  // emptiness and, unless they are leaves by size, their curvature sums with
+  // them.  Leaves by size never read their curvature (afterSampleEval returns
+  // before the curvature test).
+  auto spawn_scan = [&](const LevelArgs& la, int depth, const int* ranks) {
+    const float cell_child = 2.0f * std::ldexp(f->rootH, -(depth + 1));
+    const long long n = la.le - la.lb;
+    if ((double)(cell_child - f->P.radius) < 1e-8)
+      PI_LAUNCH(k_spawn_scan<false>, div_up(n, kSpawnWarps), 32 * kSpawnWarps, 0, s, la, la.le, ranks, depth + 1,
+                f->nd_c.p, f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p,
+                f->nd_sc.p, f->nd_curv.p, f->nd_org.p);
+    else
+      PI_LAUNCH(k_spawn_scan<true>, div_up(n, kSpawnWarps), 32 * kSpawnWarps, 0, s, la, la.le, ranks, depth + 1,
+                f->nd_c.p, f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p,
+                f->nd_sc.p, f->nd_curv.p, f->nd_org.p);
+  };
   int depth0 = 0;
-  if (f->dmin >= 2 && ctx->coop_blocks > 0) {
-    // the coarse levels 0 .. D_min - 2 in one cooperative launch
-    const int dstop = f->dmin - 1;
+  if (D >= 0) {
     DBuf<long long> lvd;
-    DBuf<int> tflag, dout;
-    lvd.alloc(ctx, s, dstop + 3);
-    tflag.alloc(ctx, s, kTopLevelNodes + 1);
-    dout.alloc(ctx, s, 1);
-    long long* const lvh = reinterpret_cast<long long*>(ctx->hpin + kPinTopOffset);
-    lvh[0] = 0;
-    lvh[1] = 1;
-    PI_CUDA(cudaMemcpyAsync(lvd.p, lvh, 2 * sizeof(long long), cudaMemcpyHostToDevice, s));
+    DBuf<unsigned> tflag;
+    lvd.alloc(ctx, s, kPinTopWords);
+    tflag.alloc(ctx, s, kTopWords);
+    flag.alloc(ctx, s, (size_t)1 << (3 * D));
+    PI_CUDA(cudaMemsetAsync(tflag.p, 0, sizeof(unsigned) * kTopWords, s));
     TopArgs ta{LevelArgs{g, f->pos.p, f->nrm.p, f->P.radius * f->P.smooth_factor, f->iso, f->P.radius, 0, 0, 1, P},
-               dstop,
-               lvd.p,
+               D,
+               top_spawn ? 1 : 0,
+               f->rootC[0],
+               f->rootC[1],
+               f->rootC[2],
+               f->rootH,
+               1 << f->dmax,
                tflag.p,
-               dout.p,
+               lvd.p,
+               flag.p,
                f->nd_c.p,
                f->nd_v.p,
                f->nd_id.p,
@@ -1489,19 +1559,32 @@ void stage_octree(pi_frame* f) {
                f->nd_sc.p,
                f->nd_curv.p,
                f->nd_org.p};
-    void* args[] = {&ta};
-    PI_CUDA(cudaLaunchCooperativeKernel((const void*)k_top_levels, dim3(ctx->coop_blocks), dim3(kTopThreads), args,
-                                        0, s));
-    count_launch();
-    int* const dh = reinterpret_cast<int*>(lvh + kPinTopWords - 1);
-    PI_CUDA(cudaMemcpyAsync(lvh, lvd.p, sizeof(long long) * (dstop + 2), cudaMemcpyDeviceToHost, s));
-    PI_CUDA(cudaMemcpyAsync(dh, dout.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    const int wide = top_base(std::min(D, kTopBlockDepth) + 1), paths = top_base(D + 1);
+    PI_LAUNCH(k_top_test, wide + div_up(paths - wide, kTopThreads / 32), kTopThreads, 0, s, ta);
+    PI_LAUNCH(k_top_nodes, div_up(paths, kTopThreads), kTopThreads, 0, s, ta);
+    long long* const lvh = reinterpret_cast<long long*>(ctx->hpin + kPinTopOffset);
+    PI_CUDA(cudaMemcpyAsync(lvh, lvd.p, sizeof(long long) * (D + 4), cudaMemcpyDeviceToHost, s));
     PI_CUDA(cudaStreamSynchronize(s));
-    depth0 = *dh;
-    for (int d = 0; d < depth0; ++d) f->levelBegin.push_back(lvh[d]);
-    lb = lvh[depth0];
-    le = lvh[depth0 + 1];
+    for (int d = 0; d <= D; ++d)
+      if (lvh[d + 1] > lvh[d]) f->levelBegin.push_back(lvh[d]);
+    lb = lvh[D], le = lvh[D + 1];
     f->nNodes = le;
+    const long long newn = 8 * lvh[D + 3];
+    if (newn > 0 && !top_spawn) {
+      ensure_nodes(f, le + newn);
+      spawn_scan(LevelArgs{g, f->pos.p, f->nrm.p, f->P.radius * f->P.smooth_factor, f->iso, f->P.radius, lb, le, 1, P},
+                 D, flag.p);
+      known = true;
+    }
+    lb = le;
+    le += newn;
+    f->nNodes = le;
+    depth0 = D + 1;
+  } else {
+    PI_LAUNCH(k_root, 1, 1, 0, s, f->rootC[0], f->rootC[1], f->rootC[2], f->rootH, 1 << f->dmax, f->nd_c.p,
+              f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p,
+              f->nd_curv.p, f->nd_org.p);
+    f->nNodes = 1;
   }
   for (int depth = depth0; le > lb; ++depth) {
     f->levelBegin.push_back(lb);
@@ -1627,18 +1710,7 @@ void stage_octree(pi_frame* f) {
     ensure_nodes(f, le + 8 * nl);  // room for the children: at most 8 per node of the level
     known = depth + 1 >= f->dmin && depth < f->dmax;
     if (known) {
-      // leaves by size never read their curvature (afterSampleEval returns
-      // before the curvature test), so their parents only settle emptiness
-      const float cell_child = 2.0f * std::ldexp(f->rootH, -(depth + 1));
-      const int child_curv = (double)(cell_child - f->P.radius) < 1e-8 ? 0 : 1;
-      if (child_curv)
-        PI_LAUNCH(k_spawn_scan<true>, div_up(nl, kSpawnWarps), 32 * kSpawnWarps, 0, s, la, le, flag.p, depth + 1, f->nd_c.p,
-                  f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p,
-                  f->nd_curv.p, f->nd_org.p);
-      else
-        PI_LAUNCH(k_spawn_scan<false>, div_up(nl, kSpawnWarps), 32 * kSpawnWarps, 0, s, la, le, flag.p, depth + 1, f->nd_c.p,
-                  f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p,
-                  f->nd_curv.p, f->nd_org.p);
+      spawn_scan(la, depth, flag.p);
     } else {
       PI_LAUNCH(k_spawn, div_up(nl, 256), 256, 0, s, lb, le, le, flag.p, f->nd_type.p, depth + 1, f->nd_c.p,
                 f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p,
