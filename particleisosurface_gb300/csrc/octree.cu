@@ -32,6 +32,8 @@
 #include <algorithm>
 #include <cmath>
 
+#include <cooperative_groups.h>
+
 #include "chunk.cuh"
 #include "device.cuh"
 #include "internal.h"
@@ -291,9 +293,11 @@ __device__ __forceinline__ uint32_t hash3(float x, float y, float z) {
 // candidates, same summation order), so each distinct point is evaluated
 // once.  Equal points share a bucket; bucket k owns hash slots
 // [2 qoff[k], 2 qoff[k+1]) and a point's first inserter becomes its
-// representative.  Representatives get consecutive places in the bucket's
-// range of `order` (on a dense level k_q_chunks then cuts them into chunks, on
-// a sparse level k_q_compact lists them in bucket order).
+// representative.  Representatives get consecutive places in the bucket: on a
+// dense level they are written to the bucket's range of `order`, which
+// k_q_chunks then cuts into chunks; on a sparse level order[i] is sample i's
+// place (-1 for the others) and k_q_compact lists them in bucket order.
+template <bool DENSE>
 __global__ void k_q_dedupe(QArgs a, long long n, const float4* __restrict__ nd_c, const float4* __restrict__ nd_v,
                            const int* __restrict__ qkey, const int* __restrict__ qoff, unsigned* __restrict__ hslot,
                            int* __restrict__ ucnt, int* __restrict__ rep, int* __restrict__ order) {
@@ -346,8 +350,9 @@ __global__ void k_q_dedupe(QArgs a, long long n, const float4* __restrict__ nd_c
     if (lane == leader) b0 = atomicAdd(ucnt + k, __popc(peers));
     b0 = __shfl_sync(peers, b0, leader);
     place = b0 + __popc(peers & ((1u << lane) - 1u));
-    order[qoff[k] + place] = (int)i;
+    if (DENSE) order[qoff[k] + place] = (int)i;
   }
+  if (!DENSE && i < n) order[i] = uniq ? place : -1;
 }
 
 // Chunks of a dense level: each bucket's distinct samples cut into runs of
@@ -562,18 +567,20 @@ __global__ void __launch_bounds__(256, 4) k_q_eval_thread(QArgs a, const int* __
   }
 }
 
-// Sparse levels: the distinct samples, placed per bucket by k_q_dedupe, made
+// Sparse levels: the distinct samples, numbered per bucket by k_q_dedupe, made
 // into one list in bucket order (ucum = exclusive scan of the bucket counts),
-// so that neighbouring threads of k_q_eval_thread walk the same cells.
-__global__ void k_q_compact(long long nb, const int* __restrict__ qoff, const int* __restrict__ ucnt,
-                            const int* __restrict__ ucum, const int* __restrict__ order, int* __restrict__ list) {
-  const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= nb) return;
-  const int u = ucnt[k];
-  if (u == 0) return;
-  const int* src = order + qoff[k];
-  int* dst = list + ucum[k];
-  for (int t = 0; t < u; ++t) dst[t] = src[t];
+// so that neighbouring threads of k_q_eval_thread walk the same cells.  A
+// thread per sample, whatever the buckets hold: a thread (or a warp) per
+// bucket waited for the fullest ones, 123 us on the finest level of a
+// 50k-particle two-radius frame, where a few hundred of 46k buckets hold all
+// 0.5M distinct samples; this takes 11 us (and 36 us instead of 21 on the two
+// sparse levels of the 1M dam break, whose buckets hold a few samples each).
+__global__ void k_q_compact(long long n, const int* __restrict__ qkey, const int* __restrict__ place,
+                            const int* __restrict__ ucum, int* __restrict__ list) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int p = place[i];
+  if (p >= 0) list[ucum[qkey[i]] + p] = (int)i;
 }
 
 // Leaves by size without QEF: afterSampleEval (src/surface_reconstructor.cpp:
@@ -1348,6 +1355,107 @@ __global__ void __launch_bounds__(64) k_vr_empty(const MultiGridView* __restrict
   }
 }
 
+// The same for the few nodes of a coarse level: a cluster of CL blocks per
+// node, a warp per cell row, lanes over the row's particles, the blocks' sums
+// combined through distributed shared memory.  A coarse node spans most of the
+// particles: a warp per node took 1172, 292, 277 and 109 us on the first four
+// levels of a 50k-particle frame (latency of one warp's serial walk); they
+// take 33, 18, 19 and 26 us this way.  Above D_min nothing decides on the curvature,
+// so its summation order is free there.
+constexpr int kWideThreads = 256;
+constexpr int kWideNodes = 1024;  // a level of more nodes fills the GPU with a warp per node
+
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kWideThreads)
+    k_vr_empty_wide(const MultiGridView* __restrict__ mg, LevelArgs a, float emax, const float4* __restrict__ nd_c,
+                    float4* __restrict__ nd_v, int8_t* __restrict__ nd_type, float* __restrict__ nd_curv,
+                    float* __restrict__ nd_minr) {
+  namespace cg = cooperative_groups;
+  constexpr int warps = kWideThreads / 32;
+  __shared__ float s_part[warps][6];  // found, min radius, normal sums, area
+  const int part = (int)(blockIdx.x % CL);
+  const long long node = a.lb + blockIdx.x / CL;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const MultiGridView& m = *mg;
+  const float4 c = nd_c[node];
+  const float h = c.w;
+  const float b1x = __fsub_rn(c.x, h), b1y = __fsub_rn(c.y, h), b1z = __fsub_rn(c.z, h);
+  const float b2x = __fadd_rn(c.x, h), b2y = __fadd_rn(c.y, h), b2z = __fadd_rn(c.z, h);
+  bool found = false;
+  float minr = 3.402823466e38f;
+  Kahan sx, sy, sz, ar;
+  for (int b = 0; b < m.nb; ++b) {
+    const BinGrid g = m.g[b];
+    const int x0 = max(cell_coord(__fsub_rn(b1x, emax), g.b0, g.cell, g.nx), 0);
+    const int y0 = max(cell_coord(__fsub_rn(b1y, emax), g.b2, g.cell, g.ny), 0);
+    const int z0 = max(cell_coord(__fsub_rn(b1z, emax), g.b4, g.cell, g.nz), 0);
+    const int x1 = min(cell_coord(__fadd_rn(b2x, emax), g.b0, g.cell, g.nx), g.nx - 1);
+    const int y1 = min(cell_coord(__fadd_rn(b2y, emax), g.b2, g.cell, g.ny), g.ny - 1);
+    const int z1 = min(cell_coord(__fadd_rn(b2z, emax), g.b4, g.cell, g.nz), g.nz - 1);
+    if (x0 > x1 || y0 > y1 || z0 > z1) continue;
+    const int nyb = y1 - y0 + 1;
+    const int rows = (z1 - z0 + 1) * nyb;
+    for (int r = part * warps + warp; r < rows; r += CL * warps) {
+      const int z = z0 + r / nyb, y = y0 + r % nyb;
+      const long long base = (long long)g.offBase + ((long long)z * g.ny + y) * g.nx;
+      const int s = __ldg(m.off + base + x0), e = __ldg(m.off + base + x1 + 1);
+#pragma unroll 2
+      for (int j = s + lane; j < e; j += 32) {
+        const float4 p = __ldg(a.pos + j);
+        const float ej = p.w * a.expand;  // r_j * smooth_factor
+        if (p.x > __fsub_rn(b1x, ej) && p.x < __fadd_rn(b2x, ej) && p.y > __fsub_rn(b1y, ej) &&
+            p.y < __fadd_rn(b2y, ej) && p.z > __fsub_rn(b1z, ej) && p.z < __fadd_rn(b2z, ej)) {
+          found = true;
+          minr = fminf(minr, p.w);
+          const float4 nv = __ldg(a.nrm + j);
+          sx.add(nv.x);
+          sy.add(nv.y);
+          sz.add(nv.z);
+          ar.add(nv.w);
+        }
+      }
+    }
+  }
+  found = __any_sync(0xffffffffu, found);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) minr = fminf(minr, __shfl_xor_sync(0xffffffffu, minr, o));
+  const float nx = warp_sum(sx.s - sx.c), ny = warp_sum(sy.s - sy.c), nz = warp_sum(sz.s - sz.c);
+  const float area = warp_sum(ar.s - ar.c);
+  if (lane == 0) {
+    float* const p = s_part[warp];
+    p[0] = found ? 1.f : 0.f, p[1] = minr, p[2] = nx, p[3] = ny, p[4] = nz, p[5] = area;
+  }
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
+  if (part == 0 && threadIdx.x == 0) {
+    bool any = false;
+    float mr = 3.402823466e38f;
+    Kahan tx, ty, tz, ta;
+    for (int q = 0; q < CL; ++q) {
+      const float* p = cluster.map_shared_rank(&s_part[0][0], q);
+      for (int w = 0; w < warps; ++w, p += 6) {
+        any = any || p[0] != 0.f;
+        mr = fminf(mr, p[1]);
+        tx.add(p[2]), ty.add(p[3]), tz.add(p[4]), ta.add(p[5]);
+      }
+    }
+    if (!any) {
+      nd_type[node] = T_EMPTY;
+      nd_curv[node] = 1.0f;
+      float4 v = nd_v[node];
+      v.w = a.iso;
+      nd_v[node] = v;
+    } else {
+      const bool leaf_by_size = 2.0f * h - mr < kAbove1em8;  // as k_vr_empty
+      nd_type[node] = (a.big && !leaf_by_size) ? T_INTERNAL : T_UNCERTAIN;
+      const float vx = tx.s - tx.c, vy = ty.s - ty.c, vz = tz.s - tz.c, va = ta.s - ta.c;
+      nd_curv[node] = (va == 0.f) ? 1.0f : sqrtf(vx * vx + vy * vy + vz * vz) / va;
+      nd_minr[node] = mr;
+    }
+  }
+  cluster.sync();  // the sums are read before their blocks end
+}
+
 // Leaves by size above D_min (variable radius only): no GridEval there, the
 // value is SingleEval at the node position (src/surface_reconstructor.cpp:
 // 245-253).
@@ -1427,8 +1535,19 @@ static void stage_octree_vr(pi_frame* f) {
     f->levelBegin.push_back(lb);
     const long long nl = le - lb;
     LevelArgs la{bg, f->pos.p, f->nrm.p, f->P.smooth_factor, f->iso, f->vrMinR, lb, le, depth < f->dmin ? 1 : 0, P};
-    PI_LAUNCH(k_vr_empty, div_up(nl, 2), 64, 0, s, f->mgv.p, la, f->vrMaxR * f->P.smooth_factor, f->nd_c.p,
-              f->nd_v.p, f->nd_type.p, f->nd_curv.p, f->nd_minr.p);
+    // by level size: a cluster of 8 blocks per node while that leaves SMs
+    // idle, a block per node up to kWideNodes, else (and on every level whose
+    // curvature decides) a warp per node
+    const float emax = f->vrMaxR * f->P.smooth_factor;
+    if (depth < f->dmin && nl <= 64)
+      PI_LAUNCH(k_vr_empty_wide<8>, (unsigned)nl * 8, kWideThreads, 0, s, f->mgv.p, la, emax, f->nd_c.p, f->nd_v.p,
+                f->nd_type.p, f->nd_curv.p, f->nd_minr.p);
+    else if (depth < f->dmin && nl <= kWideNodes)
+      PI_LAUNCH(k_vr_empty_wide<1>, (unsigned)nl, kWideThreads, 0, s, f->mgv.p, la, emax, f->nd_c.p, f->nd_v.p,
+                f->nd_type.p, f->nd_curv.p, f->nd_minr.p);
+    else
+      PI_LAUNCH(k_vr_empty, div_up(nl, 2), 64, 0, s, f->mgv.p, la, emax, f->nd_c.p, f->nd_v.p, f->nd_type.p,
+                f->nd_curv.p, f->nd_minr.p);
     if (depth < f->dmin)
       PI_LAUNCH(k_vr_big_leaf, div_up(nl, 128), 128, 0, s, f->mgv.p, la, f->nd_v.p, f->nd_type.p, f->dcount.p);
     if (depth >= f->dmin) {
@@ -1446,11 +1565,11 @@ static void stage_octree_vr(pi_frame* f) {
       PI_LAUNCH(k_q_count_node, div_up(nl, kCountThreads), kCountThreads, 0, s, qa, f->nd_c.p, f->nd_v.p,
                 f->nd_type.p, qcnt.p, qkey.p);
       exclusive_scan_i32(qcnt.p, qcnt.p, nb + 1, nullptr, f->tmp.p, s);
-      PI_LAUNCH(k_q_dedupe, div_up(qn, 256), 256, 0, s, qa, qn, f->nd_c.p, f->nd_v.p, qkey.p, qcnt.p, hslot.p,
+      PI_LAUNCH(k_q_dedupe<false>, div_up(qn, 256), 256, 0, s, qa, qn, f->nd_c.p, f->nd_v.p, qkey.p, qcnt.p, hslot.p,
                 ucnt.p, rep.p, order.p);
       int* list = reinterpret_cast<int*>(hslot.p);
       exclusive_scan_i32(ucnt.p, ucum.p, nb + 1, nullptr, f->tmp.p, s);
-      PI_LAUNCH(k_q_compact, div_up(nb, 256), 256, 0, s, nb, qcnt.p, ucnt.p, ucum.p, order.p, list);
+      PI_LAUNCH(k_q_compact, div_up(qn, 256), 256, 0, s, qn, qkey.p, order.p, ucum.p, list);
       prof_begin(ctx, s, PG_THREAD);
       PI_LAUNCH(k_vr_q_eval_thread, (int)std::min<long long>((long long)ctx->smCount * 8, div_up(qn, 256)), 256, 0,
                 s, f->mgv.p, qa, list, ucum.p + nb, f->nd_c.p, f->nd_v.p, qval.p, f->dcount.p);
@@ -1634,12 +1753,16 @@ void stage_octree(pi_frame* f) {
       PI_LAUNCH(k_q_count_node, div_up(nl, kCountThreads), kCountThreads, 0, s, qa, f->nd_c.p, f->nd_v.p,
                 f->nd_type.p, qcnt.p, qkey.p);
       exclusive_scan_i32(qcnt.p, qcnt.p, nb + 1, nullptr, f->tmp.p, s);
-      PI_LAUNCH(k_q_dedupe, div_up(qn, 256), 256, 0, s, qa, qn, f->nd_c.p, f->nd_v.p, qkey.p, qcnt.p, hslot.p,
-                ucnt.p, rep.p, order.p);
+      if (dense)
+        PI_LAUNCH(k_q_dedupe<true>, div_up(qn, 256), 256, 0, s, qa, qn, f->nd_c.p, f->nd_v.p, qkey.p, qcnt.p, hslot.p,
+                  ucnt.p, rep.p, order.p);
+      else
+        PI_LAUNCH(k_q_dedupe<false>, div_up(qn, 256), 256, 0, s, qa, qn, f->nd_c.p, f->nd_v.p, qkey.p, qcnt.p,
+                  hslot.p, ucnt.p, rep.p, order.p);
       int* list = reinterpret_cast<int*>(hslot.p);  // the hash slots are free once the samples are placed
       if (!dense) {
         exclusive_scan_i32(ucnt.p, ucum.p, nb + 1, nullptr, f->tmp.p, s);
-        PI_LAUNCH(k_q_compact, div_up(nb, 256), 256, 0, s, nb, qcnt.p, ucnt.p, ucum.p, order.p, list);
+        PI_LAUNCH(k_q_compact, div_up(qn, 256), 256, 0, s, qn, qkey.p, order.p, ucum.p, list);
       }
       int cfg = 0;
       if (dense)
