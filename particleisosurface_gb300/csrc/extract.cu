@@ -28,6 +28,7 @@
 #include "device.cuh"
 #include "dmc.h"
 #include "internal.h"
+#include "scan.cuh"
 
 namespace pisurf {
 
@@ -69,11 +70,23 @@ __device__ __forceinline__ void edge_corners(int e, int* c0, int* c1) {
   *c1 = *c0 | (1 << axis);
 }
 
-__global__ void k_leaf_flag(const int* __restrict__ nd_child, long long n, int* __restrict__ flag) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) flag[i] = nd_child[i] < 0 ? 1 : 0;
-  if (i == n) flag[i] = 0;
-}
+// Scan inputs: leaf flags of the nodes, set bits of the bitmap words.
+struct LeafNode {
+  const int* child;
+  __device__ int operator()(long long i) const { return child[i] < 0 ? 1 : 0; }
+  __device__ int4 four(long long i) const {
+    const int4 c = *reinterpret_cast<const int4*>(child + i);
+    return make_int4(c.x < 0, c.y < 0, c.z < 0, c.w < 0);
+  }
+};
+struct WordBits {
+  const unsigned* bits;
+  __device__ int operator()(long long i) const { return __popc(bits[i]); }
+  __device__ int4 four(long long i) const {
+    const uint4 b = *reinterpret_cast<const uint4*>(bits + i);
+    return make_int4(__popc(b.x), __popc(b.y), __popc(b.z), __popc(b.w));
+  }
+};
 
 __global__ void k_leaf_list(const int* __restrict__ nd_child, const int* __restrict__ scan, long long n,
                             int* __restrict__ leaves) {
@@ -181,12 +194,6 @@ __global__ void k_corner_mark(const int* __restrict__ leaves, long long nl, cons
   }
 }
 
-__global__ void k_bitmap_count(const unsigned* __restrict__ bits, long long nw, int* __restrict__ cnt) {
-  long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (w < nw) cnt[w] = __popc(bits[w]);
-  if (w == nw) cnt[w] = 0;
-}
-
 __global__ void k_bitmap_keys(const unsigned* __restrict__ bits, long long nw, const int* __restrict__ off, int bb,
                               const long long* __restrict__ blist, int B, uint64_t* __restrict__ out) {
   long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -280,6 +287,28 @@ __global__ void k_first_flag(long long n, const unsigned* __restrict__ tab, cons
   long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s < n) flag[s] = tab[where[s]] == (unsigned)s + 1u ? 1 : 0;
   if (s == n) flag[s] = 0;
+}
+
+// The same as a scan input (a sequence the scan reads once).
+struct FirstSlot {
+  const unsigned* tab;
+  const uint32_t* where;
+  __device__ int operator()(long long i) const { return tab[where[i]] == (unsigned)i + 1u ? 1 : 0; }
+  __device__ int4 four(long long i) const {
+    return make_int4((*this)(i), (*this)(i + 1), (*this)(i + 2), (*this)(i + 3));
+  }
+};
+
+// Ranks of the first slots among n: rank[n] is their number.  The flags are
+// worked out inside the scan while it reads them once; a longer scan reads its
+// input twice, and the flags' random table reads are dearer than an array.
+static void rank_first(long long n, const unsigned* tab, const uint32_t* where, int* rank, int* tmp, cudaStream_t s) {
+  if (n + 1 <= kScanOneLaunch) {
+    exclusive_scan(ScanOf<FirstSlot>{{tab, where}, n}, rank, n + 1, nullptr, tmp, s);
+    return;
+  }
+  PI_LAUNCH(k_first_flag, div_up(n + 1, 256), 256, 0, s, n, tab, where, rank);
+  exclusive_scan_i32(rank, rank, n + 1, nullptr, tmp, s);
 }
 
 // slot -> vertex (numbered in order of first slots); vertex -> its first slot
@@ -593,8 +622,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
   DBuf<int> flag, leaves, tmp;
   flag.alloc(c, s, nn + 1);
   tmp.alloc(c, s, scan_tmp_ints(nn * 8 + 1));
-  PI_LAUNCH(k_leaf_flag, div_up(nn + 1, 256), 256, 0, s, f->nd_child.p, nn, flag.p);
-  exclusive_scan_i32(flag.p, flag.p, nn + 1, nullptr, tmp.p, s);
+  exclusive_scan(ScanOf<LeafNode>{{f->nd_child.p}, nn}, flag.p, nn + 1, nullptr, tmp.p, s);
   rd.start(flag.p + nn);
   leaves.alloc(c, s, nn > 0 ? nn : 1);  // room for every node
   PI_LAUNCH(k_leaf_list, div_up(nn, 256), 256, 0, s, f->nd_child.p, flag.p, nn, leaves.p);
@@ -638,8 +666,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     PI_CUDA(cudaMemsetAsync(bits.p, 0, sizeof(unsigned) * (nw > 0 ? nw : 1), s));
     PI_LAUNCH(k_corner_mark, div_up(nk, 256), 256, 0, s, leaves.p, nl, f->nd_org.p, full, bb,
               dense ? nullptr : slot.p, bits.p);
-    PI_LAUNCH(k_bitmap_count, div_up(nw + 1, 256), 256, 0, s, bits.p, nw, cnt.p);
-    exclusive_scan_i32(cnt.p, cnt.p, nw + 1, nullptr, tmp.p, s);
+    exclusive_scan(ScanOf<WordBits>{{bits.p}, nw}, cnt.p, nw + 1, nullptr, tmp.p, s);
     nu = rd.read(cnt.p + nw);
     if (uverts.n < (size_t)(nu > 0 ? nu : 1)) uverts.alloc(c, s, nu > 0 ? nu : 1);
     PI_LAUNCH(k_bitmap_keys, div_up(nw, 256), 256, 0, s, bits.p, nw, cnt.p, bb, dense ? nullptr : blist.p, B,
@@ -752,8 +779,7 @@ void stage_extract(pi_frame* f) {
   PI_CUDA(cudaMemsetAsync(vtab.p, 0, sizeof(unsigned) * ((size_t)vmask + 1), s));
   PI_LAUNCH(k_vkey_insert, div_up(ns, 256), 256, 0, s, ns, packed ? nullptr : khi.p, klo.p, vmask, vtab.p,
             vwhere.p);
-  PI_LAUNCH(k_first_flag, div_up(ns + 1, 256), 256, 0, s, ns, vtab.p, vwhere.p, vrank.p);
-  exclusive_scan_i32(vrank.p, vrank.p, ns + 1, nullptr, tmp.p, s);
+  rank_first(ns, vtab.p, vwhere.p, vrank.p, tmp.p, s);
   read_int_start(f, vrank.p + ns);
   slot_vertex.alloc(c, s, ns > 0 ? ns : 1);
   rep.alloc(c, s, ns > 0 ? ns : 1);  // room for a vertex per slot
@@ -781,8 +807,7 @@ void stage_extract(pi_frame* f) {
   trank.alloc(c, s, nt0 + 1);
   PI_CUDA(cudaMemsetAsync(ttab.p, 0, sizeof(unsigned) * ((size_t)tmask + 1), s));
   PI_LAUNCH(k_tri_insert, div_up(nt0, 256), 256, 0, s, nt0, otri.p, tmask, ttab.p, twhere.p);
-  PI_LAUNCH(k_first_flag, div_up(nt0 + 1, 256), 256, 0, s, nt0, ttab.p, twhere.p, trank.p);
-  exclusive_scan_i32(trank.p, trank.p, nt0 + 1, nullptr, tmp.p, s);
+  rank_first(nt0, ttab.p, twhere.p, trank.p, tmp.p, s);
   read_int_start(f, trank.p + nt0);
   // room for every generated triangle and the splash icosahedra
   const long long nsp = f->P.splash ? f->nSplash : 0;

@@ -37,6 +37,7 @@
 #include "chunk.cuh"
 #include "device.cuh"
 #include "internal.h"
+#include "scan.cuh"
 
 namespace pisurf {
 
@@ -730,12 +731,14 @@ __global__ void __launch_bounds__(256) k_classify_thread(LevelArgs a, const floa
   if ((threadIdx.x & 31) == 0) stripe_add(counters, C_REF_EVALS, evals);
 }
 
-__global__ void k_internal_flag(const int8_t* __restrict__ nd_type, long long lb, long long le,
-                                int* __restrict__ flag) {
-  long long i = lb + (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= le) return;
-  flag[i - lb] = nd_type[i] == T_INTERNAL ? 1 : 0;
-}
+// INTERNAL flags of a level's nodes, for the scan that ranks them.
+struct InternalNode {
+  const int8_t* type;  // of the level's first node
+  __device__ int operator()(long long i) const { return type[i] == T_INTERNAL ? 1 : 0; }
+  __device__ int4 four(long long i) const {
+    return make_int4((*this)(i), (*this)(i + 1), (*this)(i + 2), (*this)(i + 3));
+  }
+};
 
 __global__ void k_spawn(long long lb, long long le, long long cbase, const int* __restrict__ rank,
                         const int8_t* nd_type, int child_depth, float4* __restrict__ nd_c,
@@ -1580,9 +1583,7 @@ static void stage_octree_vr(pi_frame* f) {
     }
     flag.alloc(ctx, s, nl + 1);
     if (f->tmp.n < scan_tmp_ints(nl + 1)) f->tmp.alloc(ctx, s, scan_tmp_ints(nl + 1));
-    PI_LAUNCH(k_internal_flag, div_up(nl, 256), 256, 0, s, f->nd_type.p, lb, le, flag.p);
-    PI_CUDA(cudaMemsetAsync(flag.p + nl, 0, sizeof(int), s));
-    exclusive_scan_i32(flag.p, flag.p, nl + 1, nullptr, f->tmp.p, s);
+    exclusive_scan(ScanOf<InternalNode>{{f->nd_type.p + lb}, nl}, flag.p, nl + 1, nullptr, f->tmp.p, s);
     int* const nint_h = reinterpret_cast<int*>(ctx->hpin + kPinSlots * kCounterWords + 1);
     PI_CUDA(cudaMemcpyAsync(nint_h, flag.p + nl, sizeof(int), cudaMemcpyDeviceToHost, s));
     PI_CUDA(cudaEventRecord(f->ev[kLevelEvent], s));
@@ -1820,9 +1821,7 @@ void stage_octree(pi_frame* f) {
     }
     flag.alloc(ctx, s, nl + 1);
     if (f->tmp.n < scan_tmp_ints(nl + 1)) f->tmp.alloc(ctx, s, scan_tmp_ints(nl + 1));
-    PI_LAUNCH(k_internal_flag, div_up(nl, 256), 256, 0, s, f->nd_type.p, lb, le, flag.p);
-    PI_CUDA(cudaMemsetAsync(flag.p + nl, 0, sizeof(int), s));
-    exclusive_scan_i32(flag.p, flag.p, nl + 1, nullptr, f->tmp.p, s);
+    exclusive_scan(ScanOf<InternalNode>{{f->nd_type.p + lb}, nl}, flag.p, nl + 1, nullptr, f->tmp.p, s);
     // the number of INTERNAL nodes goes to pinned host memory and is read
     // while the spawn kernel runs, so that the device is still busy when the
     // host sizes the next level
