@@ -6,7 +6,7 @@
 // are exactly the corners of leaves that lie strictly inside the root box, so
 // here they are enumerated in parallel:
 //   1. every leaf marks its interior corners (integer lattice at D_max) in
-//      a Morton-indexed lattice bitmap (sort + unique above D_max = 10); the
+//      a Morton-indexed lattice bitmap (sort + unique above D_max = 14); the
 //      set bits in index order are the dual vertices, in Z order;
 //   2. per vertex, the leaf containing each of the 8 octants is found by
 //      descending from the root; sign code, table[256] -> canonical case;
@@ -70,15 +70,7 @@ __device__ __forceinline__ void edge_corners(int e, int* c0, int* c1) {
   *c1 = *c0 | (1 << axis);
 }
 
-// Scan inputs: leaf flags of the nodes, set bits of the bitmap words.
-struct LeafNode {
-  const int* child;
-  __device__ int operator()(long long i) const { return child[i] < 0 ? 1 : 0; }
-  __device__ int4 four(long long i) const {
-    const int4 c = *reinterpret_cast<const int4*>(child + i);
-    return make_int4(c.x < 0, c.y < 0, c.z < 0, c.w < 0);
-  }
-};
+// Scan input: set bits of the bitmap words.
 struct WordBits {
   const unsigned* bits;
   __device__ int operator()(long long i) const { return __popc(bits[i]); }
@@ -88,23 +80,17 @@ struct WordBits {
   }
 };
 
-__global__ void k_leaf_list(const int* __restrict__ nd_child, const int* __restrict__ scan, long long n,
-                            int* __restrict__ leaves) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && nd_child[i] < 0) leaves[scan[i]] = (int)i;
-}
-
 // Interior corners of each leaf, key (x << 2B) | (y << B) | z, B = D_max + 1;
-// boundary corners get the all-ones key.
-__global__ void k_corner_keys(const int* __restrict__ leaves, long long nl, const int4* __restrict__ nd_org,
+// boundary corners, and those of nodes that are no leaves, get the all-ones key.
+__global__ void k_corner_keys(const int* __restrict__ nd_child, long long nn, const int4* __restrict__ nd_org,
                               int full, int B, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nl * 8) return;
-  const int4 o = nd_org[leaves[t >> 3]];
+  if (t >= nn * 8) return;
+  const int4 o = nd_org[t >> 3];
   const int k = (int)(t & 7);
   const int x = o.x + ((k & 1) ? o.w : 0), y = o.y + ((k & 2) ? o.w : 0), z = o.z + ((k & 4) ? o.w : 0);
   uint64_t key;
-  if (x > 0 && x < full && y > 0 && y < full && z > 0 && z < full)
+  if (nd_child[t >> 3] < 0 && x > 0 && x < full && y > 0 && y < full && z > 0 && z < full)
     key = ((uint64_t)x << (2 * B)) | ((uint64_t)y << B) | (uint64_t)z;
   else
     key = (1ull << (3 * B)) - 1ull;
@@ -136,29 +122,98 @@ __device__ __forceinline__ uint64_t compact3(uint64_t v) {
 // Interior leaf corners (coordinates 1 .. 2^D_max - 1) as bits of a lattice
 // bitmap indexed by the Morton code of (x - 1, y - 1, z - 1).  The Morton
 // range is cut into blocks of 2^bb codes (a 2^(bb/3)-cube of lattice
-// points).  Up to D_max = 10 (2^30 bits) every block is stored (slot = block,
+// points).  Up to D_max = 9 (2^27 bits) every block is stored (slot = block,
 // slot and blist null); above it only the blocks that hold a corner, with
 // consecutive slots in block order, so that work and memory follow the
 // surface rather than the volume of the lattice.  Either way the set bits in
 // slot order are the unique corners in Z order, which keeps the later
 // per-vertex work spatially coherent (as the reference's recursive
 // traversal is).
-__device__ __forceinline__ bool corner_code(const int* __restrict__ leaves, const int4* __restrict__ nd_org,
-                                            int full, long long t, uint64_t* idx) {
-  const int4 o = nd_org[leaves[t >> 3]];
-  const int k = (int)(t & 7);
-  const int x = o.x + ((k & 1) ? o.w : 0), y = o.y + ((k & 2) ? o.w : 0), z = o.z + ((k & 4) ? o.w : 0);
-  if (!(x > 0 && x < full && y > 0 && y < full && z > 0 && z < full)) return false;
-  *idx = spread3((uint64_t)(x - 1)) | (spread3((uint64_t)(y - 1)) << 1) | (spread3((uint64_t)(z - 1)) << 2);
+//
+// The corners are taken family by family: the eight children of a node are
+// consecutive (family f holds nodes 8 f + 1 to 8 f + 8), and when all eight are
+// leaves, as nearly every family with a leaf is, their 64 corners are the 27
+// points of a 3 x 3 x 3 lattice.  A point's Morton code is the OR of its
+// coordinates' spread codes, so the points of one bitmap word are a product of
+// per-axis sets and their bits come from shifts: two to eight words, and as many
+// atomics, a family.  A lane per corner, merging the bits of equal words across
+// the warp, took 438 us for the 4.4M leaves of a 1M dam-break frame (12 merge
+// rounds a warp); a thread per family takes 37 us and needs no leaf list.
+
+// The spread codes (x and shifts applied) of the three lattice coordinates
+// o - 1, o + w - 1, o + 2 w - 1 of one axis; code[i] = -1 where the point is not
+// interior.
+__device__ __forceinline__ void axis_codes(int o, int w, int full, int shift, long long (&code)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const int x = o + i * w;
+    code[i] = x > 0 && x < full ? (long long)(spread3((uint64_t)(x - 1)) << shift) : -1;
+  }
+}
+
+struct Family {
+  int leaves;  // bit k: child k is a leaf
+  long long cx[3], cy[3], cz[3];
+};
+
+__device__ __forceinline__ bool load_family(const int* __restrict__ nd_child, const int4* __restrict__ nd_org,
+                                            long long nf, long long f, int full, Family& fam) {
+  if (f >= nf) return false;
+  fam.leaves = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) fam.leaves |= (nd_child[8 * f + 1 + k] < 0 ? 1 : 0) << k;
+  if (fam.leaves == 0) return false;
+  const int4 o = nd_org[8 * f + 1];
+  axis_codes(o.x, o.w, full, 0, fam.cx);
+  axis_codes(o.y, o.w, full, 1, fam.cy);
+  axis_codes(o.z, o.w, full, 2, fam.cz);
   return true;
 }
 
+// visit(code) for every interior corner of the family's leaves, some of them
+// more than once.
+template <class V>
+__device__ __forceinline__ void family_corners(const Family& fam, const V& visit) {
+  for (int k = 0; k < 8; ++k) {
+    if (!((fam.leaves >> k) & 1)) continue;
+    for (int c = 0; c < 8; ++c) {
+      // lattice index per axis: the child's octant bit plus the corner's
+      const int ix = (k & 1) + (c & 1), iy = ((k >> 1) & 1) + ((c >> 1) & 1), iz = ((k >> 2) & 1) + ((c >> 2) & 1);
+      const long long x = ix == 0 ? fam.cx[0] : ix == 1 ? fam.cx[1] : fam.cx[2];
+      const long long y = iy == 0 ? fam.cy[0] : iy == 1 ? fam.cy[1] : fam.cy[2];
+      const long long z = iz == 0 ? fam.cz[0] : iz == 1 ? fam.cz[1] : fam.cz[2];
+      if (x >= 0 && y >= 0 && z >= 0) visit(x | y | z);
+    }
+  }
+}
+
+// The three points of one axis as bit sets `in` shifted by their low codes,
+// those of equal high code (bits from 5 on) merged into the first: out[i] = 0
+// where point i is merged into another or not interior.
+__device__ __forceinline__ void merge_axis(unsigned in, const long long (&code)[3], unsigned (&out)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) out[i] = code[i] >= 0 ? in << (int)(code[i] & 31) : 0u;
+#pragma unroll
+  for (int i = 1; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < i; ++j)
+      if (out[j] != 0u && out[i] != 0u && (code[j] >> 5) == (code[i] >> 5)) {
+        out[j] |= out[i];
+        out[i] = 0u;
+      }
+}
+
 // used[block] = 1 for every block that holds a corner.
-__global__ void k_block_mark(const int* __restrict__ leaves, long long nl, const int4* __restrict__ nd_org, int full,
+__global__ void k_block_mark(const int* __restrict__ nd_child, long long nf, const int4* __restrict__ nd_org, int full,
                              int bb, int* __restrict__ used) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  uint64_t idx;
-  if (t < nl * 8 && corner_code(leaves, nd_org, full, t, &idx)) used[idx >> bb] = 1;
+  Family fam;
+  if (!load_family(nd_child, nd_org, nf, (long long)blockIdx.x * blockDim.x + threadIdx.x, full, fam)) return;
+  long long last = -1;
+  family_corners(fam, [&](long long code) {
+    const long long b = code >> bb;
+    if (b != last) used[b] = 1;
+    last = b;
+  });
 }
 
 // slot -> block (the inverse of the scan of used)
@@ -168,29 +223,34 @@ __global__ void k_block_list(long long nb, const int* __restrict__ used, const i
   if (b < nb && used[b]) blist[slot[b]] = b;
 }
 
-__global__ void k_corner_mark(const int* __restrict__ leaves, long long nl, const int4* __restrict__ nd_org,
+__global__ void k_corner_mark(const int* __restrict__ nd_child, long long nf, const int4* __restrict__ nd_org,
                               int full, int bb, const int* __restrict__ slot, unsigned* __restrict__ bits) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = threadIdx.x & 31;
-  // one lane per corner; corners of sibling leaves fall in a few bitmap words,
-  // so the warp ORs its bits per word and issues one atomic per word
-  long long word = -1;
-  unsigned bit = 0u;
-  uint64_t idx;
-  if (t < nl * 8 && corner_code(leaves, nd_org, full, t, &idx)) {
-    const uint64_t in_block = idx & ((1ull << bb) - 1ull);
-    const long long blk = slot ? (long long)slot[idx >> bb] : (long long)(idx >> bb);
-    word = (blk << (bb - 5)) + (long long)(in_block >> 5);
-    bit = 1u << (unsigned)(in_block & 31ull);
+  Family fam;
+  if (!load_family(nd_child, nd_org, nf, (long long)blockIdx.x * blockDim.x + threadIdx.x, full, fam)) return;
+  auto mark = [&](long long code, unsigned m) {  // code: of any point of the word
+    const long long blk = slot ? (long long)slot[code >> bb] : code >> bb;
+    atomicOr(bits + (blk << (bb - 5)) + ((code & ((1ll << bb) - 1)) >> 5), m);
+  };
+  if (fam.leaves != 0xff) {
+    family_corners(fam, [&](long long code) { mark(code, 1u << (int)(code & 31)); });
+    return;
   }
-  unsigned todo = __ballot_sync(0xffffffffu, word >= 0);
-  while (todo) {
-    const int leader = __ffs(todo) - 1;
-    const long long lw = __shfl_sync(0xffffffffu, word, leader);
-    const bool mine = word == lw;
-    const unsigned m = __reduce_or_sync(0xffffffffu, mine ? bit : 0u);
-    if (lane == leader && (__ldg(bits + lw) & m) != m) atomicOr(bits + lw, m);
-    todo &= ~__ballot_sync(0xffffffffu, mine);
+  unsigned mx[3];
+  merge_axis(1u, fam.cx, mx);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    if (mx[i] == 0u) continue;
+    unsigned my[3];
+    merge_axis(mx[i], fam.cy, my);
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      if (my[j] == 0u) continue;
+      unsigned mz[3];
+      merge_axis(my[j], fam.cz, mz);
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        if (mz[k] != 0u) mark(fam.cx[i] | fam.cy[j] | fam.cz[k], mz[k]);
+    }
   }
 }
 
@@ -354,10 +414,14 @@ __global__ void k_unique_write(const uint64_t* __restrict__ keys, const int* __r
 }
 
 // One thread per dual vertex (a unique interior leaf corner): the eight leaves
-// around it by descent from the root, the octant of each point deciding the
-// side of a mid-plane that holds it, then the DMC case.
+// around it by descent from the root, then the DMC case.  Octant c of the corner
+// is the lattice cell (x - 1 + bit), ..., and the child that holds a cell at
+// depth d is bit D_max - 1 - d of its coordinates, so a step of the descent
+// loads the child index alone: the nodes' origins, the other half of the loads
+// and half of the instructions, are not needed (1M dam break, 5.8M corners:
+// 336 -> 299 us; what is left is the chain of dependent loads).
 __global__ void k_dual(const uint64_t* __restrict__ verts, long long nu, int B, const int* __restrict__ nd_child,
-                       const int4* __restrict__ nd_org, const float4* __restrict__ nd_v, int* __restrict__ cells,
+                       const float4* __restrict__ nd_v, int* __restrict__ cells,
                        int* __restrict__ procs, int* __restrict__ tcount, unsigned long long* __restrict__ ndual) {
   long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (u > nu) return;
@@ -368,36 +432,32 @@ __global__ void k_dual(const uint64_t* __restrict__ verts, long long nu, int B, 
   const uint64_t key = verts[u];
   const uint64_t m = (1ull << B) - 1ull;
   const int x = (int)((key >> (2 * B)) & m), y = (int)((key >> B) & m), z = (int)(key & m);
-  // the eight octant points share the descent until the node one of whose
-  // mid-planes holds the corner; each octant continues from there
+  // x - 1 and x agree above the lowest set bit of x, so the eight cells share
+  // the descent down to the highest of the three
+  const int split = 31 - __clz((x & -x) | (y & -y) | (z & -z));
+  int bit = B - 2;  // D_max - 1
   int start = 0;
-  for (int guard = 0; guard < 64; ++guard) {
+  for (; bit > split; --bit) {
     const int ch = nd_child[start];
     if (ch < 0) break;
-    const int4 o = nd_org[start];
-    const int mid = o.w >> 1;
-    if (x == o.x + mid || y == o.y + mid || z == o.z + mid) break;
-    start = ch + ((x > o.x + mid) ? 1 : 0) + ((y > o.y + mid) ? 2 : 0) + ((z > o.z + mid) ? 4 : 0);
+    start = ch + (((x >> bit) & 1) | (((y >> bit) & 1) << 1) | (((z >> bit) & 1) << 2));
   }
   // the eight descents below `start` advance in lockstep, so that their
   // loads are in flight together rather than one chain after another
   int n8[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) n8[c] = start;
-  for (int guard = 0; guard < 64; ++guard) {
+  for (; bit >= 0; --bit) {
     int ch[8];
 #pragma unroll
     for (int c = 0; c < 8; ++c) ch[c] = nd_child[n8[c]];
+    const int bx0 = ((x - 1) >> bit) & 1, by0 = (((y - 1) >> bit) & 1) << 1, bz0 = (((z - 1) >> bit) & 1) << 2;
+    const int bx1 = (x >> bit) & 1, by1 = ((y >> bit) & 1) << 1, bz1 = ((z >> bit) & 1) << 2;
     bool more = false;
 #pragma unroll
     for (int c = 0; c < 8; ++c)
       if (ch[c] >= 0) {
-        const int4 o = nd_org[n8[c]];
-        const int mid = o.w >> 1;
-        const int bx = (x > o.x + mid || (x == o.x + mid && (c & 1))) ? 1 : 0;
-        const int by = (y > o.y + mid || (y == o.y + mid && (c & 2))) ? 1 : 0;
-        const int bz = (z > o.z + mid || (z == o.z + mid && (c & 4))) ? 1 : 0;
-        n8[c] = ch[c] + (bx | (by << 1) | (bz << 2));
+        n8[c] = ch[c] + (((c & 1) ? bx1 : bx0) | ((c & 2) ? by1 : by0) | ((c & 4) ? bz1 : bz0));
         more = true;
       }
     if (!more) break;
@@ -618,20 +678,13 @@ struct CountReader {
 static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd) {
   pi_ctx* c = f->ctx;
   const long long nn = f->nNodes;
-  // 1. leaves
-  DBuf<int> flag, leaves, tmp;
-  flag.alloc(c, s, nn + 1);
-  tmp.alloc(c, s, scan_tmp_ints(nn * 8 + 1));
-  exclusive_scan(ScanOf<LeafNode>{{f->nd_child.p}, nn}, flag.p, nn + 1, nullptr, tmp.p, s);
-  rd.start(flag.p + nn);
-  leaves.alloc(c, s, nn > 0 ? nn : 1);  // room for every node
-  PI_LAUNCH(k_leaf_list, div_up(nn, 256), 256, 0, s, f->nd_child.p, flag.p, nn, leaves.p);
-  const long long nl = rd.finish();
-  f->nLeaves = nl;
+  // 1. leaves: every INTERNAL node has eight children, so the counts follow
+  const long long nf = (nn - 1) / 8;  // families
+  f->nLeaves = nn - nf;
+  DBuf<int> tmp;
   // 2. dual vertices = unique interior leaf corners
   const int B = f->dmax + 1;
   const int full = 1 << f->dmax;
-  const long long nk = nl * 8;
   DBuf<uint64_t>& uverts = f->tp_uverts;
   long long nu = 0;
   // block size: 2^bb Morton codes, bb a multiple of 3 and at least 15 (32^3
@@ -641,8 +694,10 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
   const int bb = std::max(15, ((3 * f->dmax - 24 + 2) / 3) * 3);
   if (bb <= 18) {
     const long long nb = 1LL << std::max(0, 3 * f->dmax - bb);
-    // the whole bitmap costs less than finding the used blocks up to 2^30 bits
-    const bool dense = f->dmax <= 10;
+    // up to 2^27 bits (16 MB) clearing and scanning the whole bitmap costs less
+    // than the launches and the read that find the used blocks (40 us at D_max 9
+    // against 60); at 2^30 bits it cost 230 us of a 1.7M-particle frame, the blocks 110
+    const bool dense = f->dmax <= 9;
     long long nused = nb;
     DBuf<int> used, slot;
     DBuf<long long> blist;
@@ -650,7 +705,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
       used.alloc(c, s, nb + 1);
       if (tmp.n < scan_tmp_ints(nb + 1)) tmp.alloc(c, s, scan_tmp_ints(nb + 1));
       PI_CUDA(cudaMemsetAsync(used.p, 0, sizeof(int) * (nb + 1), s));
-      PI_LAUNCH(k_block_mark, div_up(nk, 256), 256, 0, s, leaves.p, nl, f->nd_org.p, full, bb, used.p);
+      PI_LAUNCH(k_block_mark, div_up(nf, 128), 128, 0, s, f->nd_child.p, nf, f->nd_org.p, full, bb, used.p);
       slot.alloc(c, s, nb + 1);
       exclusive_scan_i32(used.p, slot.p, nb + 1, nullptr, tmp.p, s);
       nused = rd.read(slot.p + nb);
@@ -664,7 +719,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     cnt.alloc(c, s, nw + 1);
     if (tmp.n < scan_tmp_ints(nw + 1)) tmp.alloc(c, s, scan_tmp_ints(nw + 1));
     PI_CUDA(cudaMemsetAsync(bits.p, 0, sizeof(unsigned) * (nw > 0 ? nw : 1), s));
-    PI_LAUNCH(k_corner_mark, div_up(nk, 256), 256, 0, s, leaves.p, nl, f->nd_org.p, full, bb,
+    PI_LAUNCH(k_corner_mark, div_up(nf, 128), 128, 0, s, f->nd_child.p, nf, f->nd_org.p, full, bb,
               dense ? nullptr : slot.p, bits.p);
     exclusive_scan(ScanOf<WordBits>{{bits.p}, nw}, cnt.p, nw + 1, nullptr, tmp.p, s);
     nu = rd.read(cnt.p + nw);
@@ -672,6 +727,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     PI_LAUNCH(k_bitmap_keys, div_up(nw, 256), 256, 0, s, bits.p, nw, cnt.p, bb, dense ? nullptr : blist.p, B,
               uverts.p);
   } else {
+    const long long nk = nn * 8;
     const uint64_t invalid = (1ull << (3 * B)) - 1ull;
     DBuf<uint64_t> keys, keys2;
     DBuf<uint32_t> vals, vals2;
@@ -679,7 +735,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     keys2.alloc(c, s, nk);
     vals.alloc(c, s, nk);
     vals2.alloc(c, s, nk);
-    PI_LAUNCH(k_corner_keys, div_up(nk, 256), 256, 0, s, leaves.p, nl, f->nd_org.p, full, B, keys.p, vals.p);
+    PI_LAUNCH(k_corner_keys, div_up(nk, 256), 256, 0, s, f->nd_child.p, nn, f->nd_org.p, full, B, keys.p, vals.p);
     DBuf<int> rtmp;
     rtmp.alloc(c, s, radix_tmp_ints(nk));
     uint64_t *kp = keys.p, *ka = keys2.p;
@@ -687,6 +743,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     radix_sort_u64(&kp, &vp, &ka, &va, nk, 3 * B, rtmp.p, s);
     DBuf<int> uf;
     uf.alloc(c, s, nk + 1);
+    tmp.alloc(c, s, scan_tmp_ints(nk + 1));
     PI_LAUNCH(k_unique_flag, div_up(nk + 1, 256), 256, 0, s, kp, nk, invalid, uf.p);
     exclusive_scan_i32(uf.p, uf.p, nk + 1, nullptr, tmp.p, s);
     nu = rd.read(uf.p + nk);
@@ -746,7 +803,7 @@ void stage_extract(pi_frame* f) {
     counters_snapshot(f, kPinOctree);
   }
   counters_reset(f);
-  PI_LAUNCH(k_dual, div_up(nu + 1, 128), 128, 0, s, uverts, nu, B, f->nd_child.p, f->nd_org.p, f->nd_v.p,
+  PI_LAUNCH(k_dual, div_up(nu + 1, 128), 128, 0, s, uverts, nu, B, f->nd_child.p, f->nd_v.p,
             cells.p, procs.p, toff.p, f->dcount.p);
   exclusive_scan_i32(toff.p, toff.p, nu + 1, nullptr, tmp.p, s);
   const long long nt0 = read_int(f, toff.p + nu);
