@@ -32,11 +32,18 @@
 
 namespace pisurf {
 
-__constant__ int c_trans[256][8];
-__constant__ int c_flip[256];
-__constant__ int c_code[256];
-__constant__ int c_ntri[256];
-__constant__ int c_tri[256][15];
+// The DMC table packed for device reads, one word per sign code: bits 3 c to
+// 3 c + 2 the corner that canonical corner c is, bit 24 the flip, bits 25 to 28
+// the triangles, bit 29 set unless all signs are equal; and the edges (0 to 11,
+// four bits each) of its triangles' corners.  Plain loads: lanes read different
+// entries, which the constant cache would serve one after another (as it did
+// the eight corner words, the code, flip, count and edges of the unpacked
+// table).
+__device__ unsigned d_case[256];
+__device__ unsigned long long d_edges[256];
+constexpr unsigned kCaseFlip = 1u << 24, kCaseMixed = 1u << 29;
+__device__ __forceinline__ int case_corner(unsigned cs, int c) { return (cs >> (3 * c)) & 7; }
+__device__ __forceinline__ int case_triangles(unsigned cs) { return (cs >> 25) & 15; }
 
 void dmc_host_table(int trans[256][8], bool flip[256], int code[256]) {
   DmcTables t;
@@ -55,11 +62,19 @@ static void upload_tables(int device) {
   if (device >= 0 && device < 128 && done[device]) return;
   DmcTables t;
   dmc_build(&t);
-  PI_CUDA(cudaMemcpyToSymbol(c_trans, t.trans, sizeof(t.trans)));
-  PI_CUDA(cudaMemcpyToSymbol(c_flip, t.flip, sizeof(t.flip)));
-  PI_CUDA(cudaMemcpyToSymbol(c_code, t.code, sizeof(t.code)));
-  PI_CUDA(cudaMemcpyToSymbol(c_ntri, t.ntri, sizeof(t.ntri)));
-  PI_CUDA(cudaMemcpyToSymbol(c_tri, t.tri, sizeof(t.tri)));
+  unsigned cs[256];
+  unsigned long long edges[256];
+  for (int i = 0; i < 256; ++i) {
+    const int code = t.code[i];
+    const bool mixed = code != 0 && code != 255;
+    cs[i] = (t.flip[i] ? kCaseFlip : 0u) | (mixed ? kCaseMixed | ((unsigned)t.ntri[code] << 25) : 0u);
+    edges[i] = 0;
+    for (int c = 0; c < 8; ++c) cs[i] |= (unsigned)t.trans[i][c] << (3 * c);
+    if (mixed)
+      for (int k = 0; k < 3 * t.ntri[code]; ++k) edges[i] |= (unsigned long long)t.tri[code][k] << (4 * k);
+  }
+  PI_CUDA(cudaMemcpyToSymbol(d_case, cs, sizeof(cs)));
+  PI_CUDA(cudaMemcpyToSymbol(d_edges, edges, sizeof(edges)));
   if (device >= 0 && device < 128) done[device] = true;
 }
 
@@ -285,6 +300,11 @@ __device__ __forceinline__ uint32_t mix64to32(uint64_t k) {
 // per distinct key keeps the lowest slot (atomicMin), keys are compared
 // through the slots' own key arrays.  The table has more entries than
 // slots, so a probe always ends.
+// An entry is lowered only where this slot is below what it holds (it never
+// rises, so a stale read costs an atomic and nothing else): most of a key's six
+// slots come after its first.  195 -> 168 us for the 12.9M slots of a 1M
+// dam-break frame.  Homes that follow the leaf ids, so that neighbours share
+// lines, were slower (212 us: the probes of near keys run into one another).
 __global__ void k_vkey_insert(long long ns, const uint64_t* __restrict__ khi, const uint64_t* __restrict__ klo,
                               uint32_t mask, unsigned* __restrict__ tab, uint32_t* __restrict__ where) {
   long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -299,7 +319,7 @@ __global__ void k_vkey_insert(long long ns, const uint64_t* __restrict__ khi, co
     }
     const long long o = (long long)cur - 1;
     if (klo[o] == lo && (!khi || khi[o] == hi)) {
-      atomicMin(tab + h, (unsigned)s + 1u);
+      if ((unsigned)s + 1u < cur) atomicMin(tab + h, (unsigned)s + 1u);  // the entry only ever falls
       break;
     }
     h = (h + 1u) & mask;
@@ -321,9 +341,9 @@ __global__ void k_tri_insert(long long nt, const int* __restrict__ otri, uint32_
   if (t >= nt) return;
   int s0, s1, s2;
   sorted3(otri + 3 * t, s0, s1, s2);
-  uint32_t h = mix64to32(((uint64_t)(uint32_t)s0 << 42) ^ ((uint64_t)(uint32_t)s1 << 21) ^ (uint64_t)(uint32_t)s2 ^
-                         ((uint64_t)(uint32_t)s0 >> 22) * 0x9E3779B97F4A7C15ull) &
-               mask;
+  // homes by the lowest vertex, whose triangles are near in the list: 109 us
+  // scattered by a full mix, 91 us this way (4.3M triangles)
+  uint32_t h = ((uint32_t)s0 * 4u + (mix64to32(((uint64_t)(uint32_t)s1 << 32) | (uint32_t)s2) & 3u)) & mask;
   for (uint32_t i = 0; i <= mask; ++i) {
     unsigned cur = tab[h];
     if (cur == 0u) {
@@ -333,7 +353,7 @@ __global__ void k_tri_insert(long long nt, const int* __restrict__ otri, uint32_
     int o0, o1, o2;
     sorted3(otri + 3 * ((long long)cur - 1), o0, o1, o2);
     if (o0 == s0 && o1 == s1 && o2 == s2) {
-      atomicMin(tab + h, (unsigned)t + 1u);
+      if ((unsigned)t + 1u < cur) atomicMin(tab + h, (unsigned)t + 1u);
       break;
     }
     h = (h + 1u) & mask;
@@ -419,10 +439,10 @@ __global__ void k_unique_write(const uint64_t* __restrict__ keys, const int* __r
 // depth d is bit D_max - 1 - d of its coordinates, so a step of the descent
 // loads the child index alone: the nodes' origins, the other half of the loads
 // and half of the instructions, are not needed (1M dam break, 5.8M corners:
-// 336 -> 299 us; what is left is the chain of dependent loads).
+// 336 -> 299 us; 187 with the table in plain loads).
 __global__ void k_dual(const uint64_t* __restrict__ verts, long long nu, int B, const int* __restrict__ nd_child,
                        const float4* __restrict__ nd_v, int* __restrict__ cells,
-                       int* __restrict__ procs, int* __restrict__ tcount, unsigned long long* __restrict__ ndual) {
+                       uint8_t* __restrict__ procs, int* __restrict__ tcount, unsigned long long* __restrict__ ndual) {
   long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (u > nu) return;
   if (u == nu) {
@@ -466,46 +486,61 @@ __global__ void k_dual(const uint64_t* __restrict__ verts, long long nu, int B, 
 #pragma unroll
   for (int c = 0; c < 8; ++c)
     if (nd_v[n8[c]].w > 0.f) index |= 1 << c;
-  const int code = c_code[index];
-  int nt = 0;
-  if (code != 0 && code != 255) {
-    nt = c_ntri[code];
-    for (int c = 0; c < 8; ++c) cells[8 * u + c] = n8[c_trans[index][c]];
+  const unsigned cs = __ldg(d_case + index);
+  if (cs & kCaseMixed) {
+    int4* const out = reinterpret_cast<int4*>(cells + 8 * u);
+    out[0] = make_int4(n8[0], n8[1], n8[2], n8[3]);
+    out[1] = make_int4(n8[4], n8[5], n8[6], n8[7]);
     stripe_add(ndual, C_DUAL, 1ull);
   }
-  procs[u] = index;
-  tcount[u] = nt;
+  procs[u] = (uint8_t)index;
+  tcount[u] = (cs & kCaseMixed) ? case_triangles(cs) : 0;
 }
 
-__global__ void k_tri_slots(long long nu, const int* __restrict__ cells, const int* __restrict__ procs,
-                            const int* __restrict__ toff, const uint64_t* __restrict__ nd_id, int id_bits,
-                            int packed, int* __restrict__ slotA, int* __restrict__ slotB,
-                            uint64_t* __restrict__ khi, uint64_t* __restrict__ klo, int8_t* __restrict__ tflip) {
-  long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (u >= nu) return;
-  const int index = procs[u];
-  const int code = c_code[index];
-  if (code == 0 || code == 255) return;
-  const int nt = c_ntri[code];
-  const long long t0 = toff[u];
-  for (int t = 0; t < nt; ++t) {
-    tflip[t0 + t] = (int8_t)c_flip[index];
-    for (int k = 0; k < 3; ++k) {
-      int c0, c1;
-      edge_corners(c_tri[code][3 * t + k], &c0, &c1);
-      const int A = cells[8 * u + c0], Bn = cells[8 * u + c1];
-      const long long s = 3 * (t0 + t) + k;
-      slotA[s] = A;
-      slotB[s] = Bn;
-      uint64_t ia = nd_id[A], ib = nd_id[Bn];
-      uint64_t lo = ia < ib ? ia : ib, hi = ia < ib ? ib : ia;
-      if (packed) {
-        klo[s] = (lo << id_bits) | hi;
-      } else {
-        khi[s] = lo;
-        klo[s] = hi;
-      }
+// Triangle slots: the two leaves each triangle corner bisects and their sorted
+// id pair.  The slots of a block's dual vertices are one run, so a thread takes
+// every kSlotThreads-th slot of it, finds its dual vertex in the block's offsets,
+// and the stores of a warp are contiguous (a thread per dual vertex stored up to
+// 15 slots of its own, a line each: 160 us at 1M, 109 this way).
+constexpr int kSlotThreads = 256;
+__global__ void __launch_bounds__(kSlotThreads) k_tri_slots(long long nu, const int* __restrict__ cells,
+                                                            const uint8_t* __restrict__ procs,
+                                                            const int* __restrict__ toff,
+                                                            const uint64_t* __restrict__ nd_id, int id_bits, int packed,
+                                                            int* __restrict__ slotA, int* __restrict__ slotB,
+                                                            uint64_t* __restrict__ khi, uint64_t* __restrict__ klo,
+                                                            int8_t* __restrict__ tflip) {
+  __shared__ int s_off[kSlotThreads + 1];
+  const long long u0 = (long long)blockIdx.x * kSlotThreads;
+  const int nloc = (int)(nu - u0 < kSlotThreads ? nu - u0 : kSlotThreads);
+  for (int i = threadIdx.x; i <= kSlotThreads; i += kSlotThreads) s_off[i] = toff[u0 + min(i, nloc)];
+  __syncthreads();
+  const int first = s_off[0], total = 3 * (s_off[kSlotThreads] - first);
+  for (int q = threadIdx.x; q < total; q += kSlotThreads) {
+    const int t = first + q / 3, k = q % 3;
+    int i = 0;  // the last vertex whose triangles start at or before t
+#pragma unroll
+    for (int o = kSlotThreads / 2; o > 0; o >>= 1)
+      if (s_off[i + o] <= t) i += o;
+    const long long u = u0 + i;
+    const int index = procs[u];
+    const unsigned cs = __ldg(d_case + index);
+    const int e = (int)(__ldg(d_edges + index) >> (4 * (3 * (t - s_off[i]) + k))) & 15;
+    int c0, c1;
+    edge_corners(e, &c0, &c1);
+    const int A = __ldg(cells + 8 * u + case_corner(cs, c0)), Bn = __ldg(cells + 8 * u + case_corner(cs, c1));
+    const long long s = 3ll * first + q;
+    slotA[s] = A;
+    slotB[s] = Bn;
+    const uint64_t ia = __ldg(nd_id + A), ib = __ldg(nd_id + Bn);
+    const uint64_t lo = ia < ib ? ia : ib, hi = ia < ib ? ib : ia;
+    if (packed) {
+      klo[s] = (lo << id_bits) | hi;
+    } else {
+      khi[s] = lo;
+      klo[s] = hi;
     }
+    if (k == 0) tflip[t] = (cs & kCaseFlip) ? 1 : 0;
   }
 }
 
@@ -791,7 +826,8 @@ void stage_extract(pi_frame* f) {
   DBuf<int> tmp;
   tmp.alloc(c, s, scan_tmp_ints(nu + 1));
   // 3. dual cells
-  DBuf<int> cells, procs, toff;
+  DBuf<int> cells, toff;
+  DBuf<int8_t> procs;
   cells.alloc(c, s, nu * 8 > 0 ? nu * 8 : 1);
   procs.alloc(c, s, nu > 0 ? nu : 1);
   toff.alloc(c, s, nu + 1);
@@ -804,7 +840,7 @@ void stage_extract(pi_frame* f) {
   }
   counters_reset(f);
   PI_LAUNCH(k_dual, div_up(nu + 1, 128), 128, 0, s, uverts, nu, B, f->nd_child.p, f->nd_v.p,
-            cells.p, procs.p, toff.p, f->dcount.p);
+            cells.p, reinterpret_cast<uint8_t*>(procs.p), toff.p, f->dcount.p);
   exclusive_scan_i32(toff.p, toff.p, nu + 1, nullptr, tmp.p, s);
   const long long nt0 = read_int(f, toff.p + nu);
   // 4. triangle slots and vertex keys (sorted leaf-id pairs)
@@ -819,8 +855,9 @@ void stage_extract(pi_frame* f) {
   klo.alloc(c, s, ns > 0 ? ns : 1);
   if (!packed) khi.alloc(c, s, ns > 0 ? ns : 1);
   tflip.alloc(c, s, nt0 > 0 ? nt0 : 1);
-  PI_LAUNCH(k_tri_slots, div_up(nu, 128), 128, 0, s, nu, cells.p, procs.p, toff.p, f->nd_id.p, id_bits, packed,
-            slotA.p, slotB.p, khi.p, klo.p, tflip.p);
+  PI_LAUNCH(k_tri_slots, div_up(nu, kSlotThreads), kSlotThreads, 0, s, nu, cells.p,
+            reinterpret_cast<const uint8_t*>(procs.p), toff.p, f->nd_id.p, id_bits, packed, slotA.p, slotB.p, khi.p,
+            klo.p, tflip.p);
   cells.release();
   procs.release();
   toff.release();
