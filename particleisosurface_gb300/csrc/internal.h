@@ -55,7 +55,6 @@ struct GridHost {
   int nx, ny, nz;
   long long cellNum;
   int nInvalid;
-  int bits;  // radix sort width for key+1
 };
 
 // Configurations of the chunked field evaluation at octree samples
@@ -130,7 +129,6 @@ struct pi_frame {
   pisurf::DBuf<unsigned> misc;   // small scalars: bbox encodings, counters
   pisurf::DBuf<int> key;         // N, original order, -1 outside the grid
   pisurf::DBuf<uint32_t> sidx;   // N, IndexList: sorted position -> particle
-  pisurf::DBuf<uint32_t> skey;   // N, sorted key+1
   pisurf::DBuf<int> off;         // C+1 cell offsets
   pisurf::DBuf<float4> pos, xm, ga, gb, nrm;  // N, sorted order
   pisurf::DBuf<float4> xlo;      // N, sorted order: centre minus its float rounding
@@ -169,7 +167,7 @@ struct pi_frame {
   pisurf::DBuf<int8_t> spl64;   // splash flags decided in double (splash mode)
   bool f64_ready = false;
   pisurf::DBuf<int> tmp;         // scan / sort scratch
-  pisurf::DBuf<uint32_t> u32a, u32b, u32c;  // sort ping-pong scratch
+  pisurf::DBuf<uint32_t> u32a, u32b, u32c;  // scratch of the cell sort
 
   // scalars (Evaluator / SurfReconstructor members)
   float iso = 0, maxScalar = -1, influ2 = 0, sigma = 0;

@@ -291,7 +291,6 @@ void stage_hashgrid_vr(pi_frame* f) {
   gh.nx = b0.nx, gh.ny = b0.ny, gh.nz = b0.nz;
   gh.cellNum = b0.cellNum;
   gh.nInvalid = 0;
-  gh.bits = kbits + gbits;
   PI_CUDA(cudaStreamSynchronize(s));
 }
 
