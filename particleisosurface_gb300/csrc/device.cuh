@@ -167,6 +167,43 @@ __device__ __forceinline__ float field_sum(const GridView& g, const PartView& P,
   return acc.s;
 }
 
+// The same sum for one point held by the whole warp: 32 candidates of a row at
+// a time, a lane each, then the terms added in candidate order (every lane keeps
+// the sum).  The chain of one point is a tenth of a lane's alone.
+__device__ __forceinline__ float field_sum_warp(const GridView& g, const PartView& P, float qx, float qy, float qz) {
+  const int lane = threadIdx.x & 31;
+  int cx, cy, cz;
+  cell_of(g, qx, qy, qz, cx, cy, cz);
+  Kahan acc;
+  for (int dz = -1; dz <= 1; ++dz)
+    for (int dy = -1; dy <= 1; ++dy) {
+      int s, e;
+      if (!nb_row(g, cx, cy + dy, cz + dz, &s, &e)) continue;
+      for (int j0 = s; j0 < e; j0 += 32) {
+        const int j = j0 + lane;
+        bool in = false;
+        float term = 0.f;
+        if (j < e) {
+          const float4 x = __ldg(P.xm + j);
+          const float dx = qx - x.x, dyy = qy - x.y, dzz = qz - x.z;
+          if (fmaf(dx, dx, fmaf(dyy, dyy, dzz * dzz)) < x.w) {
+            const float4 a = __ldg(P.ga + j);
+            const float4 b = __ldg(P.gb + j);
+            const float4 lo = __ldg(P.xlo + j);
+            float u0, u1, u2;
+            amul(a, b, dx - lo.x, dyy - lo.y, dzz - lo.z, u0, u1, u2);
+            const float s2 = fmaf(u0, u0, fmaf(u1, u1, u2 * u2));
+            in = s2 < 4.0f;
+            if (in) term = b.z * bspline_s2(s2);
+          }
+        }
+        for (unsigned m = __ballot_sync(0xffffffffu, in); m; m &= m - 1u)
+          acc.add(__shfl_sync(0xffffffffu, term, __ffs(m) - 1));
+      }
+    }
+  return acc.s;
+}
+
 // ---------------------------------------------------------------------------
 // Variable radius: the particles binned by radius (MultiLevelSearcher,
 // src/multi_level_reseacher.cpp:6-77), one hash grid per non-empty bin with

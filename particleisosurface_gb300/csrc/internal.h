@@ -187,7 +187,9 @@ struct pi_frame {
   pisurf::DBuf<float> nd_curv;
   pisurf::DBuf<int4> nd_org;     // integer origin at depth-max resolution, size
   pisurf::DBuf<float> nd_samp;   // 27 sample values per node (QEF mode)
-  pisurf::DBuf<int8_t> npart;    // leaf level in QEF mode: each node's part (read by the QEF stream too)
+  // leaf level in QEF mode: its nodes part by part, and the parts' counts,
+  // cursors and starts in that list (both read by the QEF stream too)
+  pisurf::DBuf<int> pnodes, plist;
 
   // mesh
   long long nV = 0, nT = 0, nDual = 0;
@@ -273,9 +275,12 @@ void stage_extract(pi_frame* f);
 // after the anisotropy pass; the icosahedra at vertex v0 and triangle t0.
 void stage_splash_list(pi_frame* f);
 void splash_mesh(pi_frame* f, long long v0, long long t0);
-// QEF vertices of the leaves of level [lb, le); scratch holds at least
-// le - lb + 1 ints (device memory the caller no longer needs).
-void qef_level(pi_frame* f, long long lb, long long le, int depth, const int8_t* npart = nullptr, int part = 0);
+// QEF vertices of the leaves of level [lb, le); with parts > 0 those of part
+// `part`, whose nodes (all leaves) the frame lists.
+void qef_level(pi_frame* f, long long lb, long long le, int depth, int parts = 0, int part = 0);
+// Threads for the nodes of one of `parts` parts: twice the mean, at most all
+// (kernels over a part stride, so a larger part is only slower).
+inline long long part_share(long long nl, int parts) { return parts > 1 ? 2 * nl / parts + 256 : nl; }
 // The context stream waits for the QEF work in flight (no host wait).
 void qef_join(pi_frame* f);
 // The extraction's topology on the topology stream, after the context

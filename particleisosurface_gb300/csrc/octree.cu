@@ -419,12 +419,48 @@ __device__ __forceinline__ int part_of(const int* __restrict__ kb, int parts, in
 // octant bits grow with the coordinates, and the key orders them z, y, x,
 // then the octant's z, y, x bits.  So all of a node's samples are evaluated
 // once the parts up to its own are.  -1 for a node with no samples.
-__global__ void k_node_part(long long nl, const int* __restrict__ qkey, const int* __restrict__ pinfo, int parts,
-                            int8_t* __restrict__ npart) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nl) return;
-  const int k = qkey[t * kQ + 26];
-  npart[t] = k < 0 ? (int8_t)-1 : (int8_t)part_of(pinfo, parts, k);
+// plist: the nodes per part (counts here), their cursors and starts, parts + 1
+// words each.
+constexpr int kPartThreads = 256;
+__global__ void __launch_bounds__(kPartThreads) k_node_part(long long nl, const int* __restrict__ qkey,
+                                                            const int* __restrict__ pinfo, int parts,
+                                                            int8_t* __restrict__ npart, int* __restrict__ plist) {
+  __shared__ int s_count[kMaxQefParts];
+  const long long t = (long long)blockIdx.x * kPartThreads + threadIdx.x;
+  if (threadIdx.x < kMaxQefParts) s_count[threadIdx.x] = 0;
+  __syncthreads();
+  if (t < nl) {
+    const int k = qkey[t * kQ + 26];
+    const int p = k < 0 ? -1 : part_of(pinfo, parts, k);
+    npart[t] = (int8_t)p;
+    if (p >= 0) atomicAdd(&s_count[p], 1);
+  }
+  __syncthreads();
+  if (threadIdx.x < (unsigned)parts && s_count[threadIdx.x] > 0) atomicAdd(plist + threadIdx.x, s_count[threadIdx.x]);
+}
+
+// The nodes listed part by part (in blocks of nodes, so that a part's list runs
+// through the level in long strides): each part's classification and QEF touch
+// its own nodes only.  A pass over the whole level per part cost 50 us for the
+// classification and 15 for the leaf list, 1 ms of a 16-part 1M frame.
+__global__ void __launch_bounds__(kPartThreads) k_part_list(long long nl, int parts, const int8_t* __restrict__ npart,
+                                                            int* __restrict__ plist, int* __restrict__ list) {
+  __shared__ int s_count[kMaxQefParts], s_base[kMaxQefParts];
+  const long long t = (long long)blockIdx.x * kPartThreads + threadIdx.x;
+  if (threadIdx.x < kMaxQefParts) s_count[threadIdx.x] = 0;
+  __syncthreads();
+  const int p = t < nl ? npart[t] : -1;
+  const int mine = p >= 0 ? atomicAdd(&s_count[p], 1) : 0;
+  __syncthreads();
+  if (threadIdx.x < (unsigned)parts) {
+    int start = 0;
+    for (int q = 0; q < (int)threadIdx.x; ++q) start += plist[q];
+    if (blockIdx.x == 0) plist[2 * (parts + 1) + threadIdx.x] = start;
+    const int n = s_count[threadIdx.x];
+    s_base[threadIdx.x] = start + (n > 0 ? atomicAdd(plist + parts + 1 + threadIdx.x, n) : 0);
+  }
+  __syncthreads();
+  if (p >= 0) list[s_base[p] + mine] = (int)t;
 }
 
 // k_q_chunks with the chunks of part p in the region [pb[p], pb[p + 1]) of
@@ -687,44 +723,72 @@ __global__ void __launch_bounds__(64, 24) k_classify(LevelArgs a, const float* _
 }
 
 // k_classify for a level that needs no particle scan: its nodes are leaves
-// by size, or their curvature was summed by the parents' scan.  One thread
-// per node gathers its 28 values (independent loads in flight together)
-// instead of a warp per node; the decisions and values are k_classify's.
+// by size, or their curvature was summed by the parents' scan.  The decisions
+// and values are k_classify's.  With plist, only the nodes of part `part`, from
+// the list.
+//
+// A block takes kClassifyNodes nodes: its threads read the nodes' runs of 28
+// representatives and gather their values side by side into shared memory, a
+// thread decides per node, and the 27 sample values of the QEF go out as
+// contiguous runs again.  Scattered 4-byte stores and loads bound it (a thread
+// per node reading and writing its own runs: 52 us for a sixteenth of the 4.2M
+// leaf-level nodes of a 1M frame; 50 this way, and the frame 0.6 ms less).
+constexpr int kClassifyNodes = 128;
+constexpr int kRunPad = kQ + 1;  // odd stride: a thread per node reads without bank conflicts
 __global__ void __launch_bounds__(256) k_classify_thread(LevelArgs a, const float* __restrict__ qval,
                                                          const int* __restrict__ rep, const float4* __restrict__ nd_c,
                                                          float4* __restrict__ nd_v, int8_t* __restrict__ nd_type,
                                                          int8_t* __restrict__ nd_sc, float* __restrict__ nd_curv,
                                                          float* __restrict__ nd_samp, int qef,
                                                          unsigned long long* __restrict__ counters,
-                                                         const int8_t* __restrict__ npart, int part) {
-  const long long node = a.lb + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+                                                         const int* __restrict__ plist, const int* __restrict__ list,
+                                                         int parts, int part) {
+  __shared__ float s_val[kClassifyNodes * kRunPad];
+  __shared__ int s_node[kClassifyNodes];  // node - lb, -1: none or no samples
+  const long long n = plist ? plist[part] : a.le - a.lb;
+  if (plist) list += plist[2 * (parts + 1) + part];
   unsigned long long evals = 0;
-  if (node < a.le && (!npart || npart[node - a.lb] == part) && nd_type[node] == T_UNCERTAIN) {
-    const long long qb = (node - a.lb) * kQ;
-    float val[kQ];
-#pragma unroll
-    for (int q = 0; q < kQ; ++q) val[q] = qval[__ldg(rep + qb + q)];
-    // GridEval sign change against sample 0, ">= 0" (src/evaluator.cpp:169-172)
-    const bool origin = val[0] >= 0.f;
-    bool signchange = false;
-#pragma unroll
-    for (int q = 1; q < 27; ++q) signchange |= (val[q] >= 0.f) != origin;
-    if (qef)
-#pragma unroll
-      for (int q = 0; q < 27; ++q) nd_samp[node * 27 + q] = val[q];
-    const float4 c = nd_c[node];
-    const float cellsize = 2.0f * c.w;
-    const bool leaf_by_size = cellsize - a.radius < kAbove1em8;
-    int8_t type = T_LEAF;
-    if (!leaf_by_size && signchange && nd_curv[node] < kAbove099) type = T_INTERNAL;
-    nd_type[node] = type;
-    nd_sc[node] = signchange ? 1 : 0;
-    if (type == T_LEAF) {
-      float4 v = nd_v[node];
-      v.w = val[27];
-      nd_v[node] = v;
+  for (long long t0 = (long long)blockIdx.x * kClassifyNodes; t0 < n; t0 += (long long)gridDim.x * kClassifyNodes) {
+    if (threadIdx.x < kClassifyNodes) {
+      const long long t = t0 + threadIdx.x;
+      int node = t < n ? (plist ? list[t] : (int)t) : -1;
+      if (node >= 0 && nd_type[a.lb + node] != T_UNCERTAIN) node = -1;
+      s_node[threadIdx.x] = node;
     }
-    evals = 27 + (type == T_LEAF ? 1 : 0);
+    __syncthreads();
+    for (int i = threadIdx.x; i < kClassifyNodes * kQ; i += 256) {
+      const int k = i / kQ, q = i % kQ, node = s_node[k];
+      if (node >= 0) s_val[k * kRunPad + q] = qval[__ldg(rep + (long long)node * kQ + q)];
+    }
+    __syncthreads();
+    if (threadIdx.x < kClassifyNodes && s_node[threadIdx.x] >= 0) {
+      const long long node = a.lb + s_node[threadIdx.x];
+      const float* val = s_val + threadIdx.x * kRunPad;
+      // GridEval sign change against sample 0, ">= 0" (src/evaluator.cpp:169-172)
+      const bool origin = val[0] >= 0.f;
+      bool signchange = false;
+#pragma unroll
+      for (int q = 1; q < 27; ++q) signchange |= (val[q] >= 0.f) != origin;
+      const float4 c = nd_c[node];
+      const float cellsize = 2.0f * c.w;
+      const bool leaf_by_size = cellsize - a.radius < kAbove1em8;
+      int8_t type = T_LEAF;
+      if (!leaf_by_size && signchange && nd_curv[node] < kAbove099) type = T_INTERNAL;
+      nd_type[node] = type;
+      nd_sc[node] = signchange ? 1 : 0;
+      if (type == T_LEAF) {
+        float4 v = nd_v[node];
+        v.w = val[27];
+        nd_v[node] = v;
+      }
+      evals += 27 + (type == T_LEAF ? 1 : 0);
+    }
+    if (qef)
+      for (int i = threadIdx.x; i < kClassifyNodes * 27; i += 256) {
+        const int k = i / 27, q = i % 27, node = s_node[k];
+        if (node >= 0) nd_samp[(a.lb + node) * 27 + q] = s_val[k * kRunPad + q];
+      }
+    __syncthreads();
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) evals += __shfl_xor_sync(0xffffffffu, evals, o);
@@ -1205,22 +1269,24 @@ static void eval_chunks(pi_frame* f, int cfg, const QArgs& qa, long long qn, con
 }
 
 static void dense_eval(pi_frame* f, int cfg, const QArgs& qa, long long qn, long long nbuckets, const int* order,
-                       const int* qoff, const int* ucnt, int2* chunks, int* nchunks, float* qval,
+                       const int* qoff, const int* ucnt, int2* chunks, int* nchunks, int reserve, float* qval,
                        unsigned long long* counters) {
   cudaStream_t s = f->ctx->stream;
   const int K = kEvalTable[cfg].K;
   PI_CUDA(cudaMemsetAsync(nchunks, 0, sizeof(int), s));
   PI_LAUNCH(k_q_chunks, div_up(nbuckets, 256), 256, 0, s, nbuckets, ucnt, 32 * K, chunks, nchunks);
-  eval_chunks(f, cfg, qa, qn, order, qoff, ucnt, chunks, nchunks, nullptr, 0, qval, counters);
+  eval_chunks(f, cfg, qa, qn, order, qoff, ucnt, chunks, nchunks, nullptr, reserve, qval, counters);
 }
 
 // Configuration for a dense level of the given kind: the context's choice,
 // or, the first time, the fastest of the table timed on this level (the
-// evaluation is pure, so the runs give identical values).  A context whose K
+// evaluation is pure, so the runs give identical values; with the registers per
+// SM that the level's launches will leave free: a large block that fits twice
+// without them may fit once).  A context whose K
 // is fixed (pi_ctx_tune) runs that K with the default W and CB.
 static int eval_config_for(pi_frame* f, int kind, const QArgs& qa, long long qn, long long nbuckets,
                            const int* order, const int* qoff, const int* ucnt, int2* chunks, int* nchunks,
-                           float* qval) {
+                           int reserve, float* qval) {
   pi_ctx* ctx = f->ctx;
   if (ctx->eval_forced) return ctx->eval_forced == 1 ? 0 : ctx->eval_forced == 2 ? 1 : 2;
   if (ctx->eval_cfg[kind]) return ctx->eval_cfg[kind] - 1;
@@ -1235,7 +1301,7 @@ static int eval_config_for(pi_frame* f, int kind, const QArgs& qa, long long qn,
   scratch.alloc(ctx, s, kCounterWords);
   for (int c = 0; c < kEvalConfigs; ++c) {
     PI_CUDA(cudaEventRecord(e0, s));
-    dense_eval(f, c, qa, qn, nbuckets, order, qoff, ucnt, chunks, nchunks, qval, scratch.p);
+    dense_eval(f, c, qa, qn, nbuckets, order, qoff, ucnt, chunks, nchunks, reserve, qval, scratch.p);
     PI_CUDA(cudaEventRecord(e1, s));
     PI_CUDA(cudaEventSynchronize(e1));
     float ms = 0.f;
@@ -1765,21 +1831,28 @@ void stage_octree(pi_frame* f) {
         exclusive_scan_i32(ucnt.p, ucum.p, nb + 1, nullptr, f->tmp.p, s);
         PI_LAUNCH(k_q_compact, div_up(qn, 256), 256, 0, s, qn, qkey.p, order.p, ucum.p, list);
       }
+      const bool in_parts = dense && f->P.qef && depth == f->dmax && ctx->qef_parts > 1;
       int cfg = 0;
       if (dense)
         cfg = eval_config_for(f, depth == f->dmax ? 0 : 1, qa, qn, nb, order.p, qcnt.p, ucnt.p, chunks.p,
-                              qcnt.p + nb + 1, qval.p);
-      if (dense && f->P.qef && depth == f->dmax && ctx->qef_parts > 1) {
+                              qcnt.p + nb + 1, in_parts ? kQefReserveRegs : 0, qval.p);
+      if (in_parts) {
         // the leaf level in parts: part p's QEF beside part p + 1's sampling
         const int parts = ctx->qef_parts;
         DBuf<int> pinfo;
         pinfo.alloc(ctx, s, 3 * (parts + 1));
-        // the frame's array, so that it outlives the QEF stream's reads (the
-        // QEF of this frame's coarser levels never reads it)
-        DBuf<int8_t>& npart = f->npart;
-        if (npart.n < (size_t)nl) npart.alloc(ctx, s, nl);
+        DBuf<int8_t> npart;
+        npart.alloc(ctx, s, nl);
+        // the frame's arrays, so that they outlive the QEF stream's reads (the
+        // QEF of this frame's coarser levels never reads them)
+        if (f->plist.n < (size_t)(3 * (kMaxQefParts + 1))) f->plist.alloc(ctx, s, 3 * (kMaxQefParts + 1));
+        if (f->pnodes.n < (size_t)nl) f->pnodes.alloc(ctx, s, nl);
+        PI_CUDA(cudaMemsetAsync(f->plist.p, 0, sizeof(int) * 3 * (parts + 1), s));
         PI_LAUNCH(k_part_bounds, 1, 128, 0, s, qcnt.p, (int)nb, parts, pinfo.p);
-        PI_LAUNCH(k_node_part, div_up(nl, 256), 256, 0, s, nl, qkey.p, pinfo.p, parts, npart.p);
+        PI_LAUNCH(k_node_part, div_up(nl, kPartThreads), kPartThreads, 0, s, nl, qkey.p, pinfo.p, parts, npart.p,
+                  f->plist.p);
+        PI_LAUNCH(k_part_list, div_up(nl, kPartThreads), kPartThreads, 0, s, nl, parts, npart.p, f->plist.p,
+                  f->pnodes.p);
         PI_LAUNCH(k_q_chunks_parts, div_up(nb, 256), 256, 0, s, nb, ucnt.p, 32 * kEvalTable[cfg].K, parts, pinfo.p,
                   chunks.p);
         for (int p = 0; p < parts; ++p) {
@@ -1789,24 +1862,28 @@ void stage_octree(pi_frame* f) {
           eval_chunks(f, cfg, qa, qn, order.p, qcnt.p, ucnt.p, chunks.p, pinfo.p + 2 * (parts + 1) + p,
                       pinfo.p + parts + 1 + p, kQefReserveRegs, qval.p, f->dcount.p);
           prof_end(ctx, s, PG_CHUNK);
-          PI_LAUNCH(k_classify_thread, div_up(nl, 256), 256, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
-                    f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p,
-                    (const int8_t*)npart.p, p);
-          qef_level(f, lb, le, depth, npart.p, p);
+          // a part holds about nl / parts nodes; the blocks stride over what it
+          // holds.  (Classified on the QEF stream, in front of the part's QEF,
+          // the frame was 0.8 ms slower: the next part's evaluator takes the SMs
+          // first and the part's QEF starts late.)
+          PI_LAUNCH(k_classify_thread, div_up(part_share(nl, parts), kClassifyNodes), 256, 0, s, la, qval.p, rep.p,
+                    f->nd_c.p, f->nd_v.p, f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p,
+                    (const int*)f->plist.p, (const int*)f->pnodes.p, parts, p);
+          qef_level(f, lb, le, depth, parts, p);
         }
       } else {
       const int pg = dense ? PG_CHUNK : PG_THREAD;
       prof_begin(ctx, s, pg);
       if (dense)
-        dense_eval(f, cfg, qa, qn, nb, order.p, qcnt.p, ucnt.p, chunks.p, qcnt.p + nb + 1, qval.p, f->dcount.p);
+        dense_eval(f, cfg, qa, qn, nb, order.p, qcnt.p, ucnt.p, chunks.p, qcnt.p + nb + 1, 0, qval.p, f->dcount.p);
       else
         PI_LAUNCH(k_q_eval_thread, (int)std::min<long long>((long long)ctx->smCount * 8, div_up(qn, 256)), 256, 0,
                   s, qa, list, ucum.p + nb, f->nd_c.p, f->nd_v.p, qval.p, f->dcount.p);
       prof_end(ctx, s, pg);
       if (known || leaf_level)  // no node needs a particle scan
-        PI_LAUNCH(k_classify_thread, div_up(nl, 256), 256, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
-                  f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p,
-                  (const int8_t*)nullptr, 0);
+        PI_LAUNCH(k_classify_thread, div_up(nl, kClassifyNodes), 256, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
+                  f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p, (const int*)nullptr,
+                  (const int*)nullptr, 0, 0);
       else
         PI_LAUNCH(k_classify, div_up(nl, wpb), 32 * wpb, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
                   f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, known ? 1 : 0, f->dcount.p,
