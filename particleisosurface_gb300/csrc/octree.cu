@@ -385,7 +385,8 @@ __global__ void k_q_chunks(long long nb, const int* __restrict__ ucnt, int chunk
 // qoff (qoff[nb] slots in all) crosses p / parts of the total.  pinfo holds
 // kb[0 .. parts] (first bucket of each part), pb[0 .. parts] (chunk region of
 // each part: qoff[kb[p]], since a part never has more chunks than sample
-// slots) and the chunk counts cnt[0 .. parts - 1].
+// slots), the chunk counts cnt[0 .. parts - 1] and the chunks taken by the
+// evaluation's warps.
 __global__ void k_part_bounds(const int* __restrict__ qoff, int nb, int parts, int* __restrict__ pinfo) {
   const int p = threadIdx.x;
   if (p > parts) return;
@@ -404,7 +405,7 @@ __global__ void k_part_bounds(const int* __restrict__ qoff, int nb, int parts, i
   }
   pinfo[p] = k;
   pinfo[parts + 1 + p] = qoff[k];
-  if (p < parts) pinfo[2 * (parts + 1) + p] = 0;
+  if (p < parts) pinfo[2 * (parts + 1) + p] = pinfo[3 * (parts + 1) + p] = 0;
 }
 
 // Part of a bucket key (kb increasing, kb[0] = 0, kb[parts] = nb).
@@ -492,8 +493,8 @@ __global__ void k_q_chunks_parts(long long nb, const int* __restrict__ ucnt, int
   for (int j = 0; j < c; ++j) chunks[base + j] = make_int2((int)k, j * chunk);
 }
 
-// Field at the samples of one chunk per warp (persistent, grid-stride over
-// the chunks); a chunk holds up to 32 K samples and lane l holds samples
+// Field at the samples of one chunk per warp (persistent: warps take chunks
+// off a counter); a chunk holds up to 32 K samples and lane l holds samples
 // l, l + 32, ..., K per lane (K, W and CB are autotuned per context, see
 // eval_config_for).  All samples of a chunk share a hash cell, hence the
 // 27-cell candidate list of Evaluator::SingleEval; chunk_field filters the
@@ -510,6 +511,7 @@ __global__ void __launch_bounds__(32 * W, (K > 2 ? 24 : 32) / W) k_q_eval(QArgs 
                                                             const int2* __restrict__ chunks,
                                                             const int* __restrict__ nchunks_ptr,
                                                             const int* __restrict__ cbeg_ptr,
+                                                            int* __restrict__ next,
                                                             const float4* __restrict__ nd_c,
                                                             const float4* __restrict__ nd_v,
                                                             float* __restrict__ qval,
@@ -528,9 +530,16 @@ __global__ void __launch_bounds__(32 * W, (K > 2 ? 24 : 32) / W) k_q_eval(QArgs 
   // chunks [c0, c0 + count): a part of the level, or all of it from 0
   const int c0 = cbeg_ptr ? *cbeg_ptr : 0;
   const int cend = c0 + *nchunks_ptr;
-  const int nwarps = gridDim.x * W;
   long long pairs = 0, done = 0;
-  for (int ci = c0 + blockIdx.x * W + wib; ci < cend; ci += nwarps) {
+  // a warp takes the next chunk off a counter, asked for a chunk ahead: chunks
+  // differ in samples and candidates, and in a part of a level (a few chunks a
+  // warp) equal shares left the last warps working alone
+  const auto take = [&]() { return lane == 0 ? atomicAdd(next, 1) : 0; };
+  int ahead = take();
+  for (;;) {
+    const int ci = c0 + __shfl_sync(0xffffffffu, ahead, 0);
+    if (ci >= cend) break;
+    ahead = take();
     const int2 ch = chunks[ci];
     const int len = min(32 * K, __ldg(ucnt + ch.x) - ch.y);
     done += len;
@@ -1212,7 +1221,7 @@ __global__ void k_root(float cx, float cy, float cz, float h, int size, float4* 
 
 template <int K, int W, int CB, bool BULK>
 static void launch_eval(pi_frame* f, int cfg, const QArgs& qa, long long qn, const int* order, const int* qoff,
-                        const int* ucnt, const int2* chunks, const int* nchunks, const int* cbeg, int reserve,
+                        const int* ucnt, const int2* chunks, const int* nchunks, const int* cbeg, int* next, int reserve,
                         float* qval, unsigned long long* counters) {
   pi_ctx* ctx = f->ctx;
   static thread_local int occ[64][kEvalConfigs] = {};
@@ -1231,7 +1240,7 @@ static void launch_eval(pi_frame* f, int cfg, const QArgs& qa, long long qn, con
   if (reserve > 0) per_sm = std::max(1, std::min(per_sm, (65536 - reserve) / regs[dev][cfg]));
   const int blocks = (int)std::min<long long>((long long)ctx->smCount * per_sm, div_up(qn, 32 * W));
   PI_LAUNCH((k_q_eval<K, W, CB, BULK>), blocks, 32 * W, 0, ctx->stream, qa, order, qoff, ucnt, chunks, nchunks,
-            cbeg, f->nd_c.p, f->nd_v.p, qval, counters);
+            cbeg, next, f->nd_c.p, f->nd_v.p, qval, counters);
 }
 
 // The chunked evaluator's configurations: samples per lane K, warps per
@@ -1245,11 +1254,12 @@ const EvalConfig kEvalTable[kEvalConfigs] = {{1, 8, 96, 0}, {2, 8, 96, 0}, {4, 8
 
 // Chunk list for configuration cfg, then the chunked evaluation.
 static void eval_chunks(pi_frame* f, int cfg, const QArgs& qa, long long qn, const int* order, const int* qoff,
-                        const int* ucnt, const int2* chunks, const int* nchunks, const int* cbeg, int reserve,
+                        const int* ucnt, const int2* chunks, const int* nchunks, const int* cbeg, int* next, int reserve,
                         float* qval, unsigned long long* counters) {
 #define PI_EVAL_CASE(i, k, w, cb, bulk) \
   case i:                               \
-    launch_eval<k, w, cb, bulk>(f, i, qa, qn, order, qoff, ucnt, chunks, nchunks, cbeg, reserve, qval, counters); \
+    launch_eval<k, w, cb, bulk>(f, i, qa, qn, order, qoff, ucnt, chunks, nchunks, cbeg, next, reserve, qval,        \
+                                counters);                                                                        \
     break;
   switch (cfg) {
     PI_EVAL_CASE(0, 1, 8, 96, false)
@@ -1273,9 +1283,9 @@ static void dense_eval(pi_frame* f, int cfg, const QArgs& qa, long long qn, long
                        unsigned long long* counters) {
   cudaStream_t s = f->ctx->stream;
   const int K = kEvalTable[cfg].K;
-  PI_CUDA(cudaMemsetAsync(nchunks, 0, sizeof(int), s));
+  PI_CUDA(cudaMemsetAsync(nchunks, 0, 2 * sizeof(int), s));  // the count and the chunks taken
   PI_LAUNCH(k_q_chunks, div_up(nbuckets, 256), 256, 0, s, nbuckets, ucnt, 32 * K, chunks, nchunks);
-  eval_chunks(f, cfg, qa, qn, order, qoff, ucnt, chunks, nchunks, nullptr, reserve, qval, counters);
+  eval_chunks(f, cfg, qa, qn, order, qoff, ucnt, chunks, nchunks, nullptr, nchunks + 1, reserve, qval, counters);
 }
 
 // Configuration for a dense level of the given kind: the context's choice,
@@ -1695,7 +1705,7 @@ void stage_octree(pi_frame* f) {
   DBuf<unsigned> hslot;
   DBuf<int2> chunks;
   DBuf<float> qval;
-  qcnt.alloc(ctx, s, ek + 2);  // bucket counts, total, chunk count
+  qcnt.alloc(ctx, s, ek + 3);  // bucket counts, total, chunk count, chunks taken
   ucnt.alloc(ctx, s, ek + 1);  // distinct points per bucket (+ 1 for the scan's total)
   ucum.alloc(ctx, s, ek + 1);  // exclusive scan of ucnt (sparse levels)
   long long lb = 0, le = 1;
@@ -1840,7 +1850,7 @@ void stage_octree(pi_frame* f) {
         // the leaf level in parts: part p's QEF beside part p + 1's sampling
         const int parts = ctx->qef_parts;
         DBuf<int> pinfo;
-        pinfo.alloc(ctx, s, 3 * (parts + 1));
+        pinfo.alloc(ctx, s, 4 * (parts + 1));
         DBuf<int8_t> npart;
         npart.alloc(ctx, s, nl);
         // the frame's arrays, so that they outlive the QEF stream's reads (the
@@ -1860,7 +1870,7 @@ void stage_octree(pi_frame* f) {
           // the grid is sized by the level (a part may hold fewer slots than
           // it has parts, and the blocks stride over the part's chunks)
           eval_chunks(f, cfg, qa, qn, order.p, qcnt.p, ucnt.p, chunks.p, pinfo.p + 2 * (parts + 1) + p,
-                      pinfo.p + parts + 1 + p, kQefReserveRegs, qval.p, f->dcount.p);
+                      pinfo.p + parts + 1 + p, pinfo.p + 3 * (parts + 1) + p, kQefReserveRegs, qval.p, f->dcount.p);
           prof_end(ctx, s, PG_CHUNK);
           // a part holds about nl / parts nodes; the blocks stride over what it
           // holds.  (Classified on the QEF stream, in front of the part's QEF,
