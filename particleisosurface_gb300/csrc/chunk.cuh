@@ -111,6 +111,40 @@ __device__ __forceinline__ void eval_staged(const ChunkStage& st, int nc, const 
   }
 }
 
+// The 27-cell candidates of a cell as one run of `total` places: the nine rows
+// one after the other.  Lane r < 9 holds row r's range, so their offsets load
+// together, and a batch of 32 candidates spans rows: a row holds 5 of the 49
+// candidates of a dam-break frame's points, and row by row the filter ran nine
+// batches of five lanes where two full ones do.  (1M frame, level D_max - 1:
+// 712 -> 555 us; uniform grid of 150k particles 527 -> 450 us.)
+struct CandidateRun {
+  int total;
+  int incl;   // places up to and with this lane's row
+  int shift;  // place t of this lane's row is particle t + shift
+  __device__ __forceinline__ CandidateRun(const GridView& g, int cx, int cy, int cz) {
+    const int lane = threadIdx.x & 31;
+    int s = 0, e = 0;
+    if (lane >= 9 || !nb_row(g, cx, cy + lane % 3 - 1, cz + lane / 3 - 1, &s, &e)) s = e = 0;
+    incl = e - s;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += v;
+    }
+    total = __shfl_sync(0xffffffffu, incl, 8);
+    shift = s - (incl - (e - s));
+    if (lane >= 9) incl = 0x7fffffff;  // ends the search below
+  }
+  // particle at place t (any index for t >= total); every lane calls it
+  __device__ __forceinline__ int at(int t) const {
+    int r = 0;  // rows that end at or before t
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, incl, r + o - 1) <= t) r += o;
+    return t + __shfl_sync(0xffffffffu, shift, r);
+  }
+};
+
 // Sums over the chunk's candidates for the K points of this lane.  act[m]
 // marks the lane's valid points, and an invalid point's coordinates must be
 // NaN (its s2 is then NaN and no term passes s2 < 4); slots[m]
@@ -176,47 +210,46 @@ __device__ __forceinline__ void chunk_field(const GridView& g, const PartView& P
     __syncwarp();
     nc = 0;
   };
-  for (int dz = -1; dz <= 1; ++dz)
-    for (int dy = -1; dy <= 1; ++dy) {
-      int rs, re;
-      if (!nb_row(g, cx, cy + dy, cz + dz, &rs, &re)) continue;
-      pairs += (long long)(re - rs) * nact;
-      for (int j0 = rs; j0 < re; j0 += 32) {
-        const int j = j0 + lane;
-        bool pass = false;
-        float4 x;
-        if (j < re) {
-          x = __ldg(P.xm + j);
-          const float ex = fmaxf(fmaxf(blx - x.x, x.x - bhx), 0.f);
-          const float ey = fmaxf(fmaxf(bly - x.y, x.y - bhy), 0.f);
-          const float ez = fmaxf(fmaxf(blz - x.z, x.z - bhz), 0.f);
-          pass = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < x.w;
-        }
-        const unsigned pm = __ballot_sync(0xffffffffu, pass);
-        if (pass) {
-          const int p = nc + __popc(pm & lt);
-          float* const c0 = st.c + p;
-          c0[SC_X * CB] = x.x;
-          c0[SC_Y * CB] = x.y;
-          c0[SC_Z * CB] = x.z;
-          const float* ga = reinterpret_cast<const float*>(P.ga + j);
-          const float* gb = reinterpret_cast<const float*>(P.gb + j);
-          const float* gl = reinterpret_cast<const float*>(P.xlo + j);
-          cp_async4(c0 + SC_LX * CB, gl);
-          cp_async4(c0 + SC_LY * CB, gl + 1);
-          cp_async4(c0 + SC_LZ * CB, gl + 2);
-          cp_async4(c0 + SC_A0 * CB, ga);
-          cp_async4(c0 + SC_A1 * CB, ga + 1);
-          cp_async4(c0 + SC_A2 * CB, ga + 2);
-          cp_async4(c0 + SC_A3 * CB, ga + 3);
-          cp_async4(c0 + SC_B0 * CB, gb);
-          cp_async4(c0 + SC_B1 * CB, gb + 1);
-          cp_async4(c0 + SC_B2 * CB, gb + 2);
-        }
-        nc += __popc(pm);
-        if (nc > CB - 32) flush();
-      }
+  const CandidateRun run(g, cx, cy, cz);
+  pairs += (long long)run.total * nact;
+  // each batch's centres are loaded while the batch before is tested
+  int j = run.at(lane);
+  float4 x = make_float4(0.f, 0.f, 0.f, -1.f);
+  if (lane < run.total) x = __ldg(P.xm + j);
+  for (int t0 = 0; t0 < run.total; t0 += 32) {
+    const int jn = run.at(t0 + 32 + lane);
+    float4 xn = make_float4(0.f, 0.f, 0.f, -1.f);
+    if (t0 + 32 + lane < run.total) xn = __ldg(P.xm + jn);
+    const float ex = fmaxf(fmaxf(blx - x.x, x.x - bhx), 0.f);
+    const float ey = fmaxf(fmaxf(bly - x.y, x.y - bhy), 0.f);
+    const float ez = fmaxf(fmaxf(blz - x.z, x.z - bhz), 0.f);
+    const bool pass = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) < x.w;  // x.w < 0 past the run's end
+    const unsigned pm = __ballot_sync(0xffffffffu, pass);
+    if (pass) {
+      const int p = nc + __popc(pm & lt);
+      float* const c0 = st.c + p;
+      c0[SC_X * CB] = x.x;
+      c0[SC_Y * CB] = x.y;
+      c0[SC_Z * CB] = x.z;
+      const float* ga = reinterpret_cast<const float*>(P.ga + j);
+      const float* gb = reinterpret_cast<const float*>(P.gb + j);
+      const float* gl = reinterpret_cast<const float*>(P.xlo + j);
+      cp_async4(c0 + SC_LX * CB, gl);
+      cp_async4(c0 + SC_LY * CB, gl + 1);
+      cp_async4(c0 + SC_LZ * CB, gl + 2);
+      cp_async4(c0 + SC_A0 * CB, ga);
+      cp_async4(c0 + SC_A1 * CB, ga + 1);
+      cp_async4(c0 + SC_A2 * CB, ga + 2);
+      cp_async4(c0 + SC_A3 * CB, ga + 3);
+      cp_async4(c0 + SC_B0 * CB, gb);
+      cp_async4(c0 + SC_B1 * CB, gb + 1);
+      cp_async4(c0 + SC_B2 * CB, gb + 2);
     }
+    nc += __popc(pm);
+    if (nc > CB - 32) flush();
+    j = jn;
+    x = xn;
+  }
   flush();
 #pragma unroll
   for (int m = 0; m < K; ++m) sum[m] = s[m];
