@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "chunk.cuh"
 #include "device.cuh"
 #include "dmc.h"
 #include "internal.h"
@@ -596,36 +597,52 @@ __global__ void k_vcell_place(long long nv, const int* __restrict__ key, const i
 }
 
 template <bool VR>
-__global__ void k_bisect(BisectArgs a, long long nv, const int* __restrict__ order, const int* __restrict__ rep,
+__global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, const int* __restrict__ order, const int* __restrict__ rep,
                          const int* __restrict__ slotA,
                          const int* __restrict__ slotB, const float4* __restrict__ nd_v,
                          const uint64_t* __restrict__ nd_id, float* __restrict__ out,
                          uint64_t* __restrict__ vkeys, int2* __restrict__ vedge,
                          unsigned long long* __restrict__ counters) {
+  __shared__ __align__(16) float s_stage[VR ? 1 : kGroupWarps][VR ? 1 : GroupRoom<32>::kFloats];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nv) return;
-  const long long v = order[t];
-  const int s = rep[v];
-  const int A = slotA[s], B = slotB[s];
-  vedge[v] = make_int2(A, B);
-  float4 p = nd_v[A], q = nd_v[B];
+  const bool valid = t < nv;
+  long long v = 0;
+  int A = 0, B = 0;
+  float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
+  if (valid) {
+    v = order[t];
+    const int s = rep[v];
+    A = slotA[s], B = slotB[s];
+    p = nd_v[A], q = nd_v[B];
+  }
   const float dx = __fsub_rn(p.x, q.x), dy = __fsub_rn(p.y, q.y), dz = __fsub_rn(p.z, q.z);
   float d = __fsqrt_rn(__fadd_rn(__fmul_rn(dx, dx), __fadd_rn(__fmul_rn(dy, dy), __fmul_rn(dz, dz))));
   long long pairs = 0;
   int steps = 0;
-  while (d > a.rr && steps < 64) {
+  // a warp steps until its last edge is short enough
+  for (int it = 0; it < 64; ++it) {
+    const bool go = d > a.rr;
+    if (!__any_sync(0xffffffffu, go)) break;
     float4 m;
     m.x = __fmul_rn(__fadd_rn(p.x, q.x), 0.5f);
     m.y = __fmul_rn(__fadd_rn(p.y, q.y), 0.5f);
     m.z = __fmul_rn(__fadd_rn(p.z, q.z), 0.5f);
-    m.w = a.iso - (VR ? field_sum_vr(*a.mg, a.P, m.x, m.y, m.z, &pairs) : field_sum(a.g, a.P, m.x, m.y, m.z, &pairs));
-    if ((m.w > 0.f) == (p.w > 0.f))
-      p = m;
-    else
-      q = m;
-    d = __fmul_rn(d, 0.5f);
-    ++steps;
+    if (VR) {
+      m.w = go ? a.iso - field_sum_vr(*a.mg, a.P, m.x, m.y, m.z, &pairs) : 0.f;
+    } else {
+      m.w = a.iso - group_field<32>(a.g, a.P, m.x, m.y, m.z, go, s_stage[VR ? 0 : threadIdx.x >> 5], pairs);
+    }
+    if (go) {
+      if ((m.w > 0.f) == (p.w > 0.f))
+        p = m;
+      else
+        q = m;
+      d = __fmul_rn(d, 0.5f);
+      ++steps;
+    }
   }
+  if (!valid) return;
+  vedge[v] = make_int2(A, B);
   const float ratio = __fdiv_rn(__fsub_rn(0.0f, p.w), __fsub_rn(q.w, p.w));
   float3 r;
   if (ratio < kAbove01) {  // (double)ratio < 0.1

@@ -634,18 +634,24 @@ __global__ void k_q_compact(long long n, const int* __restrict__ qkey, const int
 // position; the 27 lattice samples of GridEval only set a sign-change flag
 // that nothing reads there (they feed NodeCalcNode, i.e. QEF mode only), so
 // only the node position is evaluated.  The node's signchange stays 0.
-__global__ void __launch_bounds__(256, 4) k_leaf_level(LevelArgs a, const float4* __restrict__ nd_c,
+__global__ void __launch_bounds__(32 * kGroupWarps, 8) k_leaf_level(LevelArgs a, const float4* __restrict__ nd_c,
                                                        float4* __restrict__ nd_v, int8_t* __restrict__ nd_type,
                                                        unsigned long long* __restrict__ counters) {
+  __shared__ __align__(16) float s_stage[kGroupWarps][GroupRoom<8>::kFloats];
+  float* const st = s_stage[threadIdx.x >> 5];
   long long pairs = 0, evals = 0;
-  for (long long node = a.lb + (long long)blockIdx.x * blockDim.x + threadIdx.x; node < a.le;
-       node += (long long)gridDim.x * blockDim.x) {
-    if (nd_type[node] != T_UNCERTAIN) continue;
-    float4 v = nd_v[node];
-    v.w = a.iso - field_sum(a.g, a.P, v.x, v.y, v.z, &pairs);
-    nd_v[node] = v;
-    nd_type[node] = T_LEAF;
-    ++evals;
+  for (long long n0 = a.lb + (long long)blockIdx.x * blockDim.x; n0 < a.le; n0 += (long long)gridDim.x * blockDim.x) {
+    const long long node = n0 + threadIdx.x;
+    const bool active = node < a.le && nd_type[node] == T_UNCERTAIN;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (active) v = nd_v[node];
+    const float sum = group_field<8>(a.g, a.P, v.x, v.y, v.z, active, st, pairs);
+    if (active) {
+      v.w = a.iso - sum;
+      nd_v[node] = v;
+      nd_type[node] = T_LEAF;
+      ++evals;
+    }
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -1804,7 +1810,8 @@ void stage_octree(pi_frame* f) {
       PI_LAUNCH(k_empty, div_up(nl, wpb), 32 * wpb, 0, s, la, f->nd_c.p, f->nd_v.p, f->nd_type.p, f->nd_curv.p);
     if (depth >= f->dmin && leaf_level && !f->P.qef) {
       prof_begin(ctx, s, PG_LEAF);
-      PI_LAUNCH(k_leaf_level, (int)std::min<long long>((long long)ctx->smCount * 8, div_up(nl, 256)), 256, 0, s, la,
+      PI_LAUNCH(k_leaf_level, (int)std::min<long long>((long long)ctx->smCount * 32, div_up(nl, 32 * kGroupWarps)),
+                32 * kGroupWarps, 0, s, la,
                 f->nd_c.p, f->nd_v.p, f->nd_type.p, f->dcount.p);
       prof_end(ctx, s, PG_LEAF);
     } else if (depth >= f->dmin) {
