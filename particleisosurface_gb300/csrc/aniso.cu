@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __re
       for (int k = 0; k < 6; ++k) a6d[k] = (double)a6[k];
       sym_eig3<double>(a6d, wd, Vd);
       g_from_eig<double>(wd, Vd, G, &stretch);
-      stripe_add(f64count, 0, 1ull);
+      stripe_add(f64count, C_FP64_EIGEN, 1ull);
     } else {
       g_from_eig<float>(w, V, G, &stretch);
     }
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(128) k_vr_cov_G(const MultiGridView* __restric
       for (int k = 0; k < 6; ++k) a6d[k] = (double)a6[k];
       sym_eig3<double>(a6d, wd, Vd);
       g_from_eig<double>(wd, Vd, G, &stretch);
-      stripe_add(f64count, 0, 1ull);
+      stripe_add(f64count, C_FP64_EIGEN, 1ull);
     } else {
       g_from_eig<float>(w, V, G, &stretch);
     }
@@ -418,7 +418,8 @@ void stage_aniso_vr(pi_frame* f) {
   f->gfull.alloc(f->ctx, s, n * 9);
   f->det.alloc(f->ctx, s, n);
   f->f64flag.alloc(f->ctx, s, n);
-  counters_reset(f);
+  counters_reset(f, 0, kCounters - 1);  // every stage's
+  f->octree_counted = f->extract_counted = false;
   PI_LAUNCH(k_vr_xmean, div_up(n, 128), 128, 0, s, f->mgv.p, f->pos.p, f->vrcs.p, n, (float)0.9, f->nrm.p,
             f->xlo.p);
   PI_LAUNCH(k_vr_cov_G, div_up(n, 128), 128, 0, s, f->mgv.p, f->pos.p, f->vrcs.p, f->nrm.p, f->xlo.p, f->xm.p, n,
@@ -451,7 +452,8 @@ void stage_aniso(pi_frame* f) {
   f->f64flag.alloc(f->ctx, s, n);
   const bool splash = f->P.splash != 0;
   if (splash) f->spl.alloc(f->ctx, s, n);
-  counters_reset(f);
+  counters_reset(f, 0, kCounters - 1);  // every stage's
+  f->octree_counted = f->extract_counted = false;
   PI_LAUNCH(k_xmean, div_up(n, 128), 128, 0, s, g, f->pos.p, n, nI, nI2, inv_h3, c_mean, f->nrm.p, f->xlo.p,
             splash ? f->spl.p : nullptr);
   PI_LAUNCH(k_cov_G, div_up(n, 128), 128, 0, s, g, f->pos.p, f->nrm.p, f->xlo.p, f->xm.p, n, nI, nI2, inv_h3, f->influ2,

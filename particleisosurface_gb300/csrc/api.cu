@@ -38,21 +38,74 @@ void ctx_account(pi_ctx* c, long long delta) {
   }
 }
 
+// The kept block that fits best: at least `bytes`, at most twice that (or 64 KiB
+// more).
+static void* keep_take(pi_ctx* c, cudaStream_t st, size_t bytes, size_t* got) {
+  if (!c || c->budget || bytes > kKeepBlock) return nullptr;
+  std::lock_guard<std::mutex> lk(c->keep_mu);
+  const size_t most = std::max(2 * bytes, bytes + 65536);
+  size_t best = c->kept.size();
+  for (size_t i = 0; i < c->kept.size(); ++i) {
+    const auto& b = c->kept[i];
+    if (b.s == st && b.bytes >= bytes && b.bytes <= most &&
+        (best == c->kept.size() || b.bytes < c->kept[best].bytes))
+      best = i;
+  }
+  if (best == c->kept.size()) return nullptr;
+  void* const p = c->kept[best].p;
+  *got = c->kept[best].bytes;
+  c->kept_bytes -= *got;
+  c->kept[best] = c->kept.back();
+  c->kept.pop_back();
+  return p;
+}
+
+static bool keep_put(pi_ctx* c, void* p, size_t bytes, cudaStream_t st) {
+  if (!c || c->budget || bytes > kKeepBlock) return false;
+  std::lock_guard<std::mutex> lk(c->keep_mu);
+  if (c->kept_bytes + bytes > kKeepBytes) return false;
+  try {
+    c->kept.push_back({p, bytes, st});
+  } catch (...) {
+    return false;
+  }
+  c->kept_bytes += bytes;
+  return true;
+}
+
+static void keep_free(pi_ctx* c) {
+  if (!c) return;
+  std::lock_guard<std::mutex> lk(c->keep_mu);
+  for (const auto& b : c->kept) cudaFreeAsync(b.p, b.s);
+  c->kept.clear();
+  c->kept_bytes = 0;
+}
+
 template <class T>
 void DBuf<T>::alloc(pi_ctx* c, cudaStream_t st, size_t count) {
   release();
   if (count == 0) count = 1;
-  ctx_account(c, (long long)(count * sizeof(T)));
-  void* q = nullptr;
-  cudaError_t e = cudaMallocAsync(&q, count * sizeof(T), st);
-  if (e != cudaSuccess) {
-    ctx_account(c, -(long long)(count * sizeof(T)));
-    (void)cudaGetLastError();
-    if (e == cudaErrorMemoryAllocation) throw NoMem("cudaMallocAsync: out of device memory");
-    throw CudaError(std::string("cudaMallocAsync: ") + cudaGetErrorString(e), (int)e);
+  const size_t bytes = count * sizeof(T);
+  ctx_account(c, (long long)bytes);
+  size_t got = bytes;
+  void* q = keep_take(c, st, bytes, &got);
+  if (!q) {
+    cudaError_t e = cudaMallocAsync(&q, bytes, st);
+    if (e == cudaErrorMemoryAllocation) {
+      (void)cudaGetLastError();
+      keep_free(c);
+      e = cudaMallocAsync(&q, bytes, st);
+    }
+    if (e != cudaSuccess) {
+      ctx_account(c, -(long long)bytes);
+      (void)cudaGetLastError();
+      if (e == cudaErrorMemoryAllocation) throw NoMem("cudaMallocAsync: out of device memory");
+      throw CudaError(std::string("cudaMallocAsync: ") + cudaGetErrorString(e), (int)e);
+    }
   }
   p = static_cast<T*>(q);
   n = count;
+  cap = got;
   ctx = c;
   s = st;
 }
@@ -60,29 +113,27 @@ void DBuf<T>::alloc(pi_ctx* c, cudaStream_t st, size_t count) {
 template <class T>
 void DBuf<T>::grow(pi_ctx* c, cudaStream_t st, size_t count, size_t keep) {
   if (count <= n) return;
-  T* old = p;
-  size_t oldn = n;
-  pi_ctx* oc = ctx;
-  cudaStream_t os = s;
-  p = nullptr;
-  n = 0;
+  DBuf<T> old;
+  std::swap(old.p, p);
+  std::swap(old.n, n);
+  std::swap(old.cap, cap);
+  old.ctx = ctx;
+  old.s = s;
   alloc(c, st, count);
-  if (old) {
-    keep = keep < oldn ? keep : oldn;  // never past the old allocation
-    if (keep) PI_CUDA(cudaMemcpyAsync(p, old, keep * sizeof(T), cudaMemcpyDeviceToDevice, st));
-    cudaFreeAsync(old, os);
-    ctx_account(oc, -(long long)(oldn * sizeof(T)));
+  if (old.p) {
+    keep = keep < old.n ? keep : old.n;  // never past the old allocation
+    if (keep) PI_CUDA(cudaMemcpyAsync(p, old.p, keep * sizeof(T), cudaMemcpyDeviceToDevice, st));
   }
 }
 
 template <class T>
 void DBuf<T>::release() {
   if (p) {
-    cudaFreeAsync(p, s);
+    if (!keep_put(ctx, p, cap, s)) cudaFreeAsync(p, s);
     ctx_account(ctx, -(long long)(n * sizeof(T)));
   }
   p = nullptr;
-  n = 0;
+  n = cap = 0;
 }
 
 template struct DBuf<float>;
@@ -108,10 +159,19 @@ float bspline_host(float ratio, float sigma) {
   return 0.0f;
 }
 
-void counters_reset(pi_frame* f) {
+void counters_reset(pi_frame* f, int first, int last) {
   cudaStream_t s = f->ctx->stream;
-  if (f->dcount.n < (size_t)kCounterWords) f->dcount.alloc(f->ctx, s, kCounterWords);
-  PI_CUDA(cudaMemsetAsync(f->dcount.p, 0, sizeof(unsigned long long) * kCounterWords, s));
+  if (f->dcount.n < (size_t)kCounterWords) {
+    f->dcount.alloc(f->ctx, s, kCounterWords);
+    first = 0, last = kCounters - 1;
+  }
+  const size_t words = (size_t)kStripes * 4;
+  PI_CUDA(cudaMemsetAsync(f->dcount.p + first * words, 0, sizeof(unsigned long long) * words * (last - first + 1), s));
+}
+
+void counters_begin(pi_frame* f, bool* counted, int first, int last) {
+  if (*counted || f->dcount.n < (size_t)kCounterWords) counters_reset(f, first, last);
+  *counted = true;
 }
 
 void counters_read(pi_frame* f, unsigned long long out[kCounters]) {
@@ -127,8 +187,6 @@ void counters_read(pi_frame* f, unsigned long long out[kCounters]) {
 }
 
 void counters_snapshot(pi_frame* f, int slot) {
-  PI_CUDA(cudaMemcpyAsync(f->ctx->hpin + (size_t)slot * kCounterWords, f->dcount.p,
-                          sizeof(unsigned long long) * kCounterWords, cudaMemcpyDeviceToHost, f->ctx->stream));
   f->pin_pending |= 1 << slot;
 }
 
@@ -143,6 +201,12 @@ void resolve_pending(pi_frame* f) {
   qef_join(f);
   topology_join(f);
   if (!f->ev_pending && !f->pin_pending) return;
+  if (f->pin_pending & ~(1 << kPinValid))
+    PI_CUDA(cudaMemcpyAsync(f->ctx->hpin, f->dcount.p, sizeof(unsigned long long) * kCounterWords,
+                            cudaMemcpyDeviceToHost, f->ctx->stream));
+  if (f->pin_pending & (1 << kPinValid))
+    PI_CUDA(cudaMemcpyAsync(reinterpret_cast<int*>(f->ctx->hpin + (size_t)kPinSlots * kCounterWords),
+                            f->off.p + f->g.cellNum, sizeof(int), cudaMemcpyDeviceToHost, f->ctx->stream));
   PI_CUDA(cudaStreamSynchronize(f->ctx->stream));
   for (int k = 0; k < 8; ++k)
     if (f->ev_pending & (1 << k)) {
@@ -154,12 +218,9 @@ void resolve_pending(pi_frame* f) {
   const unsigned long long* h = f->ctx->hpin;
   unsigned long long c[kCounters];
   pi_ctx* ctx = f->ctx;
-  if (f->pin_pending & (1 << kPinAniso)) {
-    fold_counters(h + (size_t)kPinAniso * kCounterWords, c);
-    f->fp64Count = (long long)c[0];
-  }
+  if (f->pin_pending & ~(1 << kPinValid)) fold_counters(h, c);
+  if (f->pin_pending & (1 << kPinAniso)) f->fp64Count = (long long)c[C_FP64_EIGEN];
   if (f->pin_pending & (1 << kPinOctree)) {
-    fold_counters(h + (size_t)kPinOctree * kCounterWords, c);
     // the reference's NodeCalcNode evaluates the field at the leaf's node
     // point whether or not its vertex is accepted (src/iso_method_ours.cpp:
     // 161-173): one more reference call per leaf solved
@@ -181,7 +242,6 @@ void resolve_pending(pi_frame* f) {
     }
   }
   if (f->pin_pending & (1 << kPinExtract)) {
-    fold_counters(h + (size_t)kPinExtract * kCounterWords, c);
     f->nDual = (long long)c[C_DUAL];
     f->bisectEvals = (long long)c[C_BISECT_EVALS];
     f->fieldEvals += (long long)c[C_BISECT_EVALS];
@@ -455,6 +515,7 @@ int pi_ctx_create(int device, size_t budget_bytes, pi_ctx** out) {
 static void ctx_release(pi_ctx* c) {
   if (c->refs.fetch_sub(1) != 1) return;
   cudaSetDevice(c->device);
+  keep_free(c);
   cudaStreamSynchronize(c->stream);
   if (c->topo_stream) {
     cudaStreamSynchronize(c->topo_stream);

@@ -81,7 +81,9 @@ enum Counter : int {
   C_DONE_THREAD = 13,  // evaluations performed by k_q_eval_thread (distinct samples)
   C_DONE_LEAF = 14,    // evaluations performed by k_leaf_level (one per leaf)
   C_STAGE_TIMEOUT = 15,  // bulk-staging waits that ran out (an error: the frame's values are void)
-  kCounters = 16
+  C_FP64_EIGEN = 16,  // particles whose eigen-decomposition ran in FP64
+  C_GRID_PAIRS = 17,  // candidate pairs of the uniform-grid sampler
+  kCounters = 18
 };
 constexpr int kCounterWords = kCounters * kStripes * 4;
 

@@ -380,16 +380,17 @@ struct FirstSlot {
   }
 };
 
-// Ranks of the first slots among n: rank[n] is their number.  The flags are
+// Ranks of the first slots among n: rank[n] and *total are their number.  The flags are
 // worked out inside the scan while it reads them once; a longer scan reads its
 // input twice, and the flags' random table reads are dearer than an array.
-static void rank_first(long long n, const unsigned* tab, const uint32_t* where, int* rank, int* tmp, cudaStream_t s) {
+static void rank_first(long long n, const unsigned* tab, const uint32_t* where, int* rank, int* total, int* tmp,
+                       cudaStream_t s) {
   if (n + 1 <= kScanOneLaunch) {
-    exclusive_scan(ScanOf<FirstSlot>{{tab, where}, n}, rank, n + 1, nullptr, tmp, s);
+    exclusive_scan(ScanOf<FirstSlot>{{tab, where}, n}, rank, n + 1, total, tmp, s);
     return;
   }
   PI_LAUNCH(k_first_flag, div_up(n + 1, 256), 256, 0, s, n, tab, where, rank);
-  exclusive_scan_i32(rank, rank, n + 1, nullptr, tmp, s);
+  exclusive_scan_i32(rank, rank, n + 1, total, tmp, s);
 }
 
 // slot -> vertex (numbered in order of first slots); vertex -> its first slot
@@ -682,44 +683,19 @@ static uint32_t table_mask(long long n) {
   return m - 1;
 }
 
-static int read_int(pi_frame* f, const int* d) {
-  int v = 0;
-  PI_CUDA(cudaMemcpyAsync(&v, d, sizeof(int), cudaMemcpyDeviceToHost, f->ctx->stream));
-  PI_CUDA(cudaStreamSynchronize(f->ctx->stream));
-  return v;
-}
-
-// A count read in two halves: the copy to pinned memory is queued, the
-// caller queues a kernel that does not need the count, then waits for the
-// copy only, so the device is busy while the host takes the value.
-static void read_int_start(pi_frame* f, const int* d) {
-  int* const h = reinterpret_cast<int*>(f->ctx->hpin + kPinReadOffset);
-  PI_CUDA(cudaMemcpyAsync(h, d, sizeof(int), cudaMemcpyDeviceToHost, f->ctx->stream));
-  PI_CUDA(cudaEventRecord(f->ctx->ev_read, f->ctx->stream));
-}
-static int read_int_finish(pi_frame* f) {
-  PI_CUDA(cudaEventSynchronize(f->ctx->ev_read));
-  return *reinterpret_cast<const int*>(f->ctx->hpin + kPinReadOffset);
-}
-
-// A count read on stream st through a pinned word and an event.
+// A count the host waits for on stream st: a scan stores its total in a pinned
+// word, an event follows it, and the caller may queue work that does not need
+// the count before it waits for the event (no copy, no stream-wide wait).
 struct CountReader {
   pi_frame* f;
   cudaStream_t st;
   int off;
   cudaEvent_t ev;
-  int read(const int* d) const {
-    start(d);
-    return finish();
-  }
-  void start(const int* d) const {
-    int* const h = reinterpret_cast<int*>(f->ctx->hpin + off);
-    PI_CUDA(cudaMemcpyAsync(h, d, sizeof(int), cudaMemcpyDeviceToHost, st));
-    PI_CUDA(cudaEventRecord(ev, st));
-  }
-  int finish() const {
+  int* word() const { return reinterpret_cast<int*>(f->ctx->hpin + off); }
+  void stored() const { PI_CUDA(cudaEventRecord(ev, st)); }
+  int wait() const {
     PI_CUDA(cudaEventSynchronize(ev));
-    return *reinterpret_cast<const int*>(f->ctx->hpin + off);
+    return *const_cast<const volatile int*>(word());
   }
 };
 
@@ -759,8 +735,9 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
       PI_CUDA(cudaMemsetAsync(used.p, 0, sizeof(int) * (nb + 1), s));
       PI_LAUNCH(k_block_mark, div_up(nf, 128), 128, 0, s, f->nd_child.p, nf, f->nd_org.p, full, bb, used.p);
       slot.alloc(c, s, nb + 1);
-      exclusive_scan_i32(used.p, slot.p, nb + 1, nullptr, tmp.p, s);
-      nused = rd.read(slot.p + nb);
+      exclusive_scan_i32(used.p, slot.p, nb + 1, rd.word(), tmp.p, s);
+      rd.stored();
+      nused = rd.wait();
       blist.alloc(c, s, nused > 0 ? nused : 1);
       PI_LAUNCH(k_block_list, div_up(nb, 256), 256, 0, s, nb, used.p, slot.p, blist.p);
     }
@@ -773,8 +750,9 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     PI_CUDA(cudaMemsetAsync(bits.p, 0, sizeof(unsigned) * (nw > 0 ? nw : 1), s));
     PI_LAUNCH(k_corner_mark, div_up(nf, 128), 128, 0, s, f->nd_child.p, nf, f->nd_org.p, full, bb,
               dense ? nullptr : slot.p, bits.p);
-    exclusive_scan(ScanOf<WordBits>{{bits.p}, nw}, cnt.p, nw + 1, nullptr, tmp.p, s);
-    nu = rd.read(cnt.p + nw);
+    exclusive_scan(ScanOf<WordBits>{{bits.p}, nw}, cnt.p, nw + 1, rd.word(), tmp.p, s);
+    rd.stored();
+    nu = rd.wait();
     if (uverts.n < (size_t)(nu > 0 ? nu : 1)) uverts.alloc(c, s, nu > 0 ? nu : 1);
     PI_LAUNCH(k_bitmap_keys, div_up(nw, 256), 256, 0, s, bits.p, nw, cnt.p, bb, dense ? nullptr : blist.p, B,
               uverts.p);
@@ -797,8 +775,9 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     uf.alloc(c, s, nk + 1);
     tmp.alloc(c, s, scan_tmp_ints(nk + 1));
     PI_LAUNCH(k_unique_flag, div_up(nk + 1, 256), 256, 0, s, kp, nk, invalid, uf.p);
-    exclusive_scan_i32(uf.p, uf.p, nk + 1, nullptr, tmp.p, s);
-    nu = rd.read(uf.p + nk);
+    exclusive_scan_i32(uf.p, uf.p, nk + 1, rd.word(), tmp.p, s);
+    rd.stored();
+    nu = rd.wait();
     if (uverts.n < (size_t)(nu > 0 ? nu : 1)) uverts.alloc(c, s, nu > 0 ? nu : 1);
     PI_LAUNCH(k_unique_write, div_up(nk, 256), 256, 0, s, kp, uf.p, nk, invalid, uverts.p);
   }
@@ -849,17 +828,19 @@ void stage_extract(pi_frame* f) {
   procs.alloc(c, s, nu > 0 ? nu : 1);
   toff.alloc(c, s, nu + 1);
   if (tmp.n < scan_tmp_ints(nu + 1)) tmp.alloc(c, s, scan_tmp_ints(nu + 1));
+  const CountReader rd{f, s, kPinReadOffset, c->ev_read};
   // k_dual reads the leaves' values: the octree's last QEF level, if it was
   // left running, ends here, and the octree's counters are taken
   if (f->qef_inflight) {
     qef_join(f);
     counters_snapshot(f, kPinOctree);
   }
-  counters_reset(f);
+  counters_begin(f, &f->extract_counted, C_DUAL, C_BISECT_PAIRS);
   PI_LAUNCH(k_dual, div_up(nu + 1, 128), 128, 0, s, uverts, nu, B, f->nd_child.p, f->nd_v.p,
             cells.p, reinterpret_cast<uint8_t*>(procs.p), toff.p, f->dcount.p);
-  exclusive_scan_i32(toff.p, toff.p, nu + 1, nullptr, tmp.p, s);
-  const long long nt0 = read_int(f, toff.p + nu);
+  exclusive_scan_i32(toff.p, toff.p, nu + 1, rd.word(), tmp.p, s);
+  rd.stored();
+  const long long nt0 = rd.wait();
   // 4. triangle slots and vertex keys (sorted leaf-id pairs)
   const int id_bits = 3 * f->dmax;
   const int packed = (2 * id_bits <= 64) ? 1 : 0;
@@ -890,12 +871,12 @@ void stage_extract(pi_frame* f) {
   PI_CUDA(cudaMemsetAsync(vtab.p, 0, sizeof(unsigned) * ((size_t)vmask + 1), s));
   PI_LAUNCH(k_vkey_insert, div_up(ns, 256), 256, 0, s, ns, packed ? nullptr : khi.p, klo.p, vmask, vtab.p,
             vwhere.p);
-  rank_first(ns, vtab.p, vwhere.p, vrank.p, tmp.p, s);
-  read_int_start(f, vrank.p + ns);
+  rank_first(ns, vtab.p, vwhere.p, vrank.p, rd.word(), tmp.p, s);
+  rd.stored();
   slot_vertex.alloc(c, s, ns > 0 ? ns : 1);
   rep.alloc(c, s, ns > 0 ? ns : 1);  // room for a vertex per slot
   PI_LAUNCH(k_vertex_map, div_up(ns, 256), 256, 0, s, ns, vtab.p, vwhere.p, vrank.p, slot_vertex.p, rep.p);
-  const long long nv = read_int_finish(f);
+  const long long nv = rd.wait();
   vtab.release();
   vwhere.release();
   vrank.release();
@@ -918,8 +899,8 @@ void stage_extract(pi_frame* f) {
   trank.alloc(c, s, nt0 + 1);
   PI_CUDA(cudaMemsetAsync(ttab.p, 0, sizeof(unsigned) * ((size_t)tmask + 1), s));
   PI_LAUNCH(k_tri_insert, div_up(nt0, 256), 256, 0, s, nt0, otri.p, tmask, ttab.p, twhere.p);
-  rank_first(nt0, ttab.p, twhere.p, trank.p, tmp.p, s);
-  read_int_start(f, trank.p + nt0);
+  rank_first(nt0, ttab.p, twhere.p, trank.p, rd.word(), tmp.p, s);
+  rd.stored();
   // room for every generated triangle and the splash icosahedra
   const long long nsp = f->P.splash ? f->nSplash : 0;
   const long long tcap = (nt0 + 20 * nsp) * 3;
@@ -929,7 +910,7 @@ void stage_extract(pi_frame* f) {
   f->mk.alloc(c, s, (nv + 12 * nsp) * 2 > 0 ? (nv + 12 * nsp) * 2 : 2);
   f->vedge.alloc(c, s, nv + 12 * nsp > 0 ? nv + 12 * nsp : 1);
   if (nsp > 0) PI_CUDA(cudaMemsetAsync(f->vedge.p + nv, 0xff, sizeof(int2) * 12 * nsp, s));
-  const long long nt = read_int_finish(f);
+  const long long nt = rd.wait();
   // splash icosahedra after the surface (Mesh::AppendSplash_ConstR runs
   // after generate_mesh, src/surface_reconstructor.cpp:299-320)
   if (nsp > 0) splash_mesh(f, nv, nt);

@@ -292,8 +292,15 @@ void stage_hashgrid(pi_frame* f) {
   PI_LAUNCH(k_init_misc, 1, 32, 0, s, f->misc.p);
   int blocks = (int)std::min<long long>(div_up(n, 256), (long long)f->ctx->smCount * 2);
   PI_LAUNCH(k_bbox, blocks, 256, 0, s, f->xyz.p, n, f->misc.p);
-  unsigned h[8];
+  unsigned* const h = reinterpret_cast<unsigned*>(f->ctx->hpin + kPinReadOffset);
   PI_CUDA(cudaMemcpyAsync(h, f->misc.p, sizeof(unsigned) * 8, cudaMemcpyDeviceToHost, s));
+  // the buffers that do not depend on the box, while it is worked out
+  f->key.alloc(f->ctx, s, n);
+  f->sidx.alloc(f->ctx, s, n);
+  f->u32a.alloc(f->ctx, s, n);
+  f->u32b.alloc(f->ctx, s, n);
+  f->u32c.alloc(f->ctx, s, n / kSmallCell + 1);
+  f->pos.alloc(f->ctx, s, n);
   PI_CUDA(cudaStreamSynchronize(s));
   if (h[6]) throw std::invalid_argument("non-finite particle coordinate");
   float bb[6];
@@ -314,14 +321,8 @@ void stage_hashgrid(pi_frame* f) {
   // FindStartEnd stores keys in an int (src/hash_grid.cpp:105).
   g.cellNum = grid_cell_counts(g.bounding, cell, (1LL << 31) - 2, nn);
   g.nx = nn[0], g.ny = nn[1], g.nz = nn[2];
-  f->key.alloc(f->ctx, s, n);
-  f->sidx.alloc(f->ctx, s, n);
-  f->u32a.alloc(f->ctx, s, n);
-  f->u32b.alloc(f->ctx, s, n);
-  f->u32c.alloc(f->ctx, s, n / kSmallCell + 1);
   f->tmp.alloc(f->ctx, s, scan_tmp_ints(g.cellNum + 1));
   f->off.alloc(f->ctx, s, g.cellNum + 1);
-  f->pos.alloc(f->ctx, s, n);
   // misc[7]: particles outside the grid, misc[8]: cells above kSmallCell (both
   // zeroed by k_init_misc)
   int* const big = reinterpret_cast<int*>(f->u32c.p);
@@ -336,8 +337,6 @@ void stage_hashgrid(pi_frame* f) {
             f->u32a.p, f->u32b.p, f->off.p, g.cellNum, n, f->sidx.p, f->pos.p, big, f->misc.p + 8);
   // the valid-key count (offset table total) reaches g.nInvalid in
   // resolve_pending; nothing before the end of the call reads it
-  PI_CUDA(cudaMemcpyAsync(reinterpret_cast<int*>(f->ctx->hpin + (size_t)kPinSlots * kCounterWords),
-                          f->off.p + g.cellNum, sizeof(int), cudaMemcpyDeviceToHost, s));
   f->pin_pending |= 1 << kPinValid;
   // loadRootBox result kept for the octree root (resizeRootBoxConstR)
   for (int k2 = 0; k2 < 6; ++k2) f->bbox6[k2] = bb[k2];

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -22,6 +23,7 @@ template <class T>
 struct DBuf {
   T* p = nullptr;
   size_t n = 0;
+  size_t cap = 0;  // bytes of the block (from the context's kept blocks it may be larger)
   pi_ctx* ctx = nullptr;
   cudaStream_t s = nullptr;
   DBuf() = default;
@@ -60,6 +62,7 @@ struct GridHost {
 // Configurations of the chunked field evaluation at octree samples
 // (octree.cu): samples per lane, warps per block, staged candidates per warp.
 constexpr int kMaxQefParts = 64;  // pi_ctx_tune_qef_parts
+constexpr size_t kKeepBlock = 64u << 20, kKeepBytes = 256u << 20;  // kept blocks (pi_ctx::kept)
 
 struct EvalConfig {
   int K, W, CB, bulk;
@@ -74,6 +77,20 @@ struct pi_ctx {
   cudaStream_t stream = nullptr;
   size_t budget = 0;
   std::atomic<long long> used{0};
+  // Device blocks of released buffers, kept for the next buffer of about their
+  // size on the same stream (whose order makes the reuse safe, as it does for
+  // the pool): a small frame allocates sixty buffers, and the pool's calls sat
+  // between its short kernels.  Only without a budget, blocks up to
+  // kKeepBlock, kKeepBytes in all; given back when an allocation fails and when
+  // the context goes.  Not counted in `used`, as the pool's free memory is not.
+  struct KeptBlock {
+    void* p;
+    size_t bytes;
+    cudaStream_t s;
+  };
+  std::mutex keep_mu;
+  std::vector<KeptBlock> kept;
+  size_t kept_bytes = 0;
   bool profile = false;
   // per kernel group (ProfGroup): event pairs (start, stop) not read yet, and
   // the accumulated device time, launches, candidate pairs and work units
@@ -92,10 +109,9 @@ struct pi_ctx {
   int eval_cfg[2] = {0, 0};  // chosen configuration + 1 per dense level kind (0: not yet)
   int eval_forced = 0;
   int qef_parts = 16;  // leaf level with the QEF on: parts pipelined against the QEF stream (1: none)
-  // pinned host area for reads that need no synchronisation of their own:
-  // per-stage counter snapshots (kPinSlots x kCounterWords words) and one
-  // word for the hash grid's valid-key count; folded into the frame at the
-  // end of the API call that produced them
+  // pinned host area, written by the device: the counters and the hash grid's
+  // valid-key count (copied at the end of an API call), and the counts that size
+  // the next launches, which the kernels store there themselves
   unsigned long long* hpin = nullptr;
   // the frame pi_reconstruct reuses from call to call when the context has
   // no budget (its device buffers and events carry over); freed with the
@@ -208,7 +224,8 @@ struct pi_frame {
   long long doneEvals = 0;  // evaluations the kernels performed (after deduplication)
   long long qefAccepted = 0, qefSingular = 0;
   long long gridPairs = 0;  // candidate pairs of the last uniform-grid sampling
-  pisurf::DBuf<unsigned long long> dcount;  // device counters
+  pisurf::DBuf<unsigned long long> dcount;  // device counters, zeroed by the anisotropy stage
+  bool octree_counted = false, extract_counted = false;  // stages that have added to them since
   // stage timing: ev[2k], ev[2k+1] bracket stage slot k; the times are read
   // when the frame's next synchronisation point has passed
   cudaEvent_t ev[17] = {};
@@ -219,16 +236,18 @@ struct pi_frame {
   long long host_tcap = 0;
   bool tris_sent = false;
   int ev_pending = 0;   // bit k: slot k's events recorded, time not read yet
-  int pin_pending = 0;  // bit k: pinned slot k written by this call, not folded yet
+  int pin_pending = 0;  // bits kPin...: complete on the stream, not in the frame yet
   float stage_ms[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 };
 
 namespace pisurf {
 
-// pinned snapshot slots
-constexpr int kPinAniso = 0, kPinOctree = 1, kPinExtract = 2, kPinSlots = 3;
-constexpr int kPinValid = kPinSlots;  // bit of pin_pending for the valid-key count
-// after the slots: word 0 the valid-key count, word 1 the octree level's
+// bits of pin_pending: stages whose counters, and the valid-key count, are not
+// in the frame yet
+constexpr int kPinAniso = 0, kPinOctree = 1, kPinExtract = 2, kPinValid = 3;
+// pinned words: a snapshot of the counters;
+constexpr int kPinSlots = 1;
+// after it: word 0 the valid-key count, word 1 the octree level's
 // INTERNAL count; then the coarse levels' starts and INTERNAL count
 constexpr int kPinTopOffset = kPinSlots * kCounterWords + 8;
 constexpr int kPinTopWords = 32;
@@ -238,8 +257,8 @@ constexpr int kPinTopoReadOffset = kPinReadOffset + 8;
 constexpr int kPinWords = kPinTopoReadOffset + 8;
 // event that marks the INTERNAL count's copy in the octree level loop
 constexpr int kLevelEvent = 16;
-// Copies the frame's device counters into pinned slot `slot` (stream-ordered,
-// no synchronisation); the values reach the frame in resolve_pending.
+// The counters of a stage (kPin...) are complete on the context stream; they
+// reach the frame in resolve_pending, which copies them once for all stages.
 void counters_snapshot(pi_frame* f, int slot);
 // Parameter checks of pi_frame_create (throws std::invalid_argument).
 void check_params(const pi_params* p);
@@ -323,9 +342,11 @@ void dmc_host_table(int trans[256][8], bool flip[256], int code[256]);
 void prof_begin(pi_ctx* c, cudaStream_t s, int g);
 void prof_end(pi_ctx* c, cudaStream_t s, int g);
 
-// Striped device counters of a frame: zero them / read and sum the stripes
-// (synchronises the context stream).
-void counters_reset(pi_frame* f);
+// Striped device counters of a frame: zero some / the same when the stage that
+// adds to them runs again (the anisotropy stage zeroes all for the frame) / read
+// and sum the stripes (synchronises the context stream).
+void counters_reset(pi_frame* f, int first, int last);
+void counters_begin(pi_frame* f, bool* counted, int first, int last);
 void counters_read(pi_frame* f, unsigned long long out[kCounters]);
 
 // Host scalar constants with the reference's float/double semantics.

@@ -1031,7 +1031,7 @@ struct TopArgs {
   float cx, cy, cz, half;  // root
   int size;                // the root's edge in lattice units
   unsigned* flags;         // kTopWords: non-empty paths, a bit each
-  long long* lv;           // kPinTopWords: level starts, then the INTERNAL count of level D, then levels done
+  long long* lv;           // pinned, kPinTopWords: level starts, then the INTERNAL count of level D
   int* rank;               // level D: INTERNAL nodes before each node
   float4* nd_c;
   float4* nd_v;
@@ -1608,7 +1608,7 @@ static void stage_octree_vr(pi_frame* f) {
   PartView P{f->pos.p, f->xm.p, f->ga.p, f->gb.p, f->xlo.p};
   const int ekx = bn + 4, eky = bn + 4;
   const long long nb = (long long)ekx * eky * (bn + 4);
-  counters_reset(f);
+  counters_begin(f, &f->octree_counted, 0, C_STAGE_TIMEOUT);
   DBuf<int> flag, qcnt, qkey, rep, order, ucnt, ucum;
   DBuf<unsigned> hslot;
   DBuf<float> qval;
@@ -1665,9 +1665,8 @@ static void stage_octree_vr(pi_frame* f) {
     }
     flag.alloc(ctx, s, nl + 1);
     if (f->tmp.n < scan_tmp_ints(nl + 1)) f->tmp.alloc(ctx, s, scan_tmp_ints(nl + 1));
-    exclusive_scan(ScanOf<InternalNode>{{f->nd_type.p + lb}, nl}, flag.p, nl + 1, nullptr, f->tmp.p, s);
     int* const nint_h = reinterpret_cast<int*>(ctx->hpin + kPinSlots * kCounterWords + 1);
-    PI_CUDA(cudaMemcpyAsync(nint_h, flag.p + nl, sizeof(int), cudaMemcpyDeviceToHost, s));
+    exclusive_scan(ScanOf<InternalNode>{{f->nd_type.p + lb}, nl}, flag.p, nl + 1, nint_h, f->tmp.p, s);
     PI_CUDA(cudaEventRecord(f->ev[kLevelEvent], s));
     f->nNodes = le;
     ensure_nodes(f, le + 8 * nl);
@@ -1675,7 +1674,7 @@ static void stage_octree_vr(pi_frame* f) {
               f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p, f->nd_curv.p,
               f->nd_org.p);
     PI_CUDA(cudaEventSynchronize(f->ev[kLevelEvent]));
-    const int nint = *nint_h;
+    const int nint = *const_cast<const volatile int*>(nint_h);
     const long long newn = 8LL * nint;
     f->nNodes = le + newn;
     if (nint == 0 || depth >= f->dmax) break;
@@ -1706,13 +1705,14 @@ void stage_octree(pi_frame* f) {
   PartView P{f->pos.p, f->xm.p, f->ga.p, f->gb.p, f->xlo.p};
   const int ekx = gh.nx + 4, eky = gh.ny + 4;
   const long long ek = (long long)ekx * eky * (gh.nz + 4) * 8;  // buckets: cell x octant
-  counters_reset(f);
-  DBuf<int> flag, qcnt, qkey, rep, order, ucnt, ucum;
+  counters_begin(f, &f->octree_counted, 0, C_STAGE_TIMEOUT);
+  DBuf<int> flag, qcnt, qkey, rep, order, ucum;
   DBuf<unsigned> hslot;
   DBuf<int2> chunks;
   DBuf<float> qval;
-  qcnt.alloc(ctx, s, ek + 3);  // bucket counts, total, chunk count, chunks taken
-  ucnt.alloc(ctx, s, ek + 1);  // distinct points per bucket (+ 1 for the scan's total)
+  // bucket counts, total, chunk count, chunks taken; then, from the next multiple
+  // of 4, the distinct points per bucket (+ 1 for the scan's total)
+  qcnt.alloc(ctx, s, 2 * ek + 8);
   ucum.alloc(ctx, s, ek + 1);  // exclusive scan of ucnt (sparse levels)
   long long lb = 0, le = 1;
   bool known = false;  // emptiness and curvature of this level settled by the parents' scan
@@ -1734,12 +1734,11 @@ void stage_octree(pi_frame* f) {
   };
   int depth0 = 0;
   if (D >= 0) {
-    DBuf<long long> lvd;
     DBuf<unsigned> tflag;
-    lvd.alloc(ctx, s, kPinTopWords);
     tflag.alloc(ctx, s, kTopWords);
     flag.alloc(ctx, s, (size_t)1 << (3 * D));
     PI_CUDA(cudaMemsetAsync(tflag.p, 0, sizeof(unsigned) * kTopWords, s));
+    long long* const lvh = reinterpret_cast<long long*>(ctx->hpin + kPinTopOffset);  // stored by the kernel
     TopArgs ta{LevelArgs{g, f->pos.p, f->nrm.p, f->P.radius * f->P.smooth_factor, f->iso, f->P.radius, 0, 0, 1, P},
                D,
                top_spawn ? 1 : 0,
@@ -1749,7 +1748,7 @@ void stage_octree(pi_frame* f) {
                f->rootH,
                1 << f->dmax,
                tflag.p,
-               lvd.p,
+               lvh,
                flag.p,
                f->nd_c.p,
                f->nd_v.p,
@@ -1764,8 +1763,6 @@ void stage_octree(pi_frame* f) {
     const int wide = top_base(std::min(D, kTopBlockDepth) + 1), paths = top_base(D + 1);
     PI_LAUNCH(k_top_test, wide + div_up(paths - wide, kTopThreads / 32), kTopThreads, 0, s, ta);
     PI_LAUNCH(k_top_nodes, div_up(paths, kTopThreads), kTopThreads, 0, s, ta);
-    long long* const lvh = reinterpret_cast<long long*>(ctx->hpin + kPinTopOffset);
-    PI_CUDA(cudaMemcpyAsync(lvh, lvd.p, sizeof(long long) * (D + 4), cudaMemcpyDeviceToHost, s));
     PI_CUDA(cudaStreamSynchronize(s));
     for (int d = 0; d <= D; ++d)
       if (lvh[d + 1] > lvh[d]) f->levelBegin.push_back(lvh[d]);
@@ -1826,8 +1823,9 @@ void stage_octree(pi_frame* f) {
       qval.alloc(ctx, s, qn);
       order.alloc(ctx, s, qn);
       chunks.alloc(ctx, s, qn);
-      PI_CUDA(cudaMemsetAsync(qcnt.p, 0, sizeof(int) * (nb + 2), s));
-      PI_CUDA(cudaMemsetAsync(ucnt.p, 0, sizeof(int) * (nb + 1), s));
+      const long long ustart = (nb + 3 + 3) / 4 * 4;
+      int* const ucnt = qcnt.p + ustart;
+      PI_CUDA(cudaMemsetAsync(qcnt.p, 0, sizeof(int) * (ustart + nb + 1), s));
       PI_CUDA(cudaMemsetAsync(hslot.p, 0, sizeof(unsigned) * 2 * qn, s));
       // the leaf level (node size r, samples r/2 apart) holds about 50
       // distinct samples per cell octant, the level above about 50 per cell;
@@ -1839,19 +1837,19 @@ void stage_octree(pi_frame* f) {
       exclusive_scan_i32(qcnt.p, qcnt.p, nb + 1, nullptr, f->tmp.p, s);
       if (dense)
         PI_LAUNCH(k_q_dedupe<true>, div_up(qn, 256), 256, 0, s, qa, qn, f->nd_c.p, f->nd_v.p, qkey.p, qcnt.p, hslot.p,
-                  ucnt.p, rep.p, order.p);
+                  ucnt, rep.p, order.p);
       else
         PI_LAUNCH(k_q_dedupe<false>, div_up(qn, 256), 256, 0, s, qa, qn, f->nd_c.p, f->nd_v.p, qkey.p, qcnt.p,
-                  hslot.p, ucnt.p, rep.p, order.p);
+                  hslot.p, ucnt, rep.p, order.p);
       int* list = reinterpret_cast<int*>(hslot.p);  // the hash slots are free once the samples are placed
       if (!dense) {
-        exclusive_scan_i32(ucnt.p, ucum.p, nb + 1, nullptr, f->tmp.p, s);
+        exclusive_scan_i32(ucnt, ucum.p, nb + 1, nullptr, f->tmp.p, s);
         PI_LAUNCH(k_q_compact, div_up(qn, 256), 256, 0, s, qn, qkey.p, order.p, ucum.p, list);
       }
       const bool in_parts = dense && f->P.qef && depth == f->dmax && ctx->qef_parts > 1;
       int cfg = 0;
       if (dense)
-        cfg = eval_config_for(f, depth == f->dmax ? 0 : 1, qa, qn, nb, order.p, qcnt.p, ucnt.p, chunks.p,
+        cfg = eval_config_for(f, depth == f->dmax ? 0 : 1, qa, qn, nb, order.p, qcnt.p, ucnt, chunks.p,
                               qcnt.p + nb + 1, in_parts ? kQefReserveRegs : 0, qval.p);
       if (in_parts) {
         // the leaf level in parts: part p's QEF beside part p + 1's sampling
@@ -1870,13 +1868,13 @@ void stage_octree(pi_frame* f) {
                   f->plist.p);
         PI_LAUNCH(k_part_list, div_up(nl, kPartThreads), kPartThreads, 0, s, nl, parts, npart.p, f->plist.p,
                   f->pnodes.p);
-        PI_LAUNCH(k_q_chunks_parts, div_up(nb, 256), 256, 0, s, nb, ucnt.p, 32 * kEvalTable[cfg].K, parts, pinfo.p,
+        PI_LAUNCH(k_q_chunks_parts, div_up(nb, 256), 256, 0, s, nb, ucnt, 32 * kEvalTable[cfg].K, parts, pinfo.p,
                   chunks.p);
         for (int p = 0; p < parts; ++p) {
           prof_begin(ctx, s, PG_CHUNK);
           // the grid is sized by the level (a part may hold fewer slots than
           // it has parts, and the blocks stride over the part's chunks)
-          eval_chunks(f, cfg, qa, qn, order.p, qcnt.p, ucnt.p, chunks.p, pinfo.p + 2 * (parts + 1) + p,
+          eval_chunks(f, cfg, qa, qn, order.p, qcnt.p, ucnt, chunks.p, pinfo.p + 2 * (parts + 1) + p,
                       pinfo.p + parts + 1 + p, pinfo.p + 3 * (parts + 1) + p, kQefReserveRegs, qval.p, f->dcount.p);
           prof_end(ctx, s, PG_CHUNK);
           // a part holds about nl / parts nodes; the blocks stride over what it
@@ -1892,7 +1890,7 @@ void stage_octree(pi_frame* f) {
       const int pg = dense ? PG_CHUNK : PG_THREAD;
       prof_begin(ctx, s, pg);
       if (dense)
-        dense_eval(f, cfg, qa, qn, nb, order.p, qcnt.p, ucnt.p, chunks.p, qcnt.p + nb + 1, 0, qval.p, f->dcount.p);
+        dense_eval(f, cfg, qa, qn, nb, order.p, qcnt.p, ucnt, chunks.p, qcnt.p + nb + 1, 0, qval.p, f->dcount.p);
       else
         PI_LAUNCH(k_q_eval_thread, (int)std::min<long long>((long long)ctx->smCount * 8, div_up(qn, 256)), 256, 0,
                   s, qa, list, ucum.p + nb, f->nd_c.p, f->nd_v.p, qval.p, f->dcount.p);
@@ -1915,12 +1913,11 @@ void stage_octree(pi_frame* f) {
     }
     flag.alloc(ctx, s, nl + 1);
     if (f->tmp.n < scan_tmp_ints(nl + 1)) f->tmp.alloc(ctx, s, scan_tmp_ints(nl + 1));
-    exclusive_scan(ScanOf<InternalNode>{{f->nd_type.p + lb}, nl}, flag.p, nl + 1, nullptr, f->tmp.p, s);
-    // the number of INTERNAL nodes goes to pinned host memory and is read
-    // while the spawn kernel runs, so that the device is still busy when the
-    // host sizes the next level
     int* const nint_h = reinterpret_cast<int*>(ctx->hpin + kPinSlots * kCounterWords + 1);
-    PI_CUDA(cudaMemcpyAsync(nint_h, flag.p + nl, sizeof(int), cudaMemcpyDeviceToHost, s));
+    exclusive_scan(ScanOf<InternalNode>{{f->nd_type.p + lb}, nl}, flag.p, nl + 1, nint_h, f->tmp.p, s);
+    // the scan stores the number of INTERNAL nodes in pinned host memory; it is
+    // read while the spawn kernel runs, so that the device is still busy when
+    // the host sizes the next level
     PI_CUDA(cudaEventRecord(f->ev[kLevelEvent], s));
     f->nNodes = le;
     ensure_nodes(f, le + 8 * nl);  // room for the children: at most 8 per node of the level
@@ -1933,7 +1930,7 @@ void stage_octree(pi_frame* f) {
                 f->nd_curv.p, f->nd_org.p);
     }
     PI_CUDA(cudaEventSynchronize(f->ev[kLevelEvent]));
-    const int nint = *nint_h;
+    const int nint = *const_cast<const volatile int*>(nint_h);
     const long long newn = 8LL * nint;
     f->nNodes = le + newn;
     // depth D_max nodes are leaves by size, so nothing spawns past it

@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(32 * kGridWarps, 3) k_grid_eval(GridView g, Pa
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-  if (lane == 0 && pairs) stripe_add(counters, 1, (unsigned long long)pairs);
+  if (lane == 0 && pairs) stripe_add(counters, C_GRID_PAIRS, (unsigned long long)pairs);
 }
 
 // Host restatement of cell_coord (same IEEE float expression, truncation,
@@ -153,7 +153,7 @@ long long grid_sample(pi_frame* f, float* d_out, long long cap) {
     occ[dev] = nb > 0 ? nb : 1;
   }
   const int blocks = (int)std::min<long long>((long long)ctx->smCount * occ[dev], div_up(nchunks, kGridWarps));
-  counters_reset(f);
+  counters_reset(f, C_GRID_PAIRS, C_GRID_PAIRS);
   GridView g{gh.bounding[0], gh.bounding[2], gh.bounding[4], gh.cell, gh.nx, gh.ny, gh.nz, f->off.p};
   PartView P{f->pos.p, f->xm.p, f->ga.p, f->gb.p, f->xlo.p};
   prof_begin(ctx, s, PG_GRID);
@@ -161,7 +161,7 @@ long long grid_sample(pi_frame* f, float* d_out, long long cap) {
   prof_end(ctx, s, PG_GRID);
   unsigned long long cnt[kCounters];
   counters_read(f, cnt);
-  f->gridPairs = (long long)cnt[1];
+  f->gridPairs = (long long)cnt[C_GRID_PAIRS];
   return total;
 }
 

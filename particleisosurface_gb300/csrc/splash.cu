@@ -45,10 +45,10 @@ void stage_splash_list(pi_frame* f) {
   tmp.alloc(c, s, scan_tmp_ints(n + 1));
   PI_CUDA(cudaMemsetAsync(flag.p + n, 0, sizeof(int), s));
   PI_LAUNCH(k_splash_mark, div_up(n, 256), 256, 0, s, f->spl.p, f->sidx.p, n, f->pos.p, flag.p);
-  exclusive_scan_i32(flag.p, flag.p, n + 1, nullptr, tmp.p, s);
-  int total = 0;
-  PI_CUDA(cudaMemcpyAsync(&total, flag.p + n, sizeof(int), cudaMemcpyDeviceToHost, s));
+  int* const total_h = reinterpret_cast<int*>(c->hpin + kPinReadOffset);  // stored by the scan
+  exclusive_scan_i32(flag.p, flag.p, n + 1, total_h, tmp.p, s);
   PI_CUDA(cudaStreamSynchronize(s));
+  const int total = *const_cast<const volatile int*>(total_h);
   f->nSplash = total;
   f->splList.alloc(c, s, total > 0 ? total : 1);
   PI_LAUNCH(k_splash_list, div_up(n, 256), 256, 0, s, f->spl.p, f->sidx.p, n, flag.p, f->splList.p);
