@@ -50,6 +50,7 @@ __device__ __forceinline__ float d2_exact(float dx, float dy, float dz) {
 __global__ void k_xmean(GridView g, const float4* __restrict__ pos, long long n, float nI, float nI2,
                         float inv_h3, float c_mean, float4* __restrict__ xm, float4* __restrict__ xlo,
                         int8_t* __restrict__ spl) {
+  launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   float4 p = pos[t];
@@ -171,6 +172,7 @@ __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __re
                         float4* __restrict__ ga, float4* __restrict__ gb, float* __restrict__ gfull,
                         float* __restrict__ det_out, int8_t* __restrict__ f64flag,
                         unsigned long long* __restrict__ f64count, const int8_t* __restrict__ spl) {
+  launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   float4 p = pos[t];
@@ -278,6 +280,7 @@ __global__ void __launch_bounds__(128) k_vr_xmean(const MultiGridView* __restric
                                                   const float4* __restrict__ pos, const float4* __restrict__ vrc,
                                                   long long n, float c_mean, float4* __restrict__ xm,
                                                   float4* __restrict__ xlo) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const MultiGridView& m = *mg;
@@ -330,6 +333,7 @@ __global__ void __launch_bounds__(128) k_vr_cov_G(const MultiGridView* __restric
                                                   float4* __restrict__ ga, float4* __restrict__ gb,
                                                   float* __restrict__ gfull, float* __restrict__ det_out,
                                                   int8_t* __restrict__ f64flag, unsigned long long* __restrict__ f64count) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const MultiGridView& m = *mg;

@@ -7,6 +7,7 @@
 #include <cstdio>
 #include <stdexcept>
 #include <string>
+#include <utility>
 
 namespace pisurf {
 
@@ -37,13 +38,38 @@ struct CudaError : std::runtime_error {
   } while (0)
 
 // Launch wrapper: counts the launch and checks the launch error.
-#define PI_LAUNCH(kernel, grid, block, smem, stream, ...)                 \
-  do {                                                                    \
-    if ((grid) > 0) {                                                     \
-      kernel<<<(grid), (block), (smem), (stream)>>>(__VA_ARGS__);         \
-      ::pisurf::count_launch();                                           \
-      PI_CUDA(cudaGetLastError());                                        \
-    }                                                                     \
+// Programmatic stream serialization: a kernel is brought up while the one before
+// it on the stream drains, and every kernel begins with launch_wait(), where it
+// waits until that one is complete and its writes are visible, before it touches
+// memory.  A small frame is a chain of some sixty kernels of a few microseconds:
+// 2,000 particles 758 -> 649 us, 20,000 1109 -> 972, 151,000 1457 -> 1297.  No
+// kernel lets its successor start before its blocks exit
+// (griddepcontrol.launch_dependents): the successor's waiting blocks then hold
+// the SM slots that the kernels of the other streams fill (dam break with the
+// QEF 13.98 -> 15.39 ms, small frames no faster).
+__device__ __forceinline__ void launch_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... KA, class... A>
+inline void launch_kernel(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  PI_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(std::forward<A>(args))...));
+}
+
+#define PI_LAUNCH(kernel, grid, block, smem, stream, ...)                              \
+  do {                                                                                 \
+    if ((grid) > 0) {                                                                  \
+      ::pisurf::launch_kernel(kernel, (grid), (block), (smem), (stream), __VA_ARGS__); \
+      ::pisurf::count_launch();                                                        \
+    }                                                                                  \
   } while (0)
 
 inline unsigned int div_up(long long a, long long b) { return (unsigned int)((a + b - 1) / b); }

@@ -100,6 +100,7 @@ struct WordBits {
 // boundary corners, and those of nodes that are no leaves, get the all-ones key.
 __global__ void k_corner_keys(const int* __restrict__ nd_child, long long nn, const int4* __restrict__ nd_org,
                               int full, int B, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
+  launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nn * 8) return;
   const int4 o = nd_org[t >> 3];
@@ -222,6 +223,7 @@ __device__ __forceinline__ void merge_axis(unsigned in, const long long (&code)[
 // used[block] = 1 for every block that holds a corner.
 __global__ void k_block_mark(const int* __restrict__ nd_child, long long nf, const int4* __restrict__ nd_org, int full,
                              int bb, int* __restrict__ used) {
+  launch_wait();
   Family fam;
   if (!load_family(nd_child, nd_org, nf, (long long)blockIdx.x * blockDim.x + threadIdx.x, full, fam)) return;
   long long last = -1;
@@ -235,12 +237,14 @@ __global__ void k_block_mark(const int* __restrict__ nd_child, long long nf, con
 // slot -> block (the inverse of the scan of used)
 __global__ void k_block_list(long long nb, const int* __restrict__ used, const int* __restrict__ slot,
                              long long* __restrict__ blist) {
+  launch_wait();
   const long long b = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (b < nb && used[b]) blist[slot[b]] = b;
 }
 
 __global__ void k_corner_mark(const int* __restrict__ nd_child, long long nf, const int4* __restrict__ nd_org,
                               int full, int bb, const int* __restrict__ slot, unsigned* __restrict__ bits) {
+  launch_wait();
   Family fam;
   if (!load_family(nd_child, nd_org, nf, (long long)blockIdx.x * blockDim.x + threadIdx.x, full, fam)) return;
   auto mark = [&](long long code, unsigned m) {  // code: of any point of the word
@@ -272,6 +276,7 @@ __global__ void k_corner_mark(const int* __restrict__ nd_child, long long nf, co
 
 __global__ void k_bitmap_keys(const unsigned* __restrict__ bits, long long nw, const int* __restrict__ off, int bb,
                               const long long* __restrict__ blist, int B, uint64_t* __restrict__ out) {
+  launch_wait();
   long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (w >= nw) return;
   unsigned b = bits[w];
@@ -308,6 +313,7 @@ __device__ __forceinline__ uint32_t mix64to32(uint64_t k) {
 // lines, were slower (212 us: the probes of near keys run into one another).
 __global__ void k_vkey_insert(long long ns, const uint64_t* __restrict__ khi, const uint64_t* __restrict__ klo,
                               uint32_t mask, unsigned* __restrict__ tab, uint32_t* __restrict__ where) {
+  launch_wait();
   long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= ns) return;
   const uint64_t lo = klo[s], hi = khi ? khi[s] : 0ull;
@@ -338,6 +344,7 @@ __device__ __forceinline__ void sorted3(const int* o, int& s0, int& s1, int& s2)
 
 __global__ void k_tri_insert(long long nt, const int* __restrict__ otri, uint32_t mask, unsigned* __restrict__ tab,
                              uint32_t* __restrict__ where) {
+  launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   int s0, s1, s2;
@@ -365,6 +372,7 @@ __global__ void k_tri_insert(long long nt, const int* __restrict__ otri, uint32_
 // flag[s] = 1 where slot s is its key's first (lowest) slot
 __global__ void k_first_flag(long long n, const unsigned* __restrict__ tab, const uint32_t* __restrict__ where,
                              int* __restrict__ flag) {
+  launch_wait();
   long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s < n) flag[s] = tab[where[s]] == (unsigned)s + 1u ? 1 : 0;
   if (s == n) flag[s] = 0;
@@ -396,6 +404,7 @@ static void rank_first(long long n, const unsigned* tab, const uint32_t* where, 
 // slot -> vertex (numbered in order of first slots); vertex -> its first slot
 __global__ void k_vertex_map(long long ns, const unsigned* __restrict__ tab, const uint32_t* __restrict__ where,
                              const int* __restrict__ rank, int* __restrict__ slot_vertex, int* __restrict__ rep) {
+  launch_wait();
   long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= ns) return;
   const long long first = (long long)tab[where[s]] - 1;
@@ -406,6 +415,7 @@ __global__ void k_vertex_map(long long ns, const unsigned* __restrict__ tab, con
 
 __global__ void k_tri_write(long long nt, const int* __restrict__ rank, const int* __restrict__ otri,
                             int* __restrict__ out) {
+  launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const int o = rank[t];
@@ -417,6 +427,7 @@ __global__ void k_tri_write(long long nt, const int* __restrict__ rank, const in
 
 __global__ void k_unique_flag(const uint64_t* __restrict__ keys, long long n, uint64_t invalid,
                               int* __restrict__ flag) {
+  launch_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i > n) return;
   if (i == n) {
@@ -429,6 +440,7 @@ __global__ void k_unique_flag(const uint64_t* __restrict__ keys, long long n, ui
 
 __global__ void k_unique_write(const uint64_t* __restrict__ keys, const int* __restrict__ scan, long long n,
                                uint64_t invalid, uint64_t* __restrict__ out) {
+  launch_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint64_t k = keys[i];
@@ -445,6 +457,7 @@ __global__ void k_unique_write(const uint64_t* __restrict__ keys, const int* __r
 __global__ void k_dual(const uint64_t* __restrict__ verts, long long nu, int B, const int* __restrict__ nd_child,
                        const float4* __restrict__ nd_v, int* __restrict__ cells,
                        uint8_t* __restrict__ procs, int* __restrict__ tcount, unsigned long long* __restrict__ ndual) {
+  launch_wait();
   long long u = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (u > nu) return;
   if (u == nu) {
@@ -512,6 +525,7 @@ __global__ void __launch_bounds__(kSlotThreads) k_tri_slots(long long nu, const 
                                                             int* __restrict__ slotA, int* __restrict__ slotB,
                                                             uint64_t* __restrict__ khi, uint64_t* __restrict__ klo,
                                                             int8_t* __restrict__ tflip) {
+  launch_wait();
   __shared__ int s_off[kSlotThreads + 1];
   const long long u0 = (long long)blockIdx.x * kSlotThreads;
   const int nloc = (int)(nu - u0 < kSlotThreads ? nu - u0 : kSlotThreads);
@@ -571,6 +585,7 @@ __device__ __forceinline__ int vertex_cell(const BisectArgs& a, const float4& p,
 __global__ void k_vcell_count(BisectArgs a, long long nv, const int* __restrict__ rep, const int* __restrict__ slotA,
                               const int* __restrict__ slotB, const float4* __restrict__ nd_v, int ekx, int eky,
                               int* __restrict__ cnt, int* __restrict__ key) {
+  launch_wait();
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   int k = -1;
@@ -585,6 +600,7 @@ __global__ void k_vcell_count(BisectArgs a, long long nv, const int* __restrict_
 
 __global__ void k_vcell_place(long long nv, const int* __restrict__ key, const int* __restrict__ off,
                               int* __restrict__ fill, int* __restrict__ list) {
+  launch_wait();
   const long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const int k = v < nv ? key[v] : -1;
@@ -604,6 +620,7 @@ __global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, c
                          const uint64_t* __restrict__ nd_id, float* __restrict__ out,
                          uint64_t* __restrict__ vkeys, int2* __restrict__ vedge,
                          unsigned long long* __restrict__ counters) {
+  launch_wait();
   __shared__ __align__(16) float s_stage[VR ? 1 : kGroupWarps][VR ? 1 : GroupRoom<32>::kFloats];
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = t < nv;
@@ -668,6 +685,7 @@ __global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, c
 // Oriented triangle in Mesh::insert_tri argument order.
 __global__ void k_tri_orient(long long nt, const int* __restrict__ slot_vertex, const int8_t* __restrict__ tflip,
                              int* __restrict__ otri) {
+  launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const int a = slot_vertex[3 * t], b = slot_vertex[3 * t + 1], c = slot_vertex[3 * t + 2];

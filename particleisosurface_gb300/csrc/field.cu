@@ -61,6 +61,7 @@ __device__ __forceinline__ void grad_sum(const GridView& g, const PartView& P, f
 }
 
 __global__ void __launch_bounds__(128, 12) k_normals(GridView g, PartView P, long long n, float gscale, float4* __restrict__ nrm) {
+  launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   float4 p = P.pos[t];
@@ -129,6 +130,7 @@ __device__ __forceinline__ float field_grad_sum(const GridView& g, const PartVie
 // clamps) and its place among the cell's points.
 __global__ void k_point_cell(GridView g, const float* __restrict__ pts, long long m, int* __restrict__ cnt,
                              int2* __restrict__ at) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   int cx, cy, cz;
@@ -139,6 +141,7 @@ __global__ void k_point_cell(GridView g, const float* __restrict__ pts, long lon
 
 __global__ void k_point_order(const int2* __restrict__ at, const int* __restrict__ off, long long m,
                               int* __restrict__ order) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const int2 a = at[i];
@@ -153,6 +156,7 @@ __global__ void k_point_order(const int2* __restrict__ at, const int* __restrict
 __global__ void __launch_bounds__(128) k_eval_points(GridView g, PartView P, const float* __restrict__ pts,
                                                      const int* __restrict__ order, long long m, float iso,
                                                      float gscale, float* __restrict__ val, float* __restrict__ grad) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= m) return;
   const long long i = order ? order[t] : t;
@@ -221,6 +225,7 @@ __device__ __forceinline__ void grad_sum_vr(const MultiGridView& m, const PartVi
 
 __global__ void __launch_bounds__(128) k_vr_normals(const MultiGridView* __restrict__ mg, PartView P, long long n,
                                                     float4* __restrict__ nrm) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const float4 p = P.pos[t];
@@ -231,6 +236,7 @@ __global__ void __launch_bounds__(128) k_vr_normals(const MultiGridView* __restr
 
 __global__ void k_vr_eval_points(const MultiGridView* __restrict__ mg, PartView P, const float* __restrict__ pts,
                                  long long m, float iso, float* __restrict__ val, float* __restrict__ grad) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const float qx = pts[3 * i], qy = pts[3 * i + 1], qz = pts[3 * i + 2];
@@ -240,6 +246,7 @@ __global__ void k_vr_eval_points(const MultiGridView* __restrict__ mg, PartView 
 
 __global__ void k_vr_nb_count(const MultiGridView* __restrict__ mg, const float* __restrict__ pts, long long m,
                               int* __restrict__ cnt) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const MultiGridView& v = *mg;
@@ -259,6 +266,7 @@ __global__ void k_vr_nb_count(const MultiGridView* __restrict__ mg, const float*
 
 __global__ void k_vr_nb_fill(const MultiGridView* __restrict__ mg, const float* __restrict__ pts, long long m,
                              const int* __restrict__ off, const uint32_t* __restrict__ sidx, int* __restrict__ out) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const MultiGridView& v = *mg;
@@ -328,6 +336,7 @@ void eval_points(pi_frame* f, const float* d_pts, long long m, float* d_val, flo
 
 // GetPIdxList: counts, then lists (particle indices through IndexList).
 __global__ void k_nb_count(GridView g, const float* __restrict__ pts, long long m, int* __restrict__ cnt) {
+  launch_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   int cx, cy, cz;
@@ -343,6 +352,7 @@ __global__ void k_nb_count(GridView g, const float* __restrict__ pts, long long 
 
 __global__ void k_nb_fill(GridView g, const float* __restrict__ pts, long long m, const int* __restrict__ off,
                           const uint32_t* __restrict__ sidx, int* __restrict__ out) {
+  launch_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   int cx, cy, cz;
@@ -394,6 +404,7 @@ long long neighbors(pi_frame* f, const float* h_pts, long long m, long long* h_o
 __global__ void k_in_box(GridView g, float b1x, float b1y, float b1z, float b2x, float b2y, float b2z,
                          float B1, float B3, float B5, const uint32_t* __restrict__ sidx, int* __restrict__ out,
                          long long cap, long long* __restrict__ total) {
+  launch_wait();
   b1x = fmaxf(b1x, g.b0);
   b1y = fmaxf(b1y, g.b2);
   b1z = fmaxf(b1z, g.b4);

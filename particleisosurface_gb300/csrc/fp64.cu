@@ -101,6 +101,7 @@ __device__ void jacobi_eig3_d(double A[3][3], double V[3][3]) {
 
 __global__ void k_f64_xmean(GridView g, const float4* __restrict__ pos, long long n, F64Consts k,
                             double* __restrict__ x64, int8_t* __restrict__ spl64) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const float4 pf = pos[t];
@@ -145,6 +146,7 @@ __global__ void k_f64_xmean(GridView g, const float4* __restrict__ pos, long lon
 __global__ void k_f64_G(GridView g, const float4* __restrict__ pos, long long n, F64Consts k,
                         const double* __restrict__ x64, const int8_t* __restrict__ spl64, double* __restrict__ g64,
                         double* __restrict__ det64) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   if (spl64 && spl64[t]) {  // splash: pass 1's identity
@@ -199,6 +201,7 @@ __global__ void k_f64_eval(GridView g, long long m, const float* __restrict__ pt
                            const double* __restrict__ x64, const double* __restrict__ g64,
                            const double* __restrict__ det64, const int8_t* __restrict__ spl64,
                            double* __restrict__ val, double* __restrict__ grad) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const float qf[3] = {pts[3 * i], pts[3 * i + 1], pts[3 * i + 2]};
@@ -232,6 +235,7 @@ __global__ void k_f64_eval(GridView g, long long m, const float* __restrict__ pt
 // sorted order -> original particle order, `w` doubles per particle
 __global__ void k_f64_unsort(const double* __restrict__ src, const uint32_t* __restrict__ sidx, long long n, int w,
                              double* __restrict__ dst) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const long long i = sidx[t];

@@ -28,6 +28,7 @@ static inline float fdec(unsigned e) {
 // misc[0..5] = enc(min x, max x, min y, max y, min z, max z); misc[6] = count
 // of non-finite coordinates.
 __global__ void k_bbox(const float* __restrict__ xyz, long long n, unsigned* __restrict__ misc) {
+  launch_wait();
   unsigned mn[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu}, mx[3] = {0u, 0u, 0u};
   unsigned bad = 0;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -81,6 +82,7 @@ __global__ void k_bbox(const float* __restrict__ xyz, long long n, unsigned* __r
 }
 
 __global__ void k_init_misc(unsigned* misc) {
+  launch_wait();
   int t = threadIdx.x;
   if (t < 6) misc[t] = (t & 1) ? 0u : 0xffffffffu;
   if (t >= 6 && t < 16) misc[t] = 0;
@@ -92,6 +94,7 @@ __global__ void k_init_misc(unsigned* misc) {
 __global__ void k_keys(const float* __restrict__ xyz, long long n, float b0, float b2, float b4,
                        float cell, int nx, int ny, int nz, int* __restrict__ key,
                        uint32_t* __restrict__ skey, uint32_t* __restrict__ sidx) {
+  launch_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
@@ -107,6 +110,7 @@ __global__ void k_keys(const float* __restrict__ xyz, long long n, float b0, flo
 }
 
 __global__ void k_cell_count(const int* __restrict__ key, long long n, int* __restrict__ cnt) {
+  launch_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int k = key[i];
@@ -130,6 +134,7 @@ constexpr int kSmallCell = 256;  // larger cells are radix-sorted by a block eac
 __global__ void k_cell_place(const float* __restrict__ xyz, long long n, float b0, float b2, float b4, float cell,
                              int nx, int ny, int nz, int* __restrict__ key, int* __restrict__ cnt,
                              unsigned* __restrict__ outside, uint32_t* __restrict__ place) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int cx = (int)__fdiv_rn(__fsub_rn(xyz[3 * i], b0), cell);
@@ -151,6 +156,7 @@ __device__ __forceinline__ void cell_range(const int* __restrict__ off, long lon
 
 __global__ void k_cell_scatter(const int* __restrict__ key, const uint32_t* __restrict__ place,
                                const int* __restrict__ off, long long cells, long long n, uint32_t* __restrict__ list) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   int s, e;
@@ -170,6 +176,7 @@ __global__ void k_cell_sort(const float* __restrict__ xyz, const int* __restrict
                             const uint32_t* __restrict__ list, const int* __restrict__ off, long long cells,
                             long long n, uint32_t* __restrict__ sidx, float4* __restrict__ pos, int* __restrict__ big,
                             unsigned* __restrict__ nbig) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const uint32_t i = list[t];
@@ -194,6 +201,7 @@ __global__ void __launch_bounds__(kBigThreads) k_cell_sort_big(const float* __re
                                                                uint32_t* __restrict__ sidx, float4* __restrict__ pos,
                                                                const int* __restrict__ big,
                                                                const unsigned* __restrict__ nbig) {
+  launch_wait();
   constexpr int warps = kBigThreads / 32;
   __shared__ int s_run[256];
   __shared__ int s_cnt[warps][256];

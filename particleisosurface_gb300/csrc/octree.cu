@@ -131,6 +131,7 @@ __device__ __forceinline__ int block_cells(const GrownBox& b) {
 
 __global__ void k_empty(LevelArgs a, const float4* __restrict__ nd_c, float4* __restrict__ nd_v,
                         int8_t* __restrict__ nd_type, float* __restrict__ nd_curv) {
+  launch_wait();
   const long long node = a.lb + (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (node >= a.le) return;
@@ -211,6 +212,7 @@ __global__ void __launch_bounds__(kCountThreads) k_q_count_node(QArgs a, const f
                                                                 const float4* __restrict__ nd_v,
                                                                 const int8_t* __restrict__ nd_type,
                                                                 int* __restrict__ qcnt, int* __restrict__ qkey) {
+  launch_wait();
   __shared__ int s_key[kCountThreads * kQ];
   const long long t0 = (long long)blockIdx.x * kCountThreads;
   const long long node = a.lb + t0 + threadIdx.x;
@@ -291,6 +293,7 @@ __device__ __forceinline__ uint32_t hash3(float x, float y, float z) {
 // Zeroes the hash slots of a level, two per sample counted (total = the scan's):
 // the samples of empty nodes have none, which are half of a leaf level's.
 __global__ void __launch_bounds__(256) k_q_clear(unsigned* __restrict__ hslot, const int* __restrict__ total) {
+  launch_wait();
   const long long quads = (2LL * *total + 3) / 4;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < quads;
        i += (long long)gridDim.x * blockDim.x)
@@ -315,6 +318,7 @@ template <bool DENSE>
 __global__ void k_q_dedupe(QArgs a, unsigned n, const float4* __restrict__ nd_c, const float4* __restrict__ nd_v,
                            const int* __restrict__ qkey, const int* __restrict__ qoff, unsigned* __restrict__ hslot,
                            int* __restrict__ ucnt, int* __restrict__ rep, int* __restrict__ order) {
+  launch_wait();
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const int k = i < n ? qkey[i] : -1;
@@ -374,6 +378,7 @@ __global__ void k_q_dedupe(QArgs a, unsigned n, const float4* __restrict__ nd_c,
 // `chunk` places (bucket, first place); list order is arbitrary.
 __global__ void k_q_chunks(long long nb, const int* __restrict__ ucnt, int chunk, int2* __restrict__ chunks,
                            int* __restrict__ nchunks) {
+  launch_wait();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const int u = k < nb ? ucnt[k] : 0;
@@ -402,6 +407,7 @@ __global__ void k_q_chunks(long long nb, const int* __restrict__ ucnt, int chunk
 // slots), the chunk counts cnt[0 .. parts - 1] and the chunks taken by the
 // evaluation's warps.
 __global__ void k_part_bounds(const int* __restrict__ qoff, int nb, int parts, int* __restrict__ pinfo) {
+  launch_wait();
   const int p = threadIdx.x;
   if (p > parts) return;
   int k = p == parts ? nb : 0;
@@ -440,6 +446,7 @@ constexpr int kPartThreads = 256;
 __global__ void __launch_bounds__(kPartThreads) k_node_part(long long nl, const int* __restrict__ qkey,
                                                             const int* __restrict__ pinfo, int parts,
                                                             int8_t* __restrict__ npart, int* __restrict__ plist) {
+  launch_wait();
   __shared__ int s_count[kMaxQefParts];
   const long long t = (long long)blockIdx.x * kPartThreads + threadIdx.x;
   if (threadIdx.x < kMaxQefParts) s_count[threadIdx.x] = 0;
@@ -460,6 +467,7 @@ __global__ void __launch_bounds__(kPartThreads) k_node_part(long long nl, const 
 // classification and 15 for the leaf list, 1 ms of a 16-part 1M frame.
 __global__ void __launch_bounds__(kPartThreads) k_part_list(long long nl, int parts, const int8_t* __restrict__ npart,
                                                             int* __restrict__ plist, int* __restrict__ list) {
+  launch_wait();
   __shared__ int s_count[kMaxQefParts], s_base[kMaxQefParts];
   const long long t = (long long)blockIdx.x * kPartThreads + threadIdx.x;
   if (threadIdx.x < kMaxQefParts) s_count[threadIdx.x] = 0;
@@ -482,6 +490,7 @@ __global__ void __launch_bounds__(kPartThreads) k_part_list(long long nl, int pa
 // the list, cnt[p] of them (one atomic per part and warp).
 __global__ void k_q_chunks_parts(long long nb, const int* __restrict__ ucnt, int chunk, int parts,
                                  int* __restrict__ pinfo, int2* __restrict__ chunks) {
+  launch_wait();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const int u = k < nb ? ucnt[k] : 0;
@@ -530,6 +539,7 @@ __global__ void __launch_bounds__(32 * W, (K > 2 ? 24 : 32) / W) k_q_eval(QArgs 
                                                             const float4* __restrict__ nd_v,
                                                             float* __restrict__ qval,
                                                             unsigned long long* __restrict__ counters) {
+  launch_wait();
   __shared__ __align__(16) float s_stage[W][stage_floats(CB)];
   __shared__ __align__(16) float4 s_bulk[BULK ? W : 1][BULK ? 4 * kBulkCap : 1];
   __shared__ __align__(8) uint64_t s_bar[W];
@@ -605,6 +615,7 @@ __global__ void __launch_bounds__(256, 4) k_q_eval_thread(QArgs a, const int* __
                                                        const float4* __restrict__ nd_c,
                                                        const float4* __restrict__ nd_v, float* __restrict__ qval,
                                                        unsigned long long* __restrict__ counters) {
+  launch_wait();
   const int n = *count_ptr;
   long long pairs = 0, done = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
@@ -637,6 +648,7 @@ __global__ void __launch_bounds__(256, 4) k_q_eval_thread(QArgs a, const int* __
 // sparse levels of the 1M dam break, whose buckets hold a few samples each).
 __global__ void k_q_compact(long long n, const int* __restrict__ qkey, const int* __restrict__ place,
                             const int* __restrict__ ucum, int* __restrict__ list) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int p = place[i];
@@ -651,6 +663,7 @@ __global__ void k_q_compact(long long n, const int* __restrict__ qkey, const int
 __global__ void __launch_bounds__(32 * kGroupWarps, 8) k_leaf_level(LevelArgs a, const float4* __restrict__ nd_c,
                                                        float4* __restrict__ nd_v, int8_t* __restrict__ nd_type,
                                                        unsigned long long* __restrict__ counters) {
+  launch_wait();
   __shared__ __align__(16) float s_stage[kGroupWarps][GroupRoom<8>::kFloats];
   float* const st = s_stage[threadIdx.x >> 5];
   long long pairs = 0, evals = 0;
@@ -687,6 +700,7 @@ __global__ void __launch_bounds__(64, 24) k_classify(LevelArgs a, const float* _
                            float4* __restrict__ nd_v, int8_t* __restrict__ nd_type, int8_t* __restrict__ nd_sc,
                            float* __restrict__ nd_curv, float* __restrict__ nd_samp, int qef, int curv_known,
                            unsigned long long* __restrict__ counters, const float* __restrict__ nd_minr) {
+  launch_wait();
   const long long node = a.lb + (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (node >= a.le) return;
@@ -772,6 +786,7 @@ __global__ void __launch_bounds__(256) k_classify_thread(LevelArgs a, const floa
                                                          unsigned long long* __restrict__ counters,
                                                          const int* __restrict__ plist, const int* __restrict__ list,
                                                          int parts, int part) {
+  launch_wait();
   __shared__ float s_val[kClassifyNodes * kRunPad];
   __shared__ int s_node[kClassifyNodes];  // node - lb, -1: none or no samples
   const long long n = plist ? plist[part] : a.le - a.lb;
@@ -838,6 +853,7 @@ __global__ void k_spawn(long long lb, long long le, long long cbase, const int* 
                         float4* __restrict__ nd_v, uint64_t* __restrict__ nd_id, int* __restrict__ nd_parent,
                         int* __restrict__ nd_child, int8_t* nd_ctype, int8_t* __restrict__ nd_depth,
                         int8_t* __restrict__ nd_sc, float* __restrict__ nd_curv, int4* __restrict__ nd_org) {
+  launch_wait();
   long long i = lb + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= le) return;
   if (nd_type[i] != T_INTERNAL) {
@@ -881,6 +897,7 @@ __global__ void __launch_bounds__(32 * kSpawnWarps, CURV ? 16 : 24) k_spawn_scan
                                                     int8_t* nd_type, int8_t* __restrict__ nd_depth,
                                                     int8_t* __restrict__ nd_sc, float* __restrict__ nd_curv,
                                                     int4* __restrict__ nd_org) {
+  launch_wait();
   __shared__ int s_row[kSpawnWarps][32];  // row starting at each element position of a batch
   const long long i = a.lb + (long long)blockIdx.x * kSpawnWarps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
@@ -1077,6 +1094,7 @@ __device__ __forceinline__ float4 top_centre(const TopArgs& t, int d, int id, in
 }
 
 __global__ void __launch_bounds__(kTopThreads) k_top_test(TopArgs t) {
+  launch_wait();
   __shared__ int s_found;
   constexpr int warps = kTopThreads / 32;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1121,6 +1139,7 @@ __global__ void __launch_bounds__(kTopThreads) k_top_test(TopArgs t) {
 }
 
 __global__ void __launch_bounds__(kTopThreads) k_top_nodes(TopArgs t) {
+  launch_wait();
   __shared__ unsigned s_flag[kTopWords];
   __shared__ int s_pre[kTopWords];  // INTERNAL nodes of the word's level before the word
   __shared__ int s_warp[kTopThreads / 32];
@@ -1227,6 +1246,7 @@ __global__ void __launch_bounds__(kTopThreads) k_top_nodes(TopArgs t) {
 __global__ void k_root(float cx, float cy, float cz, float h, int size, float4* nd_c, float4* nd_v,
                        uint64_t* nd_id, int* nd_parent, int* nd_child, int8_t* nd_type, int8_t* nd_depth,
                        int8_t* nd_sc, float* nd_curv, int4* nd_org) {
+  launch_wait();
   nd_c[0] = make_float4(cx, cy, cz, h);
   nd_v[0] = make_float4(cx, cy, cz, 0.f);
   nd_id[0] = 0;
@@ -1388,6 +1408,7 @@ __global__ void __launch_bounds__(64) k_vr_empty(const MultiGridView* __restrict
                                                  float emax, const float4* __restrict__ nd_c,
                                                  float4* __restrict__ nd_v, int8_t* __restrict__ nd_type,
                                                  float* __restrict__ nd_curv, float* __restrict__ nd_minr) {
+  launch_wait();
   const long long node = a.lb + (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (node >= a.le) return;
@@ -1469,6 +1490,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kWideThreads)
     k_vr_empty_wide(const MultiGridView* __restrict__ mg, LevelArgs a, float emax, const float4* __restrict__ nd_c,
                     float4* __restrict__ nd_v, int8_t* __restrict__ nd_type, float* __restrict__ nd_curv,
                     float* __restrict__ nd_minr) {
+  launch_wait();
   namespace cg = cooperative_groups;
   constexpr int warps = kWideThreads / 32;
   __shared__ float s_part[warps][6];  // found, min radius, normal sums, area
@@ -1560,6 +1582,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(kWideThreads)
 // 245-253).
 __global__ void k_vr_big_leaf(const MultiGridView* __restrict__ mg, LevelArgs a, float4* __restrict__ nd_v,
                               int8_t* __restrict__ nd_type, unsigned long long* __restrict__ counters) {
+  launch_wait();
   const long long node = a.lb + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (node >= a.le || nd_type[node] != T_UNCERTAIN) return;
   float4 v = nd_v[node];
@@ -1578,6 +1601,7 @@ __global__ void __launch_bounds__(256, 4) k_vr_q_eval_thread(const MultiGridView
                                                              const float4* __restrict__ nd_c,
                                                              const float4* __restrict__ nd_v, float* __restrict__ qval,
                                                              unsigned long long* __restrict__ counters) {
+  launch_wait();
   const int n = *count_ptr;
   long long pairs = 0, done = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {

@@ -284,6 +284,7 @@ __device__ int ldlt4(const double A[4][4], double floor, double d[4], double id[
 // list[0] counts the leaves and they follow from list[1] (each warp's in
 // node order; each leaf's result does not depend on the order).
 __global__ void k_qef_pick(const int8_t* __restrict__ nd_type, long long lb, long long le, int* __restrict__ list) {
+  launch_wait();
   const long long node = lb + (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool leaf = node < le && nd_type[node] == Q_LEAF;
@@ -536,6 +537,7 @@ __global__ void __launch_bounds__(kQefThreads, 8) k_qef(QefArgs a, const int* __
                                                         const float4* __restrict__ nd_c,
                                                         const float* __restrict__ nd_samp,
                                                         unsigned long long* __restrict__ counters) {
+  launch_wait();
   const int count = *count_ptr;
   if (start) list += *start;
   for (int t = blockIdx.x * kQefThreads + threadIdx.x; t < count; t += gridDim.x * kQefThreads) {
@@ -565,6 +567,7 @@ __global__ void __launch_bounds__(128) k_qef_accept(QefArgs a, const int* __rest
                                                     float4* __restrict__ nd_v, const float4* __restrict__ nd_c,
                                                     const float* __restrict__ nd_samp,
                                                     unsigned long long* __restrict__ counters) {
+  launch_wait();
   const int lane = threadIdx.x & 31;
   const int count = *count_ptr;
   if (start) list += *start;

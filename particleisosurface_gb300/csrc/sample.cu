@@ -44,6 +44,7 @@ struct GridRuns {
 __global__ void __launch_bounds__(32 * kGridWarps, 3) k_grid_eval(GridView g, PartView P, float iso, GridRuns R,
                                                                  float* __restrict__ out,
                                                                  unsigned long long* __restrict__ counters) {
+  launch_wait();
   __shared__ __align__(16) float s_stage[kGridWarps][kStageFloats];
   const int lane = threadIdx.x & 31;
   const int wib = threadIdx.x >> 5;

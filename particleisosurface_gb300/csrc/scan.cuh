@@ -104,6 +104,7 @@ __device__ __forceinline__ int block_before(int mine, int* s_warp, int* total) {
 template <class In, int NT, int V, int CL>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT)
     k_scan_one(In in, int* out, long long n, int* d_total) {
+  launch_wait();
   namespace cg = cooperative_groups;
   __shared__ int s_warp[NT / 32];
   __shared__ int s_total;
@@ -136,6 +137,7 @@ constexpr int kScanTile = kTileThreads * 4 * kTileV;
 
 template <class In>
 __global__ void __launch_bounds__(kTileThreads) k_scan_sums(In in, long long n, int* sums) {
+  launch_wait();
   __shared__ int s_warp[kTileThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const long long base = (long long)blockIdx.x * kScanTile;
@@ -160,6 +162,7 @@ __global__ void __launch_bounds__(kTileThreads) k_scan_sums(In in, long long n, 
 template <class In>
 __global__ void __launch_bounds__(kTileThreads) k_scan_tiles(In in, int* out, long long n, const int* sums,
                                                              int scanned, int* d_total) {
+  launch_wait();
   __shared__ int s_warp[kTileThreads / 32];
   __shared__ int s_pre[kTileThreads / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

@@ -36,6 +36,7 @@ void exclusive_scan_i32(const int* in, int* out, long long n, int* d_total, int*
 template <class K>
 __global__ void k_rs_hist(const K* __restrict__ keys, long long n, int shift, int* __restrict__ hist,
                           int nt) {
+  launch_wait();
   __shared__ int h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
@@ -53,6 +54,7 @@ template <class K>
 __global__ void k_rs_scatter(const K* __restrict__ kin, const uint32_t* __restrict__ vin,
                              K* __restrict__ kout, uint32_t* __restrict__ vout, long long n, int shift,
                              const int* __restrict__ offs, int nt) {
+  launch_wait();
   __shared__ int run[256];
   __shared__ int wc[kThreads / 32][256];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -120,6 +122,7 @@ void radix_sort_u64(uint64_t** keys, uint32_t** vals, uint64_t** kalt, uint32_t*
 }
 
 __global__ void k_iota(uint32_t* v, long long n) {
+  launch_wait();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) v[i] = (uint32_t)i;
 }

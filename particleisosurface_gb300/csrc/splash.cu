@@ -21,6 +21,7 @@ namespace pisurf {
 // Flag in particle order (for the scan) and pos.w = 1 for splash particles.
 __global__ void k_splash_mark(const int8_t* __restrict__ spl, const uint32_t* __restrict__ sidx, long long n,
                               float4* __restrict__ pos, int* __restrict__ flag) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const int s = spl[t];
@@ -31,6 +32,7 @@ __global__ void k_splash_mark(const int8_t* __restrict__ spl, const uint32_t* __
 // list[rank of the particle among the splash particles] = its sorted position.
 __global__ void k_splash_list(const int8_t* __restrict__ spl, const uint32_t* __restrict__ sidx, long long n,
                               const int* __restrict__ rank, int* __restrict__ list) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   if (spl[t]) list[rank[sidx[t]]] = (int)t;
@@ -87,6 +89,7 @@ __global__ void k_splash_mesh(IcosaTable T, long long ns, const int* __restrict_
                               const float4* __restrict__ pos, const uint32_t* __restrict__ sidx, float r,
                               long long v0, long long t0, float* __restrict__ mv, uint64_t* __restrict__ mk,
                               int* __restrict__ mt) {
+  launch_wait();
   const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= ns) return;
   const int t = list[k];

@@ -50,6 +50,7 @@ static float vr_fdec(unsigned e) {
 // block in shared memory (at most kMaxBins grids).
 __global__ void k_vr_bin_bbox(const float* __restrict__ xyz, const int* __restrict__ pbin, long long n, int ng,
                               unsigned* __restrict__ bb) {
+  launch_wait();
   __shared__ unsigned s[kMaxBins * 6];
   for (int k = threadIdx.x; k < ng * 6; k += blockDim.x) s[k] = (k & 1) ? 0u : 0xffffffffu;
   __syncthreads();
@@ -75,6 +76,7 @@ __global__ void k_vr_bin_bbox(const float* __restrict__ xyz, const int* __restri
 __global__ void k_vr_keys(const float* __restrict__ xyz, const int* __restrict__ pbin, long long n,
                           const MultiGridView* __restrict__ mg, int kbits, int* __restrict__ key,
                           uint64_t* __restrict__ skey, uint32_t* __restrict__ sidx) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int b = pbin[i];
@@ -98,6 +100,7 @@ __global__ void k_vr_keys(const float* __restrict__ xyz, const int* __restrict__
 __global__ void k_vr_cell_count(const int* __restrict__ key, const int* __restrict__ pbin, long long n,
                                 const MultiGridView* __restrict__ mg, const long long* __restrict__ cellnum,
                                 int* __restrict__ cnt) {
+  launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const int b = pbin[i];
@@ -108,6 +111,7 @@ __global__ void k_vr_cell_count(const int* __restrict__ key, const int* __restri
 __global__ void k_vr_gather_pos(const float* __restrict__ xyz, const float* __restrict__ rad,
                                 const float4* __restrict__ vrc, const uint32_t* __restrict__ sidx, long long n,
                                 float4* __restrict__ pos, float4* __restrict__ vrcs) {
+  launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
   const uint32_t i = sidx[t];
