@@ -614,7 +614,7 @@ __global__ void k_vcell_place(long long nv, const int* __restrict__ key, const i
 }
 
 template <bool VR>
-__global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, const int* __restrict__ order, const int* __restrict__ rep,
+__global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, int per_warp, const int* __restrict__ order, const int* __restrict__ rep,
                          const int* __restrict__ slotA,
                          const int* __restrict__ slotB, const float4* __restrict__ nd_v,
                          const uint64_t* __restrict__ nd_id, float* __restrict__ out,
@@ -622,8 +622,9 @@ __global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, c
                          unsigned long long* __restrict__ counters) {
   launch_wait();
   __shared__ __align__(16) float s_stage[VR ? 1 : kGroupWarps][VR ? 1 : GroupRoom<32>::kFloats];
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = t < nv;
+  const int lane = threadIdx.x & 31;
+  const long long t = ((long long)blockIdx.x * kGroupWarps + (threadIdx.x >> 5)) * per_warp + lane;
+  const bool valid = lane < per_warp && t < nv;
   long long v = 0;
   int A = 0, B = 0;
   float4 p = make_float4(0.f, 0.f, 0.f, 0.f), q = p;
@@ -971,12 +972,17 @@ void stage_extract(pi_frame* f) {
               vcnt.p, vkey.p);
     exclusive_scan_i32(vcnt.p, vcnt.p, nc + 1, nullptr, tmp.p, s);
     PI_LAUNCH(k_vcell_place, div_up(nv, 256), 256, 0, s, nv, vkey.p, vcnt.p, vfill.p, vorder.p);
+    // vertices per warp: all its lanes filter the candidates of the vertices it
+    // holds, so fewer of them shorten a warp's chain; halved while that leaves a
+    // handful of warps per SM (5,000 vertices: 69 us with 32, 46 with 4)
+    int per_warp = 32;
+    while (!f->varR && per_warp > 4 && nv < 8LL * c->smCount * per_warp) per_warp /= 2;
     prof_begin(c, s, PG_BISECT);
     if (f->varR)
-      PI_LAUNCH(k_bisect<true>, div_up(nv, 128), 128, 0, s, ba, nv, vorder.p, rep.p, slotA.p, slotB.p, f->nd_v.p,
+      PI_LAUNCH(k_bisect<true>, div_up(nv, 128), 128, 0, s, ba, nv, per_warp, vorder.p, rep.p, slotA.p, slotB.p, f->nd_v.p,
                 f->nd_id.p, f->mv.p, f->mk.p, f->vedge.p, f->dcount.p);
     else
-      PI_LAUNCH(k_bisect<false>, div_up(nv, 128), 128, 0, s, ba, nv, vorder.p, rep.p, slotA.p, slotB.p, f->nd_v.p,
+      PI_LAUNCH(k_bisect<false>, div_up(nv, per_warp * kGroupWarps), 32 * kGroupWarps, 0, s, ba, nv, per_warp, vorder.p, rep.p, slotA.p, slotB.p, f->nd_v.p,
                 f->nd_id.p, f->mv.p, f->mk.p, f->vedge.p, f->dcount.p);
     prof_end(c, s, PG_BISECT);
   }
