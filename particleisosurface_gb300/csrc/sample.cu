@@ -8,8 +8,14 @@
 //     (steps - i) / steps * min + i / steps * max per axis, x fastest.
 // The lattice points of one hash cell form a contiguous index run along each
 // axis (the cell index is monotonic in the coordinate), so a chunk is a
-// (x-run, y-run, z-run) triple: at most 5 x 5 x 5 points, all with the same
-// 27-cell candidate list, evaluated by one warp (chunk_field, 4 per lane).
+// (x-run, y-run, z-run) triple: at most 4 x 4 x 4 points, all with the same
+// 27-cell candidate list, evaluated by one warp (chunk_field, 2 per lane).  A
+// cell is four spacings wide: rounding can put a fifth point into it, which is
+// then a run of its own.  Bound by the FP32 instructions of the kernel terms.  A
+// warp takes one chunk at a time off a counter: most chunks are empty, and with a
+// fixed stride (and room for 125 points a chunk) the SMs stood idle 15 % of
+// 450 us on 150,000 particles; it is 339 us now, 357 with four chunks at a time,
+// 378 with four and 64 registers a thread (spills).
 #include <cmath>
 #include <vector>
 
@@ -19,7 +25,8 @@
 namespace pisurf {
 
 constexpr int kGridWarps = 8;
-constexpr int kRunMax = 5;  // points per axis run: a cell is 4r, the spacing r
+constexpr int kRunMax = 4;   // points per axis run: a cell is 4r, the spacing r
+constexpr int kGridSlots = 2;  // points per lane: 4^3 points of a chunk
 
 void uniform_grid_host(const pi_frame* f, float box[6], int steps[3], int dims[3]) {
   const float r = f->P.radius;
@@ -50,20 +57,25 @@ __global__ void __launch_bounds__(32 * kGridWarps, 3) k_grid_eval(GridView g, Pa
   const int wib = threadIdx.x >> 5;
   const ChunkStage st{s_stage[wib]};
   const long long nchunks = (long long)R.nrun[0] * R.nrun[1] * R.nrun[2];
-  const long long nwarps = (long long)gridDim.x * kGridWarps;
+  // chunks taken: a word between the pairs' stripes, zeroed with them
+  unsigned long long* const next = counters + (size_t)C_GRID_PAIRS * kStripes * 4 + 1;
   long long pairs = 0;
-  for (long long ci = (long long)blockIdx.x * kGridWarps + wib; ci < nchunks; ci += nwarps) {
+  for (;;) {
+    long long ci = 0;
+    if (lane == 0) ci = (long long)atomicAdd(next, 1ull);
+    ci = __shfl_sync(0xffffffffu, ci, 0);
+    if (ci >= nchunks) break;
     const int rx = (int)(ci % R.nrun[0]), ry = (int)((ci / R.nrun[0]) % R.nrun[1]),
               rz = (int)(ci / ((long long)R.nrun[0] * R.nrun[1]));
     const int x0 = __ldg(R.run[0] + rx), kx = __ldg(R.run[0] + rx + 1) - x0;
     const int y0 = __ldg(R.run[1] + ry), ky = __ldg(R.run[1] + ry + 1) - y0;
     const int z0 = __ldg(R.run[2] + rz), kz = __ldg(R.run[2] + rz + 1) - z0;
     const int npts = kx * ky * kz;
-    float x[4], y[4], z[4];
-    bool act[4], slots[4];
-    long long idx[4];
+    float x[kGridSlots], y[kGridSlots], z[kGridSlots];
+    bool act[kGridSlots], slots[kGridSlots];
+    long long idx[kGridSlots];
 #pragma unroll
-    for (int m = 0; m < 4; ++m) {
+    for (int m = 0; m < kGridSlots; ++m) {
       const int p = lane + 32 * m;
       act[m] = p < npts;
       slots[m] = npts > 32 * m;  // warp-uniform
@@ -80,10 +92,10 @@ __global__ void __launch_bounds__(32 * kGridWarps, 3) k_grid_eval(GridView g, Pa
     int cx, cy, cz;
     cell_of(g, __shfl_sync(0xffffffffu, x[0], 0), __shfl_sync(0xffffffffu, y[0], 0),
             __shfl_sync(0xffffffffu, z[0], 0), cx, cy, cz);
-    float sum[4];
-    chunk_field<4>(g, P, cx, cy, cz, x, y, z, act, slots, st, sum, pairs);
+    float sum[kGridSlots];
+    chunk_field<kGridSlots>(g, P, cx, cy, cz, x, y, z, act, slots, st, sum, pairs);
 #pragma unroll
-    for (int m = 0; m < 4; ++m)
+    for (int m = 0; m < kGridSlots; ++m)
       if (act[m]) out[idx[m]] = iso - sum[m];
   }
 #pragma unroll
