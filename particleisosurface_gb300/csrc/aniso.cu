@@ -63,37 +63,53 @@ __device__ __forceinline__ float d2_exact(const Offset& d) {
   return d2_exact(d, sq);
 }
 
-// Two Kahan sums.
-struct Kahan2 {
-  float2 s = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
-  __device__ __forceinline__ void add(const float2& v) {
-    const float2 m1 = make_float2(-1.0f, -1.0f);
-    const float2 y = __ffma2_rn(c, m1, v);
-    const float2 t = __fadd2_rn(s, y);
-    c = __ffma2_rn(y, m1, __ffma2_rn(s, m1, t));
-    s = t;
-  }
-};
-
-// The weighted sums of k_xmean: offsets and weights.
+// The weighted sums of k_xmean: offsets and weights.  With four lanes to a
+// particle each lane holds a pair of them: the even lanes x and y.
+template <int L>
 struct MeanSums {
   Kahan2 xy, zw;
-  __device__ __forceinline__ void add(const Offset& d, float w) {
-    xy.add(__fmul2_rn(d.xy, make_float2(w, w)));
-    zw.add(make_float2(__fmul_rn(d.z, w), w));
+  __device__ __forceinline__ void add(const Offset& d, float w, int sub) {
+    const float2 ww = make_float2(w, w);
+    if (L == 1) {
+      xy.add(__fmul2_rn(d.xy, ww));
+      zw.add(make_float2(__fmul_rn(d.z, w), w));
+    } else {
+      xy.add(__fmul2_rn(sub & 1 ? make_float2(d.z, 1.0f) : d.xy, ww));
+    }
+  }
+  __device__ __forceinline__ void gather() {  // all sums to the lanes that need them
+    if (L == 1) return;
+    zw.s.x = __shfl_down_sync(0xffffffffu, xy.s.x, 1, 4), zw.s.y = __shfl_down_sync(0xffffffffu, xy.s.y, 1, 4);
+    zw.c.x = __shfl_down_sync(0xffffffffu, xy.c.x, 1, 4), zw.c.y = __shfl_down_sync(0xffffffffu, xy.c.y, 1, 4);
   }
 };
 
-// Those of k_cov_G: products of the offset's components, and weights.
+// Those of k_cov_G: products of the offset's components, and weights.  With four
+// lanes to a particle lane k holds the k-th of them in c00_11.
+template <int L>
 struct CovSums {
   Kahan2 c00_11, c02_12, c01_22;
   Kahan ws;
-  __device__ __forceinline__ void add(const Offset& d, const float2& sq, float w) {
+  __device__ __forceinline__ void add(const Offset& d, const float2& sq, float w, int sub) {
     const float2 ww = make_float2(w, w);
-    c00_11.add(__fmul2_rn(sq, ww));
-    c02_12.add(__fmul2_rn(__fmul2_rn(d.xy, make_float2(d.z, d.z)), ww));
-    c01_22.add(__fmul2_rn(make_float2(__fmul_rn(d.xy.x, d.xy.y), __fmul_rn(d.z, d.z)), ww));
-    ws.add(w);
+    const float2 p02_12 = __fmul2_rn(d.xy, make_float2(d.z, d.z));
+    const float2 p01_22 = make_float2(__fmul_rn(d.xy.x, d.xy.y), __fmul_rn(d.z, d.z));
+    if (L == 1) {
+      c00_11.add(__fmul2_rn(sq, ww));
+      c02_12.add(__fmul2_rn(p02_12, ww));
+      c01_22.add(__fmul2_rn(p01_22, ww));
+      ws.add(w);
+    } else {
+      const float2 one = make_float2(1.0f, 1.0f);
+      c00_11.add(__fmul2_rn(sub & 2 ? (sub & 1 ? one : p01_22) : (sub & 1 ? p02_12 : sq), ww));
+    }
+  }
+  __device__ __forceinline__ void gather() {
+    if (L == 1) return;
+    const float2 v = c00_11.s;
+    c02_12.s.x = __shfl_down_sync(0xffffffffu, v.x, 1, 4), c02_12.s.y = __shfl_down_sync(0xffffffffu, v.y, 1, 4);
+    c01_22.s.x = __shfl_down_sync(0xffffffffu, v.x, 2, 4), c01_22.s.y = __shfl_down_sync(0xffffffffu, v.y, 2, 4);
+    ws.s = __shfl_down_sync(0xffffffffu, v.x, 3, 4);
   }
 };
 
@@ -106,40 +122,38 @@ struct CovSums {
 // Splash particles (spl not null): a particle with <= 2 candidates or <= 2
 // neighbours within 4r (the GlobalSplash marking of src/evaluator.cpp:675,690
 // switched on) gets spl = 1.
+template <int L>
 __global__ void k_xmean(GridView g, const float4* __restrict__ pos, long long n, float nI, float nI2,
                         float inv_h3, float c_mean, float4* __restrict__ xm, float4* __restrict__ xlo,
                         int8_t* __restrict__ spl) {
   launch_wait();
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  float4 p = pos[t];
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x & (L - 1);
+  const bool valid = t < n;
+  if (L == 1 && !valid) return;
+  const float4 p = valid ? pos[t] : make_float4(0.f, 0.f, 0.f, 0.f);
   int cx, cy, cz;
   cell_of(g, p.x, p.y, p.z, cx, cy, cz);
   long long cand = 0;
   int nn = 0;  // neighbours within 4r (compute_xMeans' neighbors.size())
-  MeanSums sum;
+  MeanSums<L> sum;
   for (int dz = -1; dz <= 1; ++dz)
     for (int dy = -1; dy <= 1; ++dy) {
-      int s, e;
-      if (!nb_row(g, cx, cy + dy, cz + dz, &s, &e)) continue;
-      cand += e - s;
-      // 32 candidates at a time: the distance test into a bit mask, then
-      // the weights of the set bits in candidate order
-      for (int j0 = s; j0 < e; j0 += 32) {
-        const int cnt = min(32, e - j0);
-        unsigned m = 0u;
-        for (int k = 0; k < cnt; ++k) {
-          m |= (d2_exact(offset_from(p, __ldg(pos + j0 + k))) < nI2 && j0 + k != t ? 1u : 0u) << k;
-        }
-        nn += __popc(m);
-        while (m) {
-          const int j = j0 + __ffs(m) - 1;
-          m &= m - 1u;
-          const Offset d = offset_from(p, __ldg(pos + j));
-          sum.add(d, wij_f(__fsqrt_rn(d2_exact(d)), nI, inv_h3));
-        }
+      int s = 0, e = 0;
+      if (!valid || !nb_row(g, cx, cy + dy, cz + dz, &s, &e)) {
+        if (L == 1) continue;
+        s = e = 0;
       }
+      cand += e - s;
+      nn += walk_row<L>(
+          s, e, sub, [&](int j0, int k) { return d2_exact(offset_from(p, __ldg(pos + j0 + k))) < nI2 && j0 + k != t; },
+          [&](int j) {
+            const Offset d = offset_from(p, __ldg(pos + j));
+            sum.add(d, wij_f(__fsqrt_rn(d2_exact(d)), nI, inv_h3), sub);
+          });
     }
+  sum.gather();
+  if (L > 1 && (sub != 0 || !valid)) return;
   float4 hi = make_float4(p.x, p.y, p.z, 0.f), lo = make_float4(0.f, 0.f, 0.f, 0.f);
   const float wsum = sum.zw.s.y;
   if (cand > 2 && wsum > 0.f) {
@@ -219,6 +233,7 @@ __device__ __forceinline__ void g_from_eig(const T w_in[3], const T V[3][3], flo
   *stretch = (float)(wmax / scale);
 }
 
+template <int L>
 __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __restrict__ pos, const float4* __restrict__ xm0,
                         const float4* __restrict__ xlo, float4* __restrict__ xm, long long n,
                         float nI, float nI2, float inv_h3, float h2, float inv_h, float sigma,
@@ -226,12 +241,14 @@ __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __re
                         float* __restrict__ det_out, int8_t* __restrict__ f64flag,
                         unsigned long long* __restrict__ f64count, const int8_t* __restrict__ spl) {
   launch_wait();
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  float4 p = pos[t];
-  float4 xp = xm0[t];
-  const float4 lp = xlo[t];
-  if (spl && spl[t]) {
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x & (L - 1);
+  const bool valid = t < n;
+  if (L == 1 && !valid) return;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 p = valid ? pos[t] : zero, xp = valid ? xm0[t] : zero, lp = valid ? xlo[t] : zero;
+  const bool lone = valid && spl && spl[t];
+  if (lone && sub == 0) {
     // a splash particle keeps pass 1's identity G (pass 2 skips it,
     // src/evaluator.cpp:723-726) and takes part in no field sum: its cull
     // radius is negative, so no support test passes
@@ -241,33 +258,31 @@ __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __re
     for (int k = 0; k < 9; ++k) gfull[9 * t + k] = (k % 4 == 0) ? 1.0f : 0.0f;
     det_out[t] = 1.0f;
     f64flag[t] = 0;
-    return;
   }
+  if (L == 1 && lone) return;
   int cx, cy, cz;
   cell_of(g, p.x, p.y, p.z, cx, cy, cz);
-  CovSums sum;
+  CovSums<L> sum;
   for (int dz = -1; dz <= 1; ++dz)
     for (int dy = -1; dy <= 1; ++dy) {
-      int s, e;
-      if (!nb_row(g, cx, cy + dy, cz + dz, &s, &e)) continue;
-      // 32 candidates at a time: the distance test into a bit mask, then
-      // the weighted products of the set bits in candidate order
-      for (int j0 = s; j0 < e; j0 += 32) {
-        const int cnt = min(32, e - j0);
-        unsigned m = 0u;
-        for (int k = 0; k < cnt; ++k) {
-          m |= (d2_exact(offset_from(xp, lp, __ldg(xm0 + j0 + k), __ldg(xlo + j0 + k))) < nI2 ? 1u : 0u) << k;
-        }
-        while (m) {
-          const int j = j0 + __ffs(m) - 1;
-          m &= m - 1u;
-          const Offset d = offset_from(xp, lp, __ldg(xm0 + j), __ldg(xlo + j));
-          float2 sq;
-          const float d2 = d2_exact(d, sq);
-          sum.add(d, sq, wij_f(__fsqrt_rn(d2), nI, inv_h3));
-        }
+      int s = 0, e = 0;
+      if (!valid || lone || !nb_row(g, cx, cy + dy, cz + dz, &s, &e)) {
+        if (L == 1) continue;
+        s = e = 0;
       }
+      walk_row<L>(
+          s, e, sub, [&](int j0, int k) {
+            return d2_exact(offset_from(xp, lp, __ldg(xm0 + j0 + k), __ldg(xlo + j0 + k))) < nI2;
+          },
+          [&](int j) {
+            const Offset d = offset_from(xp, lp, __ldg(xm0 + j), __ldg(xlo + j));
+            float2 sq;
+            const float d2 = d2_exact(d, sq);
+            sum.add(d, sq, wij_f(__fsqrt_rn(d2), nI, inv_h3), sub);
+          });
     }
+  sum.gather();
+  if (L > 1 && (sub != 0 || !valid || lone)) return;
   float iw = 1.0f / sum.ws.s;
   float a6[6] = {(h2 + sum.c00_11.s.x) * iw, sum.c01_22.s.x * iw,         sum.c02_12.s.x * iw,
                  (h2 + sum.c00_11.s.y) * iw, sum.c02_12.s.y * iw, (h2 + sum.c01_22.s.y) * iw};
@@ -315,44 +330,48 @@ __global__ void __launch_bounds__(128, 8) k_cov_G(GridView g, const float4* __re
 // det * Sigma_i per particle.  The radius rides in pos.w.  Candidates are the
 // bins' 27-cell lists in bin order.
 // ---------------------------------------------------------------------------
+template <int L>
 __global__ void __launch_bounds__(128) k_vr_xmean(const MultiGridView* __restrict__ mg,
                                                   const float4* __restrict__ pos, const float4* __restrict__ vrc,
                                                   long long n, float c_mean, float4* __restrict__ xm,
                                                   float4* __restrict__ xlo) {
   launch_wait();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x & (L - 1);
+  const bool valid = t < n;
+  if (L == 1 && !valid) return;
   const MultiGridView& m = *mg;
-  const float4 p = pos[t];
+  const float4 p = valid ? pos[t] : make_float4(0.f, 0.f, 0.f, 0.f);
   long long cand = 0;
-  MeanSums sum;
+  MeanSums<L> sum;
   for (int b = 0; b < m.nb; ++b) {
     const BinGrid g = m.g[b];
     const int cx = cell_coord(p.x, g.b0, g.cell, g.nx), cy = cell_coord(p.y, g.b2, g.cell, g.ny),
               cz = cell_coord(p.z, g.b4, g.cell, g.nz);
     for (int dz = -1; dz <= 1; ++dz)
       for (int dy = -1; dy <= 1; ++dy) {
-        int s, e;
-        if (!bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) continue;
-        cand += e - s;
-        // 32 candidates at a time, as k_xmean
-        for (int j0 = s; j0 < e; j0 += 32) {
-          const int cnt = min(32, e - j0);
-          unsigned hits = 0u;
-          for (int k = 0; k < cnt; ++k) {
-            const float nI = __ldg(&vrc[j0 + k].z);  // (Influnce2, Sigma, nI, 1 / nI^3) of the neighbour
-            hits |= (d2_exact(offset_from(p, __ldg(pos + j0 + k))) < __fmul_rn(nI, nI) && j0 + k != t ? 1u : 0u) << k;
-          }
-          while (hits) {
-            const int j = j0 + __ffs(hits) - 1;
-            hits &= hits - 1u;
-            const float4 cj = __ldg(vrc + j);
-            const Offset d = offset_from(p, __ldg(pos + j));
-            sum.add(d, wij_f(__fsqrt_rn(d2_exact(d)), cj.z, cj.w));
-          }
+        int s = 0, e = 0;
+        if (!valid || !bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) {
+          if (L == 1) continue;
+          s = e = 0;
         }
+        cand += e - s;
+        // vrc: (Influnce2, Sigma, nI, 1 / nI^3) of the neighbour
+        walk_row<L>(
+            s, e, sub,
+            [&](int j0, int k) {
+              const float nI = __ldg(&vrc[j0 + k].z);
+              return d2_exact(offset_from(p, __ldg(pos + j0 + k))) < __fmul_rn(nI, nI) && j0 + k != t;
+            },
+            [&](int j) {
+              const float4 cj = __ldg(vrc + j);
+              const Offset d = offset_from(p, __ldg(pos + j));
+              sum.add(d, wij_f(__fsqrt_rn(d2_exact(d)), cj.z, cj.w), sub);
+            });
       }
   }
+  sum.gather();
+  if (L > 1 && (sub != 0 || !valid)) return;
   float4 hi = make_float4(p.x, p.y, p.z, 0.f), lo = make_float4(0.f, 0.f, 0.f, 0.f);
   const float wsum = sum.zw.s.y;
   if (cand > 2 && wsum > 0.f) {
@@ -369,6 +388,7 @@ __global__ void __launch_bounds__(128) k_vr_xmean(const MultiGridView* __restric
   xlo[t] = lo;
 }
 
+template <int L>
 __global__ void __launch_bounds__(128) k_vr_cov_G(const MultiGridView* __restrict__ mg,
                                                   const float4* __restrict__ pos, const float4* __restrict__ vrc,
                                                   const float4* __restrict__ xm0,
@@ -377,46 +397,47 @@ __global__ void __launch_bounds__(128) k_vr_cov_G(const MultiGridView* __restric
                                                   float* __restrict__ gfull, float* __restrict__ det_out,
                                                   int8_t* __restrict__ f64flag, unsigned long long* __restrict__ f64count) {
   launch_wait();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x & (L - 1);
+  const bool valid = t < n;
+  if (L == 1 && !valid) return;
   const MultiGridView& m = *mg;
-  const float4 p = pos[t];
-  const float4 xp = xm0[t];
-  const float4 lp = xlo[t];
-  const float4 ci = vrc[t];
-  const float h = p.w * 2.0f;  // 2 r_i
-  const float h2 = ci.x;       // Influnce2_i
-  const float sigma = ci.y;    // Sigma_i
-  const float inv_h = 1.0f / h;
-  CovSums sum;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 p = valid ? pos[t] : zero, xp = valid ? xm0[t] : zero, lp = valid ? xlo[t] : zero;
+  CovSums<L> sum;
   for (int b = 0; b < m.nb; ++b) {
     const BinGrid g = m.g[b];
     const int cx = cell_coord(p.x, g.b0, g.cell, g.nx), cy = cell_coord(p.y, g.b2, g.cell, g.ny),
               cz = cell_coord(p.z, g.b4, g.cell, g.nz);
     for (int dz = -1; dz <= 1; ++dz)
       for (int dy = -1; dy <= 1; ++dy) {
-        int s, e;
-        if (!bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) continue;
-        for (int j0 = s; j0 < e; j0 += 32) {
-          const int cnt = min(32, e - j0);
-          unsigned hits = 0u;
-          for (int k = 0; k < cnt; ++k) {
-            const float nI = __ldg(&vrc[j0 + k].z);
-            const float d2 = d2_exact(offset_from(xp, lp, __ldg(xm0 + j0 + k), __ldg(xlo + j0 + k)));
-            hits |= (d2 < __fmul_rn(nI, nI) ? 1u : 0u) << k;
-          }
-          while (hits) {
-            const int j = j0 + __ffs(hits) - 1;
-            hits &= hits - 1u;
-            const float4 cj = __ldg(vrc + j);
-            const Offset d = offset_from(xp, lp, __ldg(xm0 + j), __ldg(xlo + j));
-            float2 sq;
-            const float d2 = d2_exact(d, sq);
-            sum.add(d, sq, wij_f(__fsqrt_rn(d2), cj.z, cj.w));
-          }
+        int s = 0, e = 0;
+        if (!valid || !bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) {
+          if (L == 1) continue;
+          s = e = 0;
         }
+        walk_row<L>(
+            s, e, sub,
+            [&](int j0, int k) {
+              const float nI = __ldg(&vrc[j0 + k].z);
+              return d2_exact(offset_from(xp, lp, __ldg(xm0 + j0 + k), __ldg(xlo + j0 + k))) < __fmul_rn(nI, nI);
+            },
+            [&](int j) {
+              const float4 cj = __ldg(vrc + j);
+              const Offset d = offset_from(xp, lp, __ldg(xm0 + j), __ldg(xlo + j));
+              float2 sq;
+              const float d2 = d2_exact(d, sq);
+              sum.add(d, sq, wij_f(__fsqrt_rn(d2), cj.z, cj.w), sub);
+            });
       }
   }
+  sum.gather();
+  if (L > 1 && (sub != 0 || !valid)) return;
+  const float4 ci = vrc[t];
+  const float h = p.w * 2.0f;  // 2 r_i
+  const float h2 = ci.x;       // Influnce2_i
+  const float sigma = ci.y;    // Sigma_i
+  const float inv_h = 1.0f / h;
   const float iw = 1.0f / sum.ws.s;
   float a6[6] = {(h2 + sum.c00_11.s.x) * iw, sum.c01_22.s.x * iw,         sum.c02_12.s.x * iw,
                  (h2 + sum.c00_11.s.y) * iw, sum.c02_12.s.y * iw, (h2 + sum.c01_22.s.y) * iw};
@@ -467,9 +488,12 @@ void stage_aniso_vr(pi_frame* f) {
   f->f64flag.alloc(f->ctx, s, n);
   counters_reset(f, 0, kCounters - 1);  // every stage's
   f->octree_counted = f->extract_counted = false;
-  PI_LAUNCH(k_vr_xmean, div_up(n, 128), 128, 0, s, f->mgv.p, f->pos.p, f->vrcs.p, n, (float)0.9, f->nrm.p,
+  const int lanes = particle_lanes(f);
+  const auto xmean = lanes == 4 ? k_vr_xmean<4> : k_vr_xmean<1>;
+  PI_LAUNCH(xmean, div_up(n * lanes, 128), 128, 0, s, f->mgv.p, f->pos.p, f->vrcs.p, n, (float)0.9, f->nrm.p,
             f->xlo.p);
-  PI_LAUNCH(k_vr_cov_G, div_up(n, 128), 128, 0, s, f->mgv.p, f->pos.p, f->vrcs.p, f->nrm.p, f->xlo.p, f->xm.p, n,
+  const auto cov = lanes == 4 ? k_vr_cov_G<4> : k_vr_cov_G<1>;
+  PI_LAUNCH(cov, div_up(n * lanes, 128), 128, 0, s, f->mgv.p, f->pos.p, f->vrcs.p, f->nrm.p, f->xlo.p, f->xm.p, n,
             f->ga.p, f->gb.p, f->gfull.p, f->det.p, f->f64flag.p, f->dcount.p);
   counters_snapshot(f, kPinAniso);
 }
@@ -501,9 +525,12 @@ void stage_aniso(pi_frame* f) {
   if (splash) f->spl.alloc(f->ctx, s, n);
   counters_reset(f, 0, kCounters - 1);  // every stage's
   f->octree_counted = f->extract_counted = false;
-  PI_LAUNCH(k_xmean, div_up(n, 128), 128, 0, s, g, f->pos.p, n, nI, nI2, inv_h3, c_mean, f->nrm.p, f->xlo.p,
+  const int lanes = particle_lanes(f);
+  const auto xmean = lanes == 4 ? k_xmean<4> : k_xmean<1>;
+  PI_LAUNCH(xmean, div_up(n * lanes, 128), 128, 0, s, g, f->pos.p, n, nI, nI2, inv_h3, c_mean, f->nrm.p, f->xlo.p,
             splash ? f->spl.p : nullptr);
-  PI_LAUNCH(k_cov_G, div_up(n, 128), 128, 0, s, g, f->pos.p, f->nrm.p, f->xlo.p, f->xm.p, n, nI, nI2, inv_h3, f->influ2,
+  const auto cov = lanes == 4 ? k_cov_G<4> : k_cov_G<1>;
+  PI_LAUNCH(cov, div_up(n * lanes, 128), 128, 0, s, g, f->pos.p, f->nrm.p, f->xlo.p, f->xm.p, n, nI, nI2, inv_h3, f->influ2,
             1.0f / h, f->sigma, f->ga.p, f->gb.p, f->gfull.p, f->det.p, f->f64flag.p, f->dcount.p,
             splash ? f->spl.p : nullptr);
   if (splash) stage_splash_list(f);

@@ -95,6 +95,58 @@ __device__ __forceinline__ bool nb_row(const GridView& g, int cx, int y, int z, 
   return *s < *e;
 }
 
+// The candidates [s, e) of a particle whose work L lanes share (L = 1, or the
+// aligned groups of 4 lanes, lane sub of which calls): 32 at a time, the cheap
+// test of each into a bit mask (the lanes test every L-th and join their masks),
+// then hit() for the set bits in candidate order, in every lane.  With L > 1 all
+// lanes of the warp call it (s = e for one without candidates).  Returns the hits.
+template <int L, class Test, class Hit>
+__device__ __forceinline__ int walk_row(int s, int e, int sub, const Test& test, const Hit& hit) {
+  static_assert(L == 1 || L == 4, "lanes per particle");
+  int hits = 0;
+  if (L == 1) {
+    for (int j0 = s; j0 < e; j0 += 32) {
+      const int cnt = min(32, e - j0);
+      unsigned m = 0u;
+      for (int k = 0; k < cnt; ++k) m |= (test(j0, k) ? 1u : 0u) << k;
+      hits += __popc(m);
+      while (m) {
+        const int j = j0 + __ffs(m) - 1;
+        m &= m - 1u;
+        hit(j);
+      }
+    }
+    return hits;
+  }
+  const int end = s + __reduce_max_sync(0xffffffffu, e - s);
+  for (int j0 = s; j0 < end; j0 += 32) {
+    const int cnt = min(32, e - j0);
+    unsigned m = 0u;
+    for (int k = sub; k < cnt; k += L) m |= (test(j0, k) ? 1u : 0u) << k;
+    m |= __shfl_xor_sync(0xffffffffu, m, 1);
+    m |= __shfl_xor_sync(0xffffffffu, m, 2);
+    hits += __popc(m);
+    while (m) {
+      const int j = j0 + __ffs(m) - 1;
+      m &= m - 1u;
+      hit(j);
+    }
+  }
+  return hits;
+}
+
+// Two Kahan sums.
+struct Kahan2 {
+  float2 s = make_float2(0.f, 0.f), c = make_float2(0.f, 0.f);
+  __device__ __forceinline__ void add(const float2& v) {
+    const float2 m1 = make_float2(-1.0f, -1.0f);
+    const float2 y = __ffma2_rn(c, m1, v);
+    const float2 t = __fadd2_rn(s, y);
+    c = __ffma2_rn(y, m1, __ffma2_rn(s, m1, t));
+    s = t;
+  }
+};
+
 // Cubic B-spline of ratio q = sqrt(s2) in [0, 2) without the Sigma factor
 // (Bspline_kernel, src/evaluator.cpp:383-396).
 __device__ __forceinline__ float bspline_s2(float s2) {

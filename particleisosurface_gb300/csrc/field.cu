@@ -12,68 +12,85 @@
 
 namespace pisurf {
 
-// Gradient-form sum at q (without the -6 h^5 factor): sum_j wdet_j u (1 - s2)^2
-// with u = A_j (q - xmean_j), s2 = |u|^2 < 1.
-__device__ __forceinline__ void grad_sum(const GridView& g, const PartView& P, float qx, float qy, float qz,
-                                         float& gx, float& gy, float& gz) {
-  int cx, cy, cz;
-  cell_of(g, qx, qy, qz, cx, cy, cz);
-  Kahan ax, ay, az;
-  for (int dz = -1; dz <= 1; ++dz)
-    for (int dy = -1; dy <= 1; ++dy) {
-      int s, e;
-      if (!nb_row(g, cx, cy + dy, cz + dz, &s, &e)) continue;
-      // 32 candidates at a time: the |d| < R / 2 test (|A d| < 1 needs it)
-      // into a bit mask, then the terms of the set bits in candidate order
-      for (int j0 = s; j0 < e; j0 += 32) {
-        const int cnt = min(32, e - j0);
-        unsigned m = 0u;
-        for (int k = 0; k < cnt; ++k) {
-          const float4 x = __ldg(P.xm + j0 + k);
-          const float dx = qx - x.x, dyy = qy - x.y, dzz = qz - x.z;
-          const float e2 = fmaf(dx, dx, fmaf(dyy, dyy, dzz * dzz));
-          m |= (e2 < 0.25f * x.w ? 1u : 0u) << k;
-        }
-        while (m) {
-          const int j = j0 + __ffs(m) - 1;
-          m &= m - 1u;
-          const float4 x = __ldg(P.xm + j);
-          const float dx = qx - x.x, dyy = qy - x.y, dzz = qz - x.z;
-          const float4 a = __ldg(P.ga + j);
-          const float4 b = __ldg(P.gb + j);
-          const float4 lo = __ldg(P.xlo + j);
-          float u0, u1, u2;
-          amul(a, b, dx - lo.x, dyy - lo.y, dzz - lo.z, u0, u1, u2);
-          const float s2 = fmaf(u0, u0, fmaf(u1, u1, u2 * u2));
-          if (s2 < 1.0f) {
-            const float om = 1.0f - s2;
-            const float f = b.z * om * om;
-            ax.add(u0 * f);
-            ay.add(u1 * f);
-            az.add(u2 * f);
-          }
-        }
+// Gradient-form sums at a point; with four lanes to a point (walk_row) the even
+// lanes hold x and y, the odd ones z.
+template <int L>
+struct GradSums {
+  Kahan2 xy;
+  Kahan x, y, z;
+  // the term of candidate j at q, in all lanes
+  template <bool SCALED>
+  __device__ __forceinline__ void add(const PartView& P, int j, float qx, float qy, float qz, int sub) {
+    const float4 c = __ldg(P.xm + j);
+    const float dx = qx - c.x, dyy = qy - c.y, dzz = qz - c.z;
+    const float4 a = __ldg(P.ga + j);
+    const float4 b = __ldg(P.gb + j);
+    const float4 lo = __ldg(P.xlo + j);
+    float u0, u1, u2;
+    amul(a, b, dx - lo.x, dyy - lo.y, dzz - lo.z, u0, u1, u2);
+    const float s2 = fmaf(u0, u0, fmaf(u1, u1, u2 * u2));
+    if (s2 < 1.0f) {
+      const float om = 1.0f - s2;
+      float f = b.z * om * om;
+      if (SCALED) f *= b.w;
+      if (L == 1) {
+        x.add(u0 * f);
+        y.add(u1 * f);
+        z.add(u2 * f);
+      } else {
+        xy.add(__fmul2_rn(sub & 1 ? make_float2(u2, u2) : make_float2(u0, u1), make_float2(f, f)));
       }
     }
-  gx = ax.s;
-  gy = ay.s;
-  gz = az.s;
+  }
+  __device__ __forceinline__ void gather() {
+    if (L == 1) return;
+    x.s = xy.s.x, y.s = xy.s.y;
+    z.s = __shfl_down_sync(0xffffffffu, xy.s.x, 1, 4);
+  }
+};
+
+// |d| < R / 2: |A d| < 1 needs it.
+__device__ __forceinline__ bool grad_reach(const float4* xm, float qx, float qy, float qz) {
+  const float4 x = __ldg(xm);
+  const float dx = qx - x.x, dyy = qy - x.y, dzz = qz - x.z;
+  return fmaf(dx, dx, fmaf(dyy, dyy, dzz * dzz)) < 0.25f * x.w;
 }
 
+// Gradient-form sum at q (without the -6 h^5 factor): sum_j wdet_j u (1 - s2)^2
+// with u = A_j (q - xmean_j), s2 = |u|^2 < 1.
+template <int L>
+__device__ __forceinline__ void grad_sum(const GridView& g, const PartView& P, float qx, float qy, float qz,
+                                         bool valid, int sub, GradSums<L>& sum) {
+  int cx, cy, cz;
+  cell_of(g, qx, qy, qz, cx, cy, cz);
+  for (int dz = -1; dz <= 1; ++dz)
+    for (int dy = -1; dy <= 1; ++dy) {
+      int s = 0, e = 0;
+      if (!valid || !nb_row(g, cx, cy + dy, cz + dz, &s, &e)) {
+        if (L == 1) continue;
+        s = e = 0;
+      }
+      walk_row<L>(
+          s, e, sub, [&](int j0, int k) { return grad_reach(P.xm + j0 + k, qx, qy, qz); },
+          [&](int j) { sum.template add<false>(P, j, qx, qy, qz, sub); });
+    }
+  sum.gather();
+}
+
+template <int L>
 __global__ void __launch_bounds__(128, 12) k_normals(GridView g, PartView P, long long n, float gscale, float4* __restrict__ nrm) {
   launch_wait();
-  long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  float4 p = P.pos[t];
-  if (p.w != 0.f) {  // a splash particle's normal stays zero
-    nrm[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-    return;
-  }
-  float gx, gy, gz;
-  grad_sum(g, P, p.x, p.y, p.z, gx, gy, gz);
-  gx *= gscale;
-  gy *= gscale;
-  gz *= gscale;
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x & (L - 1);
+  if (L == 1 && t >= n) return;
+  const float4 p = t < n ? P.pos[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool splash = p.w != 0.f;  // a splash particle's normal stays zero
+  if (t < n && splash && sub == 0) nrm[t] = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (L == 1 && splash) return;
+  GradSums<L> sum;
+  grad_sum<L>(g, P, p.x, p.y, p.z, t < n && !splash, sub, sum);
+  if (L > 1 && (sub != 0 || t >= n || splash)) return;
+  const float gx = sum.x.s * gscale, gy = sum.y.s * gscale, gz = sum.z.s * gscale;
   nrm[t] = make_float4(gx, gy, gz, sqrtf(gx * gx + gy * gy + gz * gz));
 }
 
@@ -187,50 +204,40 @@ static float grad_scale(pi_frame* f) {
 // ---- variable radius: the bins' candidate lists, per-particle scales ----
 
 // Gradient-form sum with each term scaled by its particle's -6 h_j^5 (gb.w).
+template <int L>
 __device__ __forceinline__ void grad_sum_vr(const MultiGridView& m, const PartView& P, float qx, float qy, float qz,
-                                            float& gx, float& gy, float& gz) {
-  Kahan ax, ay, az;
+                                            bool valid, int sub, GradSums<L>& sum) {
   for (int b = 0; b < m.nb; ++b) {
     const BinGrid g = m.g[b];
     const int cx = cell_coord(qx, g.b0, g.cell, g.nx), cy = cell_coord(qy, g.b2, g.cell, g.ny),
               cz = cell_coord(qz, g.b4, g.cell, g.nz);
     for (int dz = -1; dz <= 1; ++dz)
       for (int dy = -1; dy <= 1; ++dy) {
-        int s, e;
-        if (!bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) continue;
-        for (int j = s; j < e; ++j) {
-          const float4 x = __ldg(P.xm + j);
-          const float dx = qx - x.x, dyy = qy - x.y, dzz = qz - x.z;
-          if (!(fmaf(dx, dx, fmaf(dyy, dyy, dzz * dzz)) < 0.25f * x.w)) continue;
-          const float4 a = __ldg(P.ga + j);
-          const float4 bb = __ldg(P.gb + j);
-          const float4 lo = __ldg(P.xlo + j);
-          float u0, u1, u2;
-          amul(a, bb, dx - lo.x, dyy - lo.y, dzz - lo.z, u0, u1, u2);
-          const float s2 = fmaf(u0, u0, fmaf(u1, u1, u2 * u2));
-          if (s2 < 1.0f) {
-            const float om = 1.0f - s2;
-            const float fct = bb.z * om * om * bb.w;
-            ax.add(u0 * fct);
-            ay.add(u1 * fct);
-            az.add(u2 * fct);
-          }
+        int s = 0, e = 0;
+        if (!valid || !bin_row(g, m.off, cx, cy + dy, cz + dz, &s, &e)) {
+          if (L == 1) continue;
+          s = e = 0;
         }
+        walk_row<L>(
+            s, e, sub, [&](int j0, int k) { return grad_reach(P.xm + j0 + k, qx, qy, qz); },
+            [&](int j) { sum.template add<true>(P, j, qx, qy, qz, sub); });
       }
   }
-  gx = ax.s;
-  gy = ay.s;
-  gz = az.s;
+  sum.gather();
 }
 
+template <int L>
 __global__ void __launch_bounds__(128) k_vr_normals(const MultiGridView* __restrict__ mg, PartView P, long long n,
                                                     float4* __restrict__ nrm) {
   launch_wait();
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const float4 p = P.pos[t];
-  float gx, gy, gz;
-  grad_sum_vr(*mg, P, p.x, p.y, p.z, gx, gy, gz);
+  const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / L;
+  const int sub = threadIdx.x & (L - 1);
+  if (L == 1 && t >= n) return;
+  const float4 p = t < n ? P.pos[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+  GradSums<L> sum;
+  grad_sum_vr<L>(*mg, P, p.x, p.y, p.z, t < n, sub, sum);
+  if (L > 1 && (sub != 0 || t >= n)) return;
+  const float gx = sum.x.s, gy = sum.y.s, gz = sum.z.s;
   nrm[t] = make_float4(gx, gy, gz, sqrtf(gx * gx + gy * gy + gz * gz));
 }
 
@@ -241,7 +248,13 @@ __global__ void k_vr_eval_points(const MultiGridView* __restrict__ mg, PartView 
   if (i >= m) return;
   const float qx = pts[3 * i], qy = pts[3 * i + 1], qz = pts[3 * i + 2];
   val[i] = iso - field_sum_vr(*mg, P, qx, qy, qz, nullptr);
-  if (grad) grad_sum_vr(*mg, P, qx, qy, qz, grad[3 * i], grad[3 * i + 1], grad[3 * i + 2]);
+  if (grad) {
+    GradSums<1> sum;
+    grad_sum_vr<1>(*mg, P, qx, qy, qz, true, 0, sum);
+    grad[3 * i] = sum.x.s;
+    grad[3 * i + 1] = sum.y.s;
+    grad[3 * i + 2] = sum.z.s;
+  }
 }
 
 __global__ void k_vr_nb_count(const MultiGridView* __restrict__ mg, const float* __restrict__ pts, long long m,
@@ -286,11 +299,14 @@ __global__ void k_vr_nb_fill(const MultiGridView* __restrict__ mg, const float* 
 
 void stage_normals(pi_frame* f) {
   cudaStream_t s = f->ctx->stream;
+  const int lanes = particle_lanes(f);
   if (f->varR) {
-    PI_LAUNCH(k_vr_normals, div_up(f->N, 128), 128, 0, s, f->mgv.p, pview(f), f->N, f->nrm.p);
+    const auto normals = lanes == 4 ? k_vr_normals<4> : k_vr_normals<1>;
+    PI_LAUNCH(normals, div_up(f->N * lanes, 128), 128, 0, s, f->mgv.p, pview(f), f->N, f->nrm.p);
     return;
   }
-  PI_LAUNCH(k_normals, div_up(f->N, 128), 128, 0, s, gview(f), pview(f), f->N, grad_scale(f), f->nrm.p);
+  const auto normals = lanes == 4 ? k_normals<4> : k_normals<1>;
+  PI_LAUNCH(normals, div_up(f->N * lanes, 128), 128, 0, s, gview(f), pview(f), f->N, grad_scale(f), f->nrm.p);
 }
 
 // Cells of the grid grown by 2 on each side.

@@ -349,6 +349,15 @@ void counters_reset(pi_frame* f, int first, int last);
 void counters_begin(pi_frame* f, bool* counted, int first, int last);
 void counters_read(pi_frame* f, unsigned long long out[kCounters]);
 
+// Lanes that share a particle's neighbourhood in k_xmean, k_cov_G, k_normals
+// (walk_row): four while a thread per particle leaves the SMs a few warps each,
+// whose long chains nothing hides (2,000 particles: 24 -> 22, 36 -> 25, 24 -> 18 us;
+// two radii, 50,000: 92 -> 65, 99 -> 93, 95 -> 35, a list per bin).  Past that
+// the repeated work costs more (60,000: 33 -> 43, 45 -> 64 us, the third even).
+inline int particle_lanes(const pi_frame* f) {
+  return f->N <= (f->varR ? 512LL : 192LL) * f->ctx->smCount ? 4 : 1;
+}
+
 // Host scalar constants with the reference's float/double semantics.
 float bspline_host(float ratio, float sigma);
 
