@@ -320,7 +320,7 @@ static long long point_cells(const pi_frame* f) {
 // the context's budget has room for both.
 static bool order_points(const pi_frame* f, long long m) {
   const long long nc = point_cells(f);
-  if (m < 16384 || nc > 4 * m || m > 0x7fffffffLL) return false;
+  if (m < 16384 || nc > 4 * m || m > 0x7fffffffLL || nc >= 0x7fffffffLL) return false;  // places and cells are ints
   const pi_ctx* c = f->ctx;
   const long long need = 4 * (nc + 1) + 12 * m + 4 * (long long)scan_tmp_ints(nc + 1);
   return !c->budget || c->used.load() + need <= (long long)c->budget;
