@@ -14,9 +14,10 @@
 //      name leaf pairs; mesh vertices are deduplicated by the sorted leaf-id
 //      pair, as Mesh::insert_vert keys them (src/global.cpp:13-32), the
 //      first (lowest) slot of a key winning, through a hash table in L2;
-//   4. one thread per mesh vertex bisects its leaf-to-leaf segment down to
-//      r/2 with a field evaluation per step and interpolates with the 0.1/0.9
-//      snap (calc_vertices, src/visitorextract.cpp:47-84);
+//   4. each mesh vertex's leaf-to-leaf segment is bisected down to r/2 with a
+//      field evaluation per step (a warp's vertices share the candidates,
+//      group_field) and interpolated with the 0.1/0.9 snap (calc_vertices,
+//      src/visitorextract.cpp:47-84);
 //   5. triangles are oriented by the table's flip and deduplicated by their
 //      sorted vertex triple, the first generated winning (Mesh::insert_tri,
 //      src/global.cpp:34-53).

@@ -2,9 +2,11 @@
 //
 // The reference keeps a LIFO of nodes but processes the whole frontier at
 // once (inProcessSize = 10^7), so refinement is breadth-first: one level per
-// iteration.  Per level:
+// iteration.  The levels above D_min come from k_top_test and k_top_nodes; then,
+// per level:
 //   k_empty      emptiness of beforeSampleEval / checkEmptyAndCalcCurv
-//                (:152-235): one warp per node, an existence test with early
+//                (:152-235), where the parents' scan (k_spawn_scan) has not
+//                settled it: one warp per node, an existence test with early
 //                exit over the hash cells that the node box grown by
 //                r * smooth_factor touches.  Every particle strictly inside
 //                the grown box lies in those cells (the float cell index is
@@ -18,8 +20,9 @@
 //                neighbouring nodes) are evaluated once; the order inside a
 //                bucket does not affect any result.
 //   k_q_eval     field at the bucketed points (Evaluator::SingleEval,
-//                src/evaluator.cpp:60-87): one warp per chunk of <= 32
-//                samples of one bucket; the cell's 27-cell candidates are
+//                src/evaluator.cpp:60-87): one warp per chunk of <= 32 K
+//                samples of one bucket (k_q_eval_thread on levels with a few
+//                samples per bucket: a thread each); the cell's 27-cell candidates are
 //                filtered against the chunk's bounding box into shared
 //                memory, then every lane walks the survivors (broadcast
 //                loads, uniform loop bounds).
