@@ -294,8 +294,8 @@ __device__ __forceinline__ uint32_t hash3(float x, float y, float z) {
   return h;
 }
 
-// Zeroes the hash slots of a level, two per sample counted (total = the scan's):
-// the samples of empty nodes have none, which are half of a leaf level's.
+// Zeroes the hash slots of a level, two per sample counted (total = the scan's;
+// the samples of empty nodes have none).
 __global__ void __launch_bounds__(256) k_q_clear(unsigned* __restrict__ hslot, const int* __restrict__ total) {
   launch_wait();
   const long long quads = (2LL * *total + 3) / 4;
@@ -794,9 +794,15 @@ __global__ void __launch_bounds__(64, 24) k_classify(LevelArgs a, const float* _
 // contiguous runs again.  Scattered 4-byte stores and loads bound it (a thread
 // per node reading and writing its own runs: 52 us for a sixteenth of the 4.2M
 // leaf-level nodes of a 1M frame; 50 this way, and the frame 0.6 ms less).
+// A thread gathers seven values at a time, so that their chains of two loads
+// overlap: a level of 2,000 particles 17 -> 9 us; all fourteen at once take
+// registers that the evaluation beside it on a QEF frame lacks.
 constexpr int kClassifyNodes = 128;
+constexpr int kClassifyThreads = 256;
+constexpr int kPer = 7;  // values a thread gathers at a time
+static_assert(kClassifyNodes * kQ % (kPer * kClassifyThreads) == 0, "the gather's rounds are whole");
 constexpr int kRunPad = kQ + 1;  // odd stride: a thread per node reads without bank conflicts
-__global__ void __launch_bounds__(256) k_classify_thread(LevelArgs a, const float* __restrict__ qval,
+__global__ void __launch_bounds__(kClassifyThreads) k_classify_thread(LevelArgs a, const float* __restrict__ qval,
                                                          const int* __restrict__ rep, const float4* __restrict__ nd_c,
                                                          float4* __restrict__ nd_v, int8_t* __restrict__ nd_type,
                                                          int8_t* __restrict__ nd_sc, float* __restrict__ nd_curv,
@@ -811,16 +817,36 @@ __global__ void __launch_bounds__(256) k_classify_thread(LevelArgs a, const floa
   if (plist) list += plist[2 * (parts + 1) + part];
   unsigned long long evals = 0;
   for (long long t0 = (long long)blockIdx.x * kClassifyNodes; t0 < n; t0 += (long long)gridDim.x * kClassifyNodes) {
+    float4 c = make_float4(0.f, 0.f, 0.f, 0.f), v = c;
+    float curv = 0.f;
     if (threadIdx.x < kClassifyNodes) {
       const long long t = t0 + threadIdx.x;
       int node = t < n ? (plist ? list[t] : (int)t) : -1;
-      if (node >= 0 && nd_type[a.lb + node] != T_UNCERTAIN) node = -1;
+      if (node >= 0) {  // the node's records load beside its type
+        c = nd_c[a.lb + node];
+        v = nd_v[a.lb + node];
+        curv = nd_curv[a.lb + node];
+        if (nd_type[a.lb + node] != T_UNCERTAIN) node = -1;
+      }
       s_node[threadIdx.x] = node;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < kClassifyNodes * kQ; i += 256) {
-      const int k = i / kQ, q = i % kQ, node = s_node[k];
-      if (node >= 0) s_val[k * kRunPad + q] = qval[__ldg(rep + (long long)node * kQ + q)];
+#pragma unroll 1
+    for (int i0 = threadIdx.x; i0 < kClassifyNodes * kQ; i0 += kPer * kClassifyThreads) {
+      int r[kPer];
+      float val[kPer];
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int i = i0 + u * kClassifyThreads, node = s_node[i / kQ];
+        r[u] = node >= 0 ? __ldg(rep + (long long)node * kQ + i % kQ) : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) val[u] = r[u] >= 0 ? qval[r[u]] : 0.f;
+#pragma unroll
+      for (int u = 0; u < kPer; ++u) {
+        const int i = i0 + u * kClassifyThreads;
+        s_val[i / kQ * kRunPad + i % kQ] = val[u];
+      }
     }
     __syncthreads();
     if (threadIdx.x < kClassifyNodes && s_node[threadIdx.x] >= 0) {
@@ -831,22 +857,20 @@ __global__ void __launch_bounds__(256) k_classify_thread(LevelArgs a, const floa
       bool signchange = false;
 #pragma unroll
       for (int q = 1; q < 27; ++q) signchange |= (val[q] >= 0.f) != origin;
-      const float4 c = nd_c[node];
       const float cellsize = 2.0f * c.w;
       const bool leaf_by_size = cellsize - a.radius < kAbove1em8;
       int8_t type = T_LEAF;
-      if (!leaf_by_size && signchange && nd_curv[node] < kAbove099) type = T_INTERNAL;
+      if (!leaf_by_size && signchange && curv < kAbove099) type = T_INTERNAL;
       nd_type[node] = type;
       nd_sc[node] = signchange ? 1 : 0;
       if (type == T_LEAF) {
-        float4 v = nd_v[node];
         v.w = val[27];
         nd_v[node] = v;
       }
       evals += 27 + (type == T_LEAF ? 1 : 0);
     }
     if (qef)
-      for (int i = threadIdx.x; i < kClassifyNodes * 27; i += 256) {
+      for (int i = threadIdx.x; i < kClassifyNodes * 27; i += kClassifyThreads) {
         const int k = i / 27, q = i % 27, node = s_node[k];
         if (node >= 0) nd_samp[(a.lb + node) * 27 + q] = s_val[k * kRunPad + q];
       }
@@ -1939,7 +1963,7 @@ void stage_octree(pi_frame* f) {
           // holds.  (Classified on the QEF stream, in front of the part's QEF,
           // the frame was 0.8 ms slower: the next part's evaluator takes the SMs
           // first and the part's QEF starts late.)
-          PI_LAUNCH(k_classify_thread, div_up(part_share(nl, parts), kClassifyNodes), 256, 0, s, la, qval.p, rep.p,
+          PI_LAUNCH(k_classify_thread, div_up(part_share(nl, parts), kClassifyNodes), kClassifyThreads, 0, s, la, qval.p, rep.p,
                     f->nd_c.p, f->nd_v.p, f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p,
                     (const int*)f->plist.p, (const int*)f->pnodes.p, parts, p);
           qef_level(f, lb, le, depth, parts, p);
@@ -1954,7 +1978,7 @@ void stage_octree(pi_frame* f) {
                   kEvalThreads, 0, s, qa, list, ucum.p + nb, qcnt.p + nb + 2, f->nd_c.p, f->nd_v.p, qval.p, f->dcount.p);
       prof_end(ctx, s, pg);
       if (known || leaf_level)  // no node needs a particle scan
-        PI_LAUNCH(k_classify_thread, div_up(nl, kClassifyNodes), 256, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
+        PI_LAUNCH(k_classify_thread, div_up(nl, kClassifyNodes), kClassifyThreads, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
                   f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p, (const int*)nullptr,
                   (const int*)nullptr, 0, 0);
       else
