@@ -661,6 +661,17 @@ __global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, i
       ++steps;
     }
   }
+  // group_field books a window's pairs on the lanes that hold its rows, whether
+  // they have a vertex or not: summed over the warp before those without leave
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+    steps += __shfl_xor_sync(0xffffffffu, steps, o);
+  }
+  if (lane == 0 && steps > 0) {
+    stripe_add(counters, C_BISECT_EVALS, (unsigned long long)steps);
+    stripe_add(counters, C_BISECT_PAIRS, (unsigned long long)pairs);
+  }
   if (!valid) return;
   vedge[v] = make_int2(A, B);
   const float ratio = __fdiv_rn(__fsub_rn(0.0f, p.w), __fsub_rn(q.w, p.w));
@@ -680,8 +691,6 @@ __global__ void __launch_bounds__(128, 8) k_bisect(BisectArgs a, long long nv, i
   uint64_t ia = nd_id[A], ib = nd_id[B];
   vkeys[2 * v] = ia < ib ? ia : ib;
   vkeys[2 * v + 1] = ia < ib ? ib : ia;
-  stripe_add(counters, C_BISECT_EVALS, (unsigned long long)steps);
-  stripe_add(counters, C_BISECT_PAIRS, (unsigned long long)pairs);
 }
 
 // Oriented triangle in Mesh::insert_tri argument order.
