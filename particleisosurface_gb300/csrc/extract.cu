@@ -958,11 +958,10 @@ void stage_extract(pi_frame* f) {
   BisectArgs ba{GridView{gh.bounding[0], gh.bounding[2], gh.bounding[4], gh.cell, gh.nx, gh.ny, gh.nz, f->off.p},
                 PartView{f->pos.p, f->xm.p, f->ga.p, f->gb.p, f->xlo.p}, f->iso, f->P.radius / 2, nullptr};
   if (f->varR) {
-    // bucket the vertices by a grid of cells 4 * maxR over the root box;
-    // bisect down to half the searcher's minimum radius
-    // (src/visitorextract.cpp:54)
-    const float bcell = f->vrMaxR * 4.0f;
-    const int bn = std::max(1, (int)std::ceil(2.0f * f->rootH / bcell));
+    // bucket the vertices by a grid over the root box; bisect down to half the
+    // searcher's minimum radius (src/visitorextract.cpp:54)
+    float bcell;
+    const int bn = vr_bucket_grid(f, &bcell);
     ba.g = GridView{f->rootC[0] - f->rootH, f->rootC[1] - f->rootH, f->rootC[2] - f->rootH, bcell, bn, bn, bn, nullptr};
     ba.rr = f->vrMinR / 2;
     ba.mg = f->mgv.p;

@@ -294,6 +294,12 @@ void stage_extract(pi_frame* f);
 // after the anisotropy pass; the icosahedra at vertex v0 and triangle t0.
 void stage_splash_list(pi_frame* f);
 void splash_mesh(pi_frame* f, long long v0, long long t0);
+// Sample and vertex buckets are numbered with ints.
+constexpr long long kMaxBuckets = 0x7fffffff - 1;
+// Variable radius: the grid over the root box that buckets samples and vertices,
+// cells per axis and cell size: 4 * maxR, doubled while the cells (grown by 2 on
+// each side) are more than kMaxBuckets.
+int vr_bucket_grid(const pi_frame* f, float* cell);
 // QEF vertices of the leaves of level [lb, le); with parts > 0 those of part
 // `part`, whose nodes (all leaves) the frame lists.
 void qef_level(pi_frame* f, long long lb, long long le, int depth, int parts = 0, int part = 0);

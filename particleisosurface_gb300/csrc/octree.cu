@@ -1666,6 +1666,17 @@ __global__ void __launch_bounds__(256, 4) k_vr_q_eval_thread(const MultiGridView
   }
 }
 
+// Samples of a level of nl nodes.  Their numbers are ints (in the bucket scans,
+// the representatives, the orders and the counters that warps take samples off,
+// which run past the last sample by 32 a warp).
+static long long level_samples(long long nl) {
+  constexpr long long most = (1LL << 31) - (1LL << 24);
+  if (nl * kQ > most)
+    throw std::length_error("octree level of " + std::to_string(nl) + " nodes: its " + std::to_string(nl * kQ) +
+                            " samples exceed the limit of " + std::to_string(most));
+  return nl * kQ;
+}
+
 // genIsoOurs state 0 with per-particle radii: every level runs the
 // emptiness scan above, then (depth >= D_min) the sampling, one thread per
 // distinct sample, and the classification with each node's min_radius.
@@ -1680,10 +1691,9 @@ static void stage_octree_vr(pi_frame* f) {
             f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p,
             f->nd_curv.p, f->nd_org.p);
   f->nNodes = 1;
-  // sample buckets: a grid of cells 4 * maxR over the root box (it holds
-  // every sample), whole cells
-  const float bcell = f->vrMaxR * 4.0f;
-  const int bn = std::max(1, (int)std::ceil(2.0f * f->rootH / bcell));
+  // sample buckets: a grid over the root box (it holds every sample), whole cells
+  float bcell;
+  const int bn = vr_bucket_grid(f, &bcell);
   GridView bg{f->rootC[0] - f->rootH, f->rootC[1] - f->rootH, f->rootC[2] - f->rootH, bcell, bn, bn, bn, nullptr};
   PartView P{f->pos.p, f->xm.p, f->ga.p, f->gb.p, f->xlo.p};
   const int ekx = bn + 4, eky = bn + 4;
@@ -1716,7 +1726,7 @@ static void stage_octree_vr(pi_frame* f) {
     if (depth < f->dmin)
       PI_LAUNCH(k_vr_big_leaf, div_up(nl, 128), 128, 0, s, f->mgv.p, la, f->nd_v.p, f->nd_type.p, f->dcount.p);
     if (depth >= f->dmin) {
-      const long long qn = nl * kQ;
+      const long long qn = level_samples(nl);
       if (f->tmp.n < scan_tmp_ints(nb + 1)) f->tmp.alloc(ctx, s, scan_tmp_ints(nb + 1));
       qkey.alloc(ctx, s, qn);
       rep.alloc(ctx, s, qn);
@@ -1785,7 +1795,14 @@ void stage_octree(pi_frame* f) {
   GridView g{gh.bounding[0], gh.bounding[2], gh.bounding[4], gh.cell, gh.nx, gh.ny, gh.nz, f->off.p};
   PartView P{f->pos.p, f->xm.p, f->ga.p, f->gb.p, f->xlo.p};
   const int ekx = gh.nx + 4, eky = gh.ny + 4;
-  const long long ek = (long long)ekx * eky * (gh.nz + 4) * 8;  // buckets: cell x octant
+  // buckets: cells (of the grid grown by 2, which a thin grid multiplies), and on
+  // the leaf level cell octants while their numbers fit an int
+  const long long cells = (long long)ekx * eky * (gh.nz + 4);
+  if (cells > kMaxBuckets)
+    throw std::length_error("octree sample buckets: " + std::to_string(cells) + " cells exceed the limit of " +
+                            std::to_string(kMaxBuckets));
+  const bool by_octant = cells <= kMaxBuckets / 8;
+  const long long ek = by_octant ? cells * 8 : cells;
   counters_begin(f, &f->octree_counted, 0, C_STAGE_TIMEOUT);
   DBuf<int> flag, qcnt, qkey, rep, order, ucum;
   DBuf<unsigned> hslot;
@@ -1893,10 +1910,10 @@ void stage_octree(pi_frame* f) {
                 f->nd_c.p, f->nd_v.p, f->nd_type.p, f->dcount.p);
       prof_end(ctx, s, PG_LEAF);
     } else if (depth >= f->dmin) {
-      const long long qn = nl * kQ;
+      const long long qn = level_samples(nl);
       // buckets: cell octants on the leaf level, whole cells above it
-      const int octants = depth == f->dmax ? 1 : 0;
-      const long long nb = octants ? ek : ek / 8;
+      const int octants = depth == f->dmax && by_octant ? 1 : 0;
+      const long long nb = octants ? ek : cells;
       if (f->tmp.n < scan_tmp_ints(nb + 1)) f->tmp.alloc(ctx, s, scan_tmp_ints(nb + 1));
       qkey.alloc(ctx, s, qn);
       rep.alloc(ctx, s, qn);

@@ -353,4 +353,11 @@ void host_root_and_scalars_vr(pi_frame* f) {
   f->sigma = (float)(1 / std::pow(smin, 6));
 }
 
+int vr_bucket_grid(const pi_frame* f, float* cell) {
+  for (*cell = f->vrMaxR * 4.0f;; *cell *= 2.0f) {
+    const int n = std::max(1, (int)std::ceil(2.0f * f->rootH / *cell));
+    if ((long long)(n + 4) * (n + 4) * (n + 4) <= kMaxBuckets) return n;
+  }
+}
+
 }  // namespace pisurf
