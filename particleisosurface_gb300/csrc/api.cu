@@ -113,17 +113,15 @@ void DBuf<T>::alloc(pi_ctx* c, cudaStream_t st, size_t count) {
 template <class T>
 void DBuf<T>::grow(pi_ctx* c, cudaStream_t st, size_t count, size_t keep) {
   if (count <= n) return;
-  DBuf<T> old;
-  std::swap(old.p, p);
-  std::swap(old.n, n);
-  std::swap(old.cap, cap);
-  old.ctx = ctx;
-  old.s = s;
-  alloc(c, st, count);
-  if (old.p) {
-    keep = keep < old.n ? keep : old.n;  // never past the old allocation
-    if (keep) PI_CUDA(cudaMemcpyAsync(p, old.p, keep * sizeof(T), cudaMemcpyDeviceToDevice, st));
-  }
+  DBuf<T> big;
+  big.alloc(c, st, count);  // where this fails the buffer stays as it is
+  keep = keep < n ? keep : n;  // never past the old allocation
+  if (p && keep) PI_CUDA(cudaMemcpyAsync(big.p, p, keep * sizeof(T), cudaMemcpyDeviceToDevice, st));
+  std::swap(p, big.p);
+  std::swap(n, big.n);
+  std::swap(cap, big.cap);
+  std::swap(ctx, big.ctx);
+  std::swap(s, big.s);
 }
 
 template <class T>

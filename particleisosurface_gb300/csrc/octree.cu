@@ -1415,9 +1415,13 @@ static void ensure_nodes(pi_frame* f, long long need) {
   // large enough and no samples yet
   const bool samp_ok = !f->P.qef || (long long)f->nd_samp.n >= need * 27;
   const bool minr_ok = !f->varR || (long long)f->nd_minr.n >= need;
-  if ((long long)f->nd_c.n >= need && samp_ok && minr_ok) return;
+  // growing may have failed part of the way (no memory), so each array is looked at
+  const size_t least = std::min({f->nd_c.n, f->nd_v.n, f->nd_id.n, f->nd_parent.n, f->nd_child.n, f->nd_type.n,
+                                 f->nd_depth.n, f->nd_sc.n, f->nd_curv.n, f->nd_org.n});
+  if ((long long)least >= need && samp_ok && minr_ok) return;
   qef_join(f);  // the QEF in flight writes node arrays that are about to move
-  long long cap = std::max<long long>(need, (long long)(f->nd_c.n * 3 / 2) + 1024);
+  long long cap = f->nd_c.n;
+  if (cap < need) cap = std::max(need, cap * 3 / 2 + 1024);
   pi_ctx* c = f->ctx;
   cudaStream_t s = c->stream;
   long long keep = f->nNodes;

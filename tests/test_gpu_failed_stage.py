@@ -1,0 +1,68 @@
+"""A frame whose stages fail for want of memory (PI_ERR_NOMEM under a budget)
+stays usable: a later attempt finds every node array and counts from zero."""
+import numpy as np
+import pytest
+
+from particleisosurface_gb300 import _native as N
+from particleisosurface_gb300 import build as B
+from particleisosurface_gb300 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _nomem(call):
+    with pytest.raises(N.PiError) as e:
+        call()
+    assert e.value.code == N.PI_ERR_NOMEM
+
+
+def _bytes(fr, stages):
+    c = N.Context(0)
+    f = N.Frame(c, N.default_params(fr.radius)).upload(fr.xyz)
+    for s in stages:
+        getattr(f, s)()
+    b = c.stats()["bytes"]
+    f.close()
+    c.close()
+    return b
+
+
+COUNTS = ("num_nodes", "num_leaves", "num_dual_cells", "num_vertices", "num_triangles", "field_evals",
+          "candidate_pairs", "bisection_evals", "fp64_eigen", "field_evals_performed", "qef_accepted", "qef_singular")
+
+
+@pytest.mark.parametrize("qef", [False, True])
+@pytest.mark.parametrize("share", [0.1, 0.3, 0.6, 0.9])
+def test_counts_after_a_failed_attempt(qef, share):
+    """Another frame takes the memory that the octree or the extraction needs; when
+    it is gone the stage runs again, and every count is a first run's."""
+    B.build()
+    fr = synth.slab_and_sphere(n=20000, seed=1)
+    p = N.default_params(fr.radius, qef=qef)
+    lo, hi = _bytes(fr, ["hashgrid", "aniso", "normals"]), 1 << 30
+    whole = None
+    while hi - lo > 1 << 16:  # the least budget of the whole frame
+        b = (lo + hi) // 2
+        c = N.Context(0, budget_bytes=b)
+        f = N.Frame(c, p).upload(fr.xyz)
+        try:
+            info = f.run().info()
+            whole, hi = {k: info[k] for k in COUNTS}, b
+        except N.PiError as e:
+            assert e.code == N.PI_ERR_NOMEM
+            lo = b
+        f.close()
+        c.close()
+    base = _bytes(fr, ["hashgrid", "aniso", "normals"])
+    # node arrays that have grown stay: a second attempt may need more than a first
+    c = N.Context(0, budget_bytes=2 * hi)
+    other = N.Frame(c, p)
+    f = N.Frame(c, p).upload(fr.xyz).hashgrid().aniso().normals()
+    # 12 bytes a particle: what the other frame leaves is `share` of what the rest needs
+    other.upload(np.zeros((int(hi + (1 - share) * (hi - base)) // 12, 3), np.float32))
+    _nomem(lambda: f.octree().extract())
+    other.close()
+    info = f.octree().extract().info()
+    assert {k: info[k] for k in COUNTS} == whole
+    f.close()
+    c.close()
