@@ -353,6 +353,9 @@ static void run_stage(pi_frame* f, int target) {
   ev_record(f, 2 * slot);
   switch (target) {
     case 2:
+      // counts that an attempt which failed later left unread are not this
+      // attempt's, whose offset table may not be there if it fails too
+      f->pin_pending = 0;
       if (f->varR)
         stage_hashgrid_vr(f);
       else

@@ -1,5 +1,6 @@
 """A frame whose stages fail for want of memory (PI_ERR_NOMEM under a budget)
-stays usable: a later attempt finds every node array and counts from zero."""
+stays usable: its info can be read, and a later attempt finds every node array
+and counts from zero."""
 import numpy as np
 import pytest
 
@@ -25,6 +26,26 @@ def _bytes(fr, stages):
     f.close()
     c.close()
     return b
+
+
+def test_info_after_two_failed_attempts():
+    """The first attempt fails behind the hash stage and leaves its count of valid
+    keys unread; the second one fails in the hash stage, at a table of 10^8 cells."""
+    B.build()
+    fr = synth.small_blob(n=2000, seed=3)
+    c = N.Context(0, budget_bytes=_bytes(fr, ["hashgrid"]) + 16384)
+    f = N.Frame(c, N.default_params(fr.radius)).upload(fr.xyz)
+    _nomem(f.run)
+    wide = fr.xyz.copy()
+    wide[0] = wide.max(0) + 500 * 4 * fr.radius
+    f.upload(wide)
+    _nomem(f.run)
+    info = f.info()
+    assert info["num_particles"] == fr.n and info["num_triangles"] == 0
+    f.upload(fr.xyz).hashgrid()
+    assert f.info()["num_invalid_keys"] == int(np.sum(f.dump(N.DUMP_KEYS) < 0))
+    f.close()
+    c.close()
 
 
 COUNTS = ("num_nodes", "num_leaves", "num_dual_cells", "num_vertices", "num_triangles", "field_evals",
