@@ -342,15 +342,7 @@ struct NvtxRange {
   ~NvtxRange() { nvtxRangePop(); }
 };
 
-static void run_stage(pi_frame* f, int target) {
-  // target: 2 hash, 3 aniso, 4 normals, 5 octree, 6 mesh
-  if (f->stage >= target) return;
-  need(f, target - 1);
-  static const char* const names[7] = {"", "", "pisurf hash grid", "pisurf anisotropy", "pisurf normals",
-                                        "pisurf octree", "pisurf extraction"};
-  NvtxRange range(names[target]);
-  const int slot = target == 2 ? 1 : target == 3 ? 2 : target == 4 ? 3 : target == 5 ? 4 : 6;
-  ev_record(f, 2 * slot);
+static void stage_work(pi_frame* f, int target) {
   switch (target) {
     case 2:
       // counts that an attempt which failed later left unread are not this
@@ -383,6 +375,26 @@ static void run_stage(pi_frame* f, int target) {
     case 6:
       stage_extract(f);
       break;
+  }
+}
+
+static void run_stage(pi_frame* f, int target) {
+  // target: 2 hash, 3 aniso, 4 normals, 5 octree, 6 mesh
+  if (f->stage >= target) return;
+  need(f, target - 1);
+  static const char* const names[7] = {"", "", "pisurf hash grid", "pisurf anisotropy", "pisurf normals",
+                                        "pisurf octree", "pisurf extraction"};
+  NvtxRange range(names[target]);
+  const int slot = target == 2 ? 1 : target == 3 ? 2 : target == 4 ? 3 : target == 5 ? 4 : 6;
+  ev_record(f, 2 * slot);
+  try {
+    stage_work(f, target);
+  } catch (...) {
+    // the helper streams' work on the frame comes before whatever the context
+    // stream does to its buffers next
+    qef_join(f);
+    topology_join(f);
+    throw;
   }
   ev_record(f, 2 * slot + 1);
   ev_close(f, slot);
@@ -849,7 +861,6 @@ int pi_run(pi_frame* f) {
     for (int t = 2; t <= 6; ++t) run_stage(f, t);
   } catch (...) {
     f->defer_qef_join = f->extract_follows = false;
-    topology_join(f);
     throw;
   }
   f->defer_qef_join = f->extract_follows = false;

@@ -817,9 +817,14 @@ void topology_start(pi_frame* f) {
   pi_ctx* c = f->ctx;
   cudaStream_t ts = c->topo_stream;
   PI_CUDA(cudaStreamWaitEvent(ts, c->ev_topo_in, 0));
-  extract_topology(f, ts, CountReader{f, ts, kPinTopoReadOffset, c->ev_topo_read});
-  PI_CUDA(cudaEventRecord(c->ev_topo_done, ts));
   f->tp_inflight = true;
+  try {
+    extract_topology(f, ts, CountReader{f, ts, kPinTopoReadOffset, c->ev_topo_read});
+  } catch (...) {
+    cudaEventRecord(c->ev_topo_done, ts);  // what was launched is joined all the same
+    throw;
+  }
+  PI_CUDA(cudaEventRecord(c->ev_topo_done, ts));
 }
 
 void topology_join(pi_frame* f) {
@@ -859,11 +864,8 @@ void stage_extract(pi_frame* f) {
   if (tmp.n < scan_tmp_ints(nu + 1)) tmp.alloc(c, s, scan_tmp_ints(nu + 1));
   const CountReader rd{f, s, kPinReadOffset, c->ev_read};
   // k_dual reads the leaves' values: the octree's last QEF level, if it was
-  // left running, ends here, and the octree's counters are taken
-  if (f->qef_inflight) {
-    qef_join(f);
-    counters_snapshot(f, kPinOctree);
-  }
+  // left running, ends here
+  qef_join(f);
   counters_begin(f, &f->extract_counted, C_DUAL, C_BISECT_PAIRS);
   PI_LAUNCH(k_dual, div_up(nu + 1, 128), 128, 0, s, uverts, nu, B, f->nd_child.p, f->nd_v.p,
             cells.p, reinterpret_cast<uint8_t*>(procs.p), toff.p, f->dcount.p);

@@ -257,8 +257,9 @@ constexpr int kPinTopoReadOffset = kPinReadOffset + 8;
 constexpr int kPinWords = kPinTopoReadOffset + 8;
 // event that marks the INTERNAL count's copy in the octree level loop
 constexpr int kLevelEvent = 16;
-// The counters of a stage (kPin...) are complete on the context stream; they
-// reach the frame in resolve_pending, which copies them once for all stages.
+// The counters of a stage (kPin...) are complete on the context stream (the
+// octree's when the QEF stream's work is joined); they reach the frame in
+// resolve_pending, which joins it and copies them once for all stages.
 void counters_snapshot(pi_frame* f, int slot);
 // Parameter checks of pi_frame_create (throws std::invalid_argument).
 void check_params(const pi_params* p);

@@ -2041,12 +2041,10 @@ void stage_octree(pi_frame* f) {
     lb = le;
     le = le + newn;
   }
-  // the last level's QEF may run on while the extraction builds the mesh
-  // topology (stage_extract joins it before it reads node values, and takes
-  // the octree's counters then)
-  if (f->defer_qef_join && f->qef_inflight) return;
-  qef_join(f);
   counters_snapshot(f, kPinOctree);
+  // the last level's QEF may run on while the extraction builds the mesh
+  // topology (stage_extract joins it before it reads node values)
+  if (!f->defer_qef_join) qef_join(f);
 }
 
 }  // namespace pisurf

@@ -52,17 +52,11 @@ COUNTS = ("num_nodes", "num_leaves", "num_dual_cells", "num_vertices", "num_tria
           "candidate_pairs", "bisection_evals", "fp64_eigen", "field_evals_performed", "qef_accepted", "qef_singular")
 
 
-@pytest.mark.parametrize("qef", [False, True])
-@pytest.mark.parametrize("share", [0.1, 0.3, 0.6, 0.9])
-def test_counts_after_a_failed_attempt(qef, share):
-    """Another frame takes the memory that the octree or the extraction needs; when
-    it is gone the stage runs again, and every count is a first run's."""
-    B.build()
-    fr = synth.slab_and_sphere(n=20000, seed=1)
-    p = N.default_params(fr.radius, qef=qef)
+def _least_budget(fr, p):
+    """The least budget of the whole frame, and its counts."""
     lo, hi = _bytes(fr, ["hashgrid", "aniso", "normals"]), 1 << 30
     whole = None
-    while hi - lo > 1 << 16:  # the least budget of the whole frame
+    while hi - lo > 1 << 16:
         b = (lo + hi) // 2
         c = N.Context(0, budget_bytes=b)
         f = N.Frame(c, p).upload(fr.xyz)
@@ -74,16 +68,33 @@ def test_counts_after_a_failed_attempt(qef, share):
             lo = b
         f.close()
         c.close()
+    return hi, whole
+
+
+@pytest.mark.parametrize("staged", [False, True])
+@pytest.mark.parametrize("qef", [False, True])
+@pytest.mark.parametrize("share", [0.1, 0.3, 0.6, 0.9])
+def test_counts_after_a_failed_attempt(qef, share, staged):
+    """Another frame takes the memory that the octree or the extraction needs; when
+    it is gone the stage runs again, at once or after its info was read, and every
+    count is a first run's."""
+    B.build()
+    fr = synth.slab_and_sphere(n=20000, seed=1)
+    p = N.default_params(fr.radius, qef=qef)
+    least, whole = _least_budget(fr, p)
     base = _bytes(fr, ["hashgrid", "aniso", "normals"])
     # node arrays that have grown stay: a second attempt may need more than a first
-    c = N.Context(0, budget_bytes=2 * hi)
+    c = N.Context(0, budget_bytes=2 * least)
     other = N.Frame(c, p)
     f = N.Frame(c, p).upload(fr.xyz).hashgrid().aniso().normals()
+    rest = (lambda: f.octree().extract()) if staged else f.run
     # 12 bytes a particle: what the other frame leaves is `share` of what the rest needs
-    other.upload(np.zeros((int(hi + (1 - share) * (hi - base)) // 12, 3), np.float32))
-    _nomem(lambda: f.octree().extract())
+    other.upload(np.zeros((int(least + (1 - share) * (least - base)) // 12, 3), np.float32))
+    _nomem(rest)
+    if share != 0.6:
+        f.info()
     other.close()
-    info = f.octree().extract().info()
+    info = rest().info()
     assert {k: info[k] for k in COUNTS} == whole
     f.close()
     c.close()
