@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(kBigThreads) k_cell_sort_big(const float* __re
 
 void stage_upload_host(pi_frame* f, const float* xyz, long long n) {
   cudaStream_t s = f->ctx->stream;
+  f->stage = 0;  // no particles until they are here: the results are of another count
   f->N = n;
   f->xyz.alloc(f->ctx, s, (size_t)n * 3);
   PI_CUDA(cudaMemcpyAsync(f->xyz.p, xyz, sizeof(float) * 3 * n, cudaMemcpyHostToDevice, s));
@@ -268,6 +269,7 @@ void stage_upload_host(pi_frame* f, const float* xyz, long long n) {
 
 void stage_upload_device(pi_frame* f, const float* d_xyz, long long n) {
   cudaStream_t s = f->ctx->stream;
+  f->stage = 0;  // no particles until they are here: the results are of another count
   f->N = n;
   f->xyz.alloc(f->ctx, s, (size_t)n * 3);
   PI_CUDA(cudaMemcpyAsync(f->xyz.p, d_xyz, sizeof(float) * 3 * n, cudaMemcpyDeviceToDevice, s));

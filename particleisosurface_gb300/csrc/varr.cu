@@ -138,6 +138,7 @@ void stage_upload_radii(pi_frame* f, const float* radii, long long n) {
                        (float)(1.0 / ((double)nI * nI * nI)));
   }
   cudaStream_t s = f->ctx->stream;
+  if (f->varR) f->stage = 0;  // its radii go; no results until the new ones are here
   f->rad.alloc(f->ctx, s, n);
   f->vrc.alloc(f->ctx, s, n);
   PI_CUDA(cudaMemcpyAsync(f->rad.p, radii, sizeof(float) * n, cudaMemcpyHostToDevice, s));

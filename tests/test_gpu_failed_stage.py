@@ -48,6 +48,40 @@ def test_info_after_two_failed_attempts():
     c.close()
 
 
+def _state(call):
+    with pytest.raises(N.PiError) as e:
+        call()
+    assert e.value.code == N.PI_ERR_STATE
+
+
+def test_failed_uploads_leave_no_results():
+    """The results of a frame are of the particles it had before an upload that fails;
+    none can be asked for until there are particles again."""
+    B.build()
+    fr = synth.two_radius_frame(n=2000, seed=6)
+    p = N.default_params(float(fr.radii.min()))
+    probe = N.Context(0)
+    f = N.Frame(probe, p).upload(fr.xyz).upload_radii(fr.radii).hashgrid().aniso()
+    used = probe.stats()["bytes"]
+    want = f.dump(N.DUMP_XMEANS)
+    f.close()
+    probe.close()
+    c = N.Context(0, budget_bytes=used + (1 << 20))
+    f = N.Frame(c, p).upload(fr.xyz).upload_radii(fr.radii).hashgrid().aniso()
+    _nomem(lambda: f.upload(np.zeros((1 << 20, 3), np.float32)))
+    _state(lambda: f.dump(N.DUMP_XMEANS))
+    _state(f.hashgrid)
+    f.upload(fr.xyz).upload_radii(fr.radii).hashgrid().aniso()
+    assert np.array_equal(f.dump(N.DUMP_XMEANS), want)
+    g = N.Frame(c, p)  # one that has never held any
+    _nomem(lambda: g.upload(np.zeros((1 << 20, 3), np.float32)))
+    _state(lambda: g.upload_radii(fr.radii))
+    _state(g.hashgrid)
+    g.close()
+    f.close()
+    c.close()
+
+
 COUNTS = ("num_nodes", "num_leaves", "num_dual_cells", "num_vertices", "num_triangles", "field_evals",
           "candidate_pairs", "bisection_evals", "fp64_eigen", "field_evals_performed", "qef_accepted", "qef_singular")
 
