@@ -38,34 +38,46 @@ void ctx_account(pi_ctx* c, long long delta) {
   }
 }
 
+// Takes kept block b off the list (keep_mu held).
+static pi_ctx::KeptBlock keep_remove(pi_ctx* c, std::vector<pi_ctx::KeptBlock>::iterator b) {
+  const pi_ctx::KeptBlock k = *b;
+  c->kept_bytes -= k.bytes;
+  c->kept.erase(b);
+  return k;
+}
+
+static bool keep_below(const pi_ctx::KeptBlock& b, size_t bytes) { return b.bytes < bytes; }
+
 // The kept block that fits best: at least `bytes`, at most twice that (or 64 KiB
 // more).
 static void* keep_take(pi_ctx* c, cudaStream_t st, size_t bytes, size_t* got) {
   if (!c || c->budget || bytes > kKeepBlock) return nullptr;
   std::lock_guard<std::mutex> lk(c->keep_mu);
   const size_t most = std::max(2 * bytes, bytes + 65536);
-  size_t best = c->kept.size();
-  for (size_t i = 0; i < c->kept.size(); ++i) {
-    const auto& b = c->kept[i];
-    if (b.s == st && b.bytes >= bytes && b.bytes <= most &&
-        (best == c->kept.size() || b.bytes < c->kept[best].bytes))
-      best = i;
-  }
-  if (best == c->kept.size()) return nullptr;
-  void* const p = c->kept[best].p;
-  *got = c->kept[best].bytes;
-  c->kept_bytes -= *got;
-  c->kept[best] = c->kept.back();
-  c->kept.pop_back();
-  return p;
+  auto b = std::lower_bound(c->kept.begin(), c->kept.end(), bytes, keep_below);
+  while (b != c->kept.end() && b->bytes <= most && b->s != st) ++b;
+  if (b == c->kept.end() || b->bytes > most) return nullptr;
+  const pi_ctx::KeptBlock k = keep_remove(c, b);
+  *got = k.bytes;
+  return k.p;
 }
 
 static bool keep_put(pi_ctx* c, void* p, size_t bytes, cudaStream_t st) {
   if (!c || c->budget || bytes > kKeepBlock) return false;
   std::lock_guard<std::mutex> lk(c->keep_mu);
-  if (c->kept_bytes + bytes > kKeepBytes) return false;
+  const uint64_t now = ++c->keep_clock;
+  while (c->kept_bytes + bytes > kKeepBytes || c->kept.size() >= kKeepCount) {
+    auto b = std::min_element(c->kept.begin(), c->kept.end(),
+                              [](const auto& x, const auto& y) { return x.when < y.when; });
+    if (now - b->when <= kKeepAge) {
+      b = c->kept.end() - 1;
+      if (b->bytes <= bytes) return false;
+    }
+    const pi_ctx::KeptBlock k = keep_remove(c, b);
+    cudaFreeAsync(k.p, k.s);
+  }
   try {
-    c->kept.push_back({p, bytes, st});
+    c->kept.insert(std::lower_bound(c->kept.begin(), c->kept.end(), bytes, keep_below), {p, bytes, st, now});
   } catch (...) {
     return false;
   }

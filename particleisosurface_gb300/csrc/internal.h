@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
+#include <cstdint>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -62,7 +63,10 @@ struct GridHost {
 // Configurations of the chunked field evaluation at octree samples
 // (octree.cu): samples per lane, warps per block, staged candidates per warp.
 constexpr int kMaxQefParts = 64;  // pi_ctx_tune_qef_parts
-constexpr size_t kKeepBlock = 64u << 20, kKeepBytes = 256u << 20;  // kept blocks (pi_ctx::kept)
+// kept blocks (pi_ctx::kept): bytes of one, bytes and number of all, and the
+// releases (several frames' worth) after which one counts as stale
+constexpr size_t kKeepBlock = 64u << 20, kKeepBytes = 256u << 20, kKeepCount = 512;
+constexpr uint64_t kKeepAge = 1024;
 
 struct EvalConfig {
   int K, W, CB, bulk;
@@ -81,16 +85,21 @@ struct pi_ctx {
   // size on the same stream (whose order makes the reuse safe, as it does for
   // the pool): a small frame allocates sixty buffers, and the pool's calls sat
   // between its short kernels.  Only without a budget, blocks up to
-  // kKeepBlock, kKeepBytes in all; given back when an allocation fails and when
+  // kKeepBlock, kKeepBytes in all.  When they are full a block gives way that
+  // nothing has asked for in a while, else the largest: many small blocks are
+  // what a small frame needs, and a large frame's few calls of the pool are
+  // little beside its kernels.  Given back when an allocation fails and when
   // the context goes.  Not counted in `used`, as the pool's free memory is not.
   struct KeptBlock {
     void* p;
     size_t bytes;
     cudaStream_t s;
+    uint64_t when;  // keep_clock at its release
   };
   std::mutex keep_mu;
-  std::vector<KeptBlock> kept;
+  std::vector<KeptBlock> kept;  // by size
   size_t kept_bytes = 0;
+  uint64_t keep_clock = 0;  // releases
   bool profile = false;
   // per kernel group (ProfGroup): event pairs (start, stop) not read yet, and
   // the accumulated device time, launches, candidate pairs and work units
