@@ -85,12 +85,29 @@ static bool keep_put(pi_ctx* c, void* p, size_t bytes, cudaStream_t st) {
   return true;
 }
 
-static void keep_free(pi_ctx* c) {
-  if (!c) return;
-  std::lock_guard<std::mutex> lk(c->keep_mu);
-  for (const auto& b : c->kept) cudaFreeAsync(b.p, b.s);
-  c->kept.clear();
-  c->kept_bytes = 0;
+// The streams of the blocks given back are waited for where the memory is wanted
+// at once.
+static void keep_free(pi_ctx* c, bool wait) {
+  std::vector<pi_ctx::KeptBlock> kept;
+  {
+    std::lock_guard<std::mutex> lk(c->keep_mu);
+    kept.swap(c->kept);
+    c->kept_bytes = 0;
+  }
+  for (const auto& b : kept) cudaFreeAsync(b.p, b.s);
+  cudaStream_t waited = nullptr;
+  for (const auto& b : kept)
+    if (wait && b.s != waited) cudaStreamSynchronize(waited = b.s);
+}
+
+// The contexts alive, so that an allocation that fails can have what they keep.
+static std::mutex g_ctx_mu;
+static std::vector<pi_ctx*> g_ctxs;
+
+static void keep_free_device(int device) {
+  std::lock_guard<std::mutex> lk(g_ctx_mu);
+  for (pi_ctx* c : g_ctxs)
+    if (c->device == device) keep_free(c, true);
 }
 
 template <class T>
@@ -105,7 +122,7 @@ void DBuf<T>::alloc(pi_ctx* c, cudaStream_t st, size_t count) {
     cudaError_t e = cudaMallocAsync(&q, bytes, st);
     if (e == cudaErrorMemoryAllocation) {
       (void)cudaGetLastError();
-      keep_free(c);
+      if (c) keep_free_device(c->device);
       e = cudaMallocAsync(&q, bytes, st);
     }
     if (e != cudaSuccess) {
@@ -533,14 +550,22 @@ int pi_ctx_create(int device, size_t budget_bytes, pi_ctx** out) {
   PI_CUDA(cudaDeviceGetDefaultMemPool(&pool, device));
   uint64_t thr = UINT64_MAX;
   PI_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
+  {
+    std::lock_guard<std::mutex> lk(g_ctx_mu);
+    g_ctxs.push_back(c.get());
+  }
   *out = c.release();
   PI_API_END
 }
 
 static void ctx_release(pi_ctx* c) {
   if (c->refs.fetch_sub(1) != 1) return;
+  {
+    std::lock_guard<std::mutex> lk(g_ctx_mu);
+    g_ctxs.erase(std::find(g_ctxs.begin(), g_ctxs.end(), c));
+  }
   cudaSetDevice(c->device);
-  keep_free(c);
+  keep_free(c, false);
   cudaStreamSynchronize(c->stream);
   if (c->topo_stream) {
     cudaStreamSynchronize(c->topo_stream);

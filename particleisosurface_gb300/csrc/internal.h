@@ -88,8 +88,9 @@ struct pi_ctx {
   // kKeepBlock, kKeepBytes in all.  When they are full a block gives way that
   // nothing has asked for in a while, else the largest: many small blocks are
   // what a small frame needs, and a large frame's few calls of the pool are
-  // little beside its kernels.  Given back when an allocation fails and when
-  // the context goes.  Not counted in `used`, as the pool's free memory is not.
+  // little beside its kernels.  Given back when an allocation of any context
+  // of the device fails and when the context goes.  Not counted in `used`, as
+  // the pool's free memory is not.
   struct KeptBlock {
     void* p;
     size_t bytes;

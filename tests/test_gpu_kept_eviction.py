@@ -1,6 +1,7 @@
 """What a context keeps of released device blocks serves the frames that follow:
 small frames take next to nothing from the pool after a large frame has filled
-the list.  Seen through the pool's own counters."""
+the list, and a context gets the memory that an idle one keeps.  Seen through the
+pool's own counters."""
 import ctypes as C
 
 import pytest
@@ -11,7 +12,7 @@ from particleisosurface_gb300 import synth
 
 pytestmark = pytest.mark.gpu
 
-USED_CURRENT, USED_HIGH = 7, 8  # CU_MEMPOOL_ATTR_USED_MEM_...
+RESERVED, USED_CURRENT, USED_HIGH = 5, 7, 8  # CU_MEMPOOL_ATTR_RESERVED_MEM_CURRENT, ..._USED_MEM_...
 
 
 class Pool:
@@ -59,3 +60,30 @@ def test_small_frames_after_a_large_one(first):
     _frame(ctx, small)
     assert pool.taken_by(lambda: _frame(ctx, small)) < whole // 20
     ctx.close()
+
+
+def test_an_idle_context_gives_its_blocks():
+    B.build()
+    fr = synth.dam_break(n=300_000, seed=2)
+    idle, other, probe = N.Context(0), N.Context(0), N.Context(0)
+    pool = Pool()
+    need = pool.taken_by(lambda: _frame(probe, fr))
+    probe.close()
+    _frame(idle, synth.dam_break(n=600_000, seed=2))
+    kept = pool.get(USED_CURRENT)
+    assert kept > 200 << 20
+    assert pool.cu.cuCtxSynchronize() == 0 and pool.cu.cuMemPoolTrimTo(pool.pool, C.c_size_t(0)) == 0
+    # the device's memory goes but for 100 MB less than the frame needs, which the
+    # idle context keeps twice over
+    left = need - (pool.get(RESERVED) - kept) - (100 << 20)
+    assert left > 0
+    free, total = C.c_size_t(), C.c_size_t()
+    assert pool.cu.cuMemGetInfo_v2(C.byref(free), C.byref(total)) == 0
+    block = C.c_uint64()
+    assert pool.cu.cuMemAlloc_v2(C.byref(block), C.c_size_t(free.value - left)) == 0
+    try:
+        _frame(other, fr)
+    finally:
+        assert pool.cu.cuMemFree_v2(block) == 0
+    other.close()
+    idle.close()
