@@ -127,7 +127,10 @@ __global__ void k_cell_count(const int* __restrict__ key, long long n, int* __re
 // launches and block barriers).  Particles outside the grid (key -1) form a range
 // of their own at the front, as the reference's sort puts them.
 // ---------------------------------------------------------------------------
-constexpr int kSmallCell = 256;  // larger cells are radix-sorted by a block each
+constexpr int kSmallCell = 256;   // larger cells are radix-sorted by a block each
+constexpr int kHugeCell = 4096;   // still larger ones are split over blocks by index windows
+constexpr int kWindowWords = 10240;  // bits of a window's particles, in shared memory
+constexpr int kWindows = 32;         // windows at least
 
 // Key, and the particle's place in its cell (cnt: cell counts, zeroed;
 // *outside: particles of key -1).
@@ -171,11 +174,12 @@ __device__ __forceinline__ void put_particle(const float* __restrict__ xyz, uint
 }
 
 // A thread per particle counts the lower indices of its cell; the first one of
-// a cell above kSmallCell lists the cell instead.
+// a cell above kSmallCell lists the cell instead (big: [0, listed), the cells
+// above kHugeCell from its end; nbig: both counts).
 __global__ void k_cell_sort(const float* __restrict__ xyz, const int* __restrict__ key,
                             const uint32_t* __restrict__ list, const int* __restrict__ off, long long cells,
                             long long n, uint32_t* __restrict__ sidx, float4* __restrict__ pos, int* __restrict__ big,
-                            unsigned* __restrict__ nbig) {
+                            long long listed, unsigned* __restrict__ nbig) {
   launch_wait();
   const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) return;
@@ -184,7 +188,12 @@ __global__ void k_cell_sort(const float* __restrict__ xyz, const int* __restrict
   int s, e;
   cell_range(off, cells, n, k, &s, &e);
   if (e - s > kSmallCell) {
-    if (t == s) big[atomicAdd(nbig, 1u)] = k;
+    if (t == s) {
+      if (e - s > kHugeCell)
+        big[listed - 1 - atomicAdd(nbig + 1, 1u)] = k;
+      else
+        big[atomicAdd(nbig, 1u)] = k;
+    }
     return;
   }
   int rank = 0;
@@ -192,20 +201,88 @@ __global__ void k_cell_sort(const float* __restrict__ xyz, const int* __restrict
   put_particle(xyz, i, s + rank, sidx, pos);
 }
 
-// The listed cells: a block per cell, stable 8-bit radix passes over the
-// particle indices (list and alt in turn; four passes end in list).
+// A window of a huge cell's particles, by a block: the indices of [w width,
+// (w + 1) width) as bits, and the number of lower ones; what comes before a
+// particle in the cell is then a count of bits.  Every window reads all of the
+// cell's list, so that none waits for another.
 constexpr int kBigThreads = 256;
+__device__ void cell_window(const float* __restrict__ xyz, const uint32_t* __restrict__ list, long long n, int s, int e,
+                            uint32_t w, uint32_t width, unsigned* bits, int* s_sum, uint32_t* __restrict__ sidx,
+                            float4* __restrict__ pos) {
+  constexpr int warps = kBigThreads / 32;
+  const int x = threadIdx.x, lane = x & 31, warp = x >> 5;
+  const int words = (int)(width / 32);
+  const uint32_t lo = w * width;
+  for (int k = x; k < words; k += kBigThreads) bits[k] = 0u;
+  __syncthreads();
+  int below = 0;
+  auto take = [&](long long t, uint32_t i) {
+    if (t < s || t >= e) return;
+    if (i < lo)
+      ++below;
+    else if (i - lo < width)
+      atomicOr(bits + ((i - lo) >> 5), 1u << (i & 31u));  // lo is a multiple of 32
+  };
+#pragma unroll 4
+  for (long long q = s / 4 + x; q < (e + 3) / 4; q += kBigThreads) {
+    if (4 * q + 3 < n) {
+      const uint4 v = reinterpret_cast<const uint4*>(list)[q];
+      take(4 * q, v.x), take(4 * q + 1, v.y), take(4 * q + 2, v.z), take(4 * q + 3, v.w);
+    } else {
+      for (long long t = 4 * q; t < n; ++t) take(t, list[t]);
+    }
+  }
+  below = __reduce_add_sync(0xffffffffu, below);
+  if (lane == 0) s_sum[warp] = below;
+  __syncthreads();
+  // a thread's run of words
+  const int run = (words + kBigThreads - 1) / kBigThreads, k0 = min(x * run, words), k1 = min(k0 + run, words);
+  int count = 0;
+  for (int k = k0; k < k1; ++k) count += __popc(bits[k]);
+  int inc = count;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  if (lane == 31) s_sum[warps + warp] = inc;
+  __syncthreads();
+  long long at = s + inc - count;
+  for (int k = 0; k < warps; ++k) at += s_sum[k] + (k < warp ? s_sum[warps + k] : 0);
+  for (int k = k0; k < k1; ++k)
+    for (unsigned b = bits[k]; b != 0u; b &= b - 1u)
+      put_particle(xyz, lo + 32u * k + (uint32_t)(__ffs(b) - 1), at++, sidx, pos);
+  __syncthreads();
+}
+
+// The listed cells.  Up to kHugeCell a block per cell, stable 8-bit radix passes
+// over the particle indices (list and alt in turn; four passes end in list).
+// Larger ones (a clump, or a lattice's face on the grid's upper bound, all of
+// which has key -1) in windows: one block's passes, three barriers for 256
+// particles each, took 390 us of a 1M lattice with 30,000 particles on the
+// bound and 13.3 ms of 1M particles in one cell.
 __global__ void __launch_bounds__(kBigThreads) k_cell_sort_big(const float* __restrict__ xyz, uint32_t* list,
                                                                uint32_t* alt, const int* __restrict__ off,
                                                                long long cells, long long n,
                                                                uint32_t* __restrict__ sidx, float4* __restrict__ pos,
-                                                               const int* __restrict__ big,
+                                                               const int* __restrict__ big, long long listed,
                                                                const unsigned* __restrict__ nbig) {
   launch_wait();
   constexpr int warps = kBigThreads / 32;
+  __shared__ unsigned s_bits[kWindowWords];
   __shared__ int s_run[256];
-  __shared__ int s_cnt[warps][256];
   const int x = threadIdx.x, lane = x & 31, warp = x >> 5;
+  // windows as wide as the bits allow, or narrower
+  const uint32_t span = max((uint32_t)kWindows, (uint32_t)((n + 32ll * kWindowWords - 1) / (32ll * kWindowWords)));
+  const uint32_t width = (uint32_t)((n + 32ll * span - 1) / (32ll * span)) * 32u;
+  const uint32_t windows = (uint32_t)((n + width - 1) / width);
+  for (long long t = blockIdx.x; t < (long long)nbig[1] * windows; t += gridDim.x) {
+    int s, e;
+    cell_range(off, cells, n, big[listed - 1 - t / windows], &s, &e);
+    cell_window(xyz, list, n, s, e, (uint32_t)(t % windows), width, s_bits, s_run, sidx, pos);
+  }
+  int(*const s_cnt)[256] = reinterpret_cast<int(*)[256]>(s_bits);
+  static_assert(warps * 256 <= kWindowWords && 2 * warps <= 256, "shared by the two paths");
   for (unsigned b = blockIdx.x; b < *nbig; b += gridDim.x) {
     int s, e;
     cell_range(off, cells, n, big[b], &s, &e);
@@ -309,7 +386,7 @@ void stage_hashgrid(pi_frame* f) {
   f->sidx.alloc(f->ctx, s, n);
   f->u32a.alloc(f->ctx, s, n);
   f->u32b.alloc(f->ctx, s, n);
-  f->u32c.alloc(f->ctx, s, n / kSmallCell + 1);
+  f->u32c.alloc(f->ctx, s, n / kSmallCell + 1);  // a listed cell holds more than kSmallCell
   f->pos.alloc(f->ctx, s, n);
   PI_CUDA(cudaStreamSynchronize(s));
   if (h[6]) throw std::invalid_argument("non-finite particle coordinate");
@@ -333,18 +410,19 @@ void stage_hashgrid(pi_frame* f) {
   g.nx = nn[0], g.ny = nn[1], g.nz = nn[2];
   f->tmp.alloc(f->ctx, s, scan_tmp_ints(g.cellNum + 1));
   f->off.alloc(f->ctx, s, g.cellNum + 1);
-  // misc[7]: particles outside the grid, misc[8]: cells above kSmallCell (both
-  // zeroed by k_init_misc)
+  // misc[7]: particles outside the grid, misc[8], misc[9]: cells above kSmallCell
+  // and kHugeCell (zeroed by k_init_misc)
   int* const big = reinterpret_cast<int*>(f->u32c.p);
+  const long long listed = n / kSmallCell + 1;
   PI_CUDA(cudaMemsetAsync(f->off.p, 0, sizeof(int) * (g.cellNum + 1), s));
   PI_LAUNCH(k_cell_place, div_up(n, 256), 256, 0, s, f->xyz.p, n, g.bounding[0], g.bounding[2], g.bounding[4], cell,
             g.nx, g.ny, g.nz, f->key.p, f->off.p, f->misc.p + 7, f->u32b.p);
   exclusive_scan_i32(f->off.p, f->off.p, g.cellNum + 1, nullptr, f->tmp.p, s);
   PI_LAUNCH(k_cell_scatter, div_up(n, 256), 256, 0, s, f->key.p, f->u32b.p, f->off.p, g.cellNum, n, f->u32a.p);
   PI_LAUNCH(k_cell_sort, div_up(n, 256), 256, 0, s, f->xyz.p, f->key.p, f->u32a.p, f->off.p, g.cellNum, n, f->sidx.p,
-            f->pos.p, big, f->misc.p + 8);
-  PI_LAUNCH(k_cell_sort_big, (int)std::min<long long>(n / kSmallCell, f->ctx->smCount), kBigThreads, 0, s, f->xyz.p,
-            f->u32a.p, f->u32b.p, f->off.p, g.cellNum, n, f->sidx.p, f->pos.p, big, f->misc.p + 8);
+            f->pos.p, big, listed, f->misc.p + 8);
+  PI_LAUNCH(k_cell_sort_big, (int)std::min<long long>(n / kSmallCell, 4ll * f->ctx->smCount), kBigThreads, 0, s,
+            f->xyz.p, f->u32a.p, f->u32b.p, f->off.p, g.cellNum, n, f->sidx.p, f->pos.p, big, listed, f->misc.p + 8);
   // the valid-key count (offset table total) reaches g.nInvalid in
   // resolve_pending; nothing before the end of the call reads it
   f->pin_pending |= 1 << kPinValid;
