@@ -133,20 +133,31 @@ constexpr int kWindowWords = 10240;  // bits of a window's particles, in shared 
 constexpr int kWindows = 32;         // windows at least
 
 // Key, and the particle's place in its cell (cnt: cell counts, zeroed;
-// *outside: particles of key -1).
+// *outside: particles of key -1).  A warp's particles of one cell add their
+// number once: one by one, the additions of 1M particles in one cell took 0.9 ms.
 __global__ void k_cell_place(const float* __restrict__ xyz, long long n, float b0, float b2, float b4, float cell,
                              int nx, int ny, int nz, int* __restrict__ key, int* __restrict__ cnt,
                              unsigned* __restrict__ outside, uint32_t* __restrict__ place) {
   launch_wait();
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  int k = -2;  // a lane past the end
+  if (i < n) {
+    const int cx = (int)__fdiv_rn(__fsub_rn(xyz[3 * i], b0), cell);
+    const int cy = (int)__fdiv_rn(__fsub_rn(xyz[3 * i + 1], b2), cell);
+    const int cz = (int)__fdiv_rn(__fsub_rn(xyz[3 * i + 2], b4), cell);
+    k = -1;
+    if (cx >= 0 && cx < nx && cy >= 0 && cy < ny && cz >= 0 && cz < nz) k = (int)(((long long)cz * ny + cy) * nx + cx);
+  }
+  const unsigned peers = __match_any_sync(0xffffffffu, k);
+  const int lead = __ffs(peers) - 1;
+  int first = 0;
+  if (lane == lead && k >= -1)
+    first = k >= 0 ? atomicAdd(cnt + k, __popc(peers)) : (int)atomicAdd(outside, (unsigned)__popc(peers));
+  first = __shfl_sync(0xffffffffu, first, lead);
   if (i >= n) return;
-  const int cx = (int)__fdiv_rn(__fsub_rn(xyz[3 * i], b0), cell);
-  const int cy = (int)__fdiv_rn(__fsub_rn(xyz[3 * i + 1], b2), cell);
-  const int cz = (int)__fdiv_rn(__fsub_rn(xyz[3 * i + 2], b4), cell);
-  int k = -1;
-  if (cx >= 0 && cx < nx && cy >= 0 && cy < ny && cz >= 0 && cz < nz) k = (int)(((long long)cz * ny + cy) * nx + cx);
   key[i] = k;
-  place[i] = k >= 0 ? (uint32_t)atomicAdd(cnt + k, 1) : atomicAdd(outside, 1u);
+  place[i] = (uint32_t)(first + __popc(peers & ((1u << lane) - 1u)));
 }
 
 // Sorted range of cell k (-1: the particles outside the grid).
