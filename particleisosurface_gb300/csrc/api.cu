@@ -1036,7 +1036,7 @@ int pi_eval_field(pi_frame* f, const float* pts, int64_t m, float* scalar, float
   dv.alloc(f->ctx, s, m);
   if (grad) dg.alloc(f->ctx, s, m * 3);
   PI_CUDA(cudaMemcpyAsync(dp.p, pts, sizeof(float) * 3 * m, cudaMemcpyHostToDevice, s));
-  eval_points(f, dp.p, m, dv.p, grad ? dg.p : nullptr);
+  eval_points(f, pts, dp.p, m, dv.p, grad ? dg.p : nullptr);
   PI_CUDA(cudaMemcpyAsync(scalar, dv.p, sizeof(float) * m, cudaMemcpyDeviceToHost, s));
   if (grad) PI_CUDA(cudaMemcpyAsync(grad, dg.p, sizeof(float) * 3 * m, cudaMemcpyDeviceToHost, s));
   PI_CUDA(cudaStreamSynchronize(s));

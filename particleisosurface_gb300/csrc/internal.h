@@ -343,7 +343,7 @@ std::vector<double> load_hdf5_dataset(const char* path, const char* name, std::v
 std::vector<std::string> load_xdmf(const char* dir, const char* file, int target_frame);
 void write_ply(const char* path, const float* verts, long long nv, const int32_t* tris, long long nt,
                int one_based);
-void eval_points(pi_frame* f, const float* d_pts, long long m, float* d_val, float* d_grad);
+void eval_points(pi_frame* f, const float* h_pts, const float* d_pts, long long m, float* d_val, float* d_grad);
 // FP64 oracle (fp64.cu): per-particle state on demand; values at device
 // points; the state in original particle order into host arrays (each may be
 // null); iso, MaxScalar, Influnce2, Sigma in double.
