@@ -19,9 +19,6 @@
 
 namespace pisurf {
 
-struct NoMem : std::runtime_error {
-  using std::runtime_error::runtime_error;
-};
 struct StateError : std::runtime_error {
   using std::runtime_error::runtime_error;
 };

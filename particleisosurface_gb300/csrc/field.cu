@@ -358,14 +358,11 @@ static bool points_scattered(const pi_frame* f, const float* h, long long m) {
 
 // Whether m points are put in cell order first: from the count where the five
 // launches of the ordering (15 us) are less than the scattered loads they save,
-// while the cells' table is no larger than the points' own arrays, where
-// the context's budget has room for both, and where the points are scattered.
+// while the cells' table is no larger than the points' own arrays, and where the
+// points are scattered.
 static bool order_points(const pi_frame* f, const float* h_pts, long long m) {
   const long long nc = point_cells(f);
   if (m < 16384 || nc > 4 * m || m > 0x7fffffffLL || nc >= 0x7fffffffLL) return false;  // places and cells are ints
-  const pi_ctx* c = f->ctx;
-  const long long need = 4 * (nc + 1) + 12 * m + 4 * (long long)scan_tmp_ints(nc + 1);
-  if (c->budget && c->used.load() + need > (long long)c->budget) return false;
   return points_scattered(f, h_pts, m);
 }
 
@@ -378,12 +375,20 @@ void eval_points(pi_frame* f, const float* h_pts, const float* d_pts, long long 
   const GridView g = gview(f);
   DBuf<int> cnt, order, tmp;
   DBuf<int2> at;
-  if (order_points(f, h_pts, m)) {
-    const long long nc = point_cells(f);
-    cnt.alloc(f->ctx, s, nc + 1);
-    at.alloc(f->ctx, s, m);
-    order.alloc(f->ctx, s, m);
-    tmp.alloc(f->ctx, s, scan_tmp_ints(nc + 1));
+  bool ordered = order_points(f, h_pts, m);
+  const long long nc = point_cells(f);
+  try {
+    if (ordered) {
+      cnt.alloc(f->ctx, s, nc + 1);
+      at.alloc(f->ctx, s, m);
+      order.alloc(f->ctx, s, m);
+      tmp.alloc(f->ctx, s, scan_tmp_ints(nc + 1));
+    }
+  } catch (const NoMem&) {  // the caller's order needs none of them
+    ordered = false;
+    cnt.release(), at.release(), order.release(), tmp.release();
+  }
+  if (ordered) {
     PI_CUDA(cudaMemsetAsync(cnt.p, 0, sizeof(int) * (nc + 1), s));
     PI_LAUNCH(k_point_cell, div_up(m, 256), 256, 0, s, g, d_pts, m, cnt.p, at.p, f->iso, grad_scale(f),
               d_val, d_grad);
@@ -391,8 +396,8 @@ void eval_points(pi_frame* f, const float* h_pts, const float* d_pts, long long 
     PI_LAUNCH(k_point_order, div_up(m, 256), 256, 0, s, at.p, cnt.p, m, order.p);
   }
   // the scan's last entry is the number of points that have a place
-  PI_LAUNCH(k_eval_points, div_up(m, 128), 128, 0, s, g, pview(f), d_pts, order.p, cnt.p ? cnt.p + point_cells(f) : nullptr,
-            m, f->iso, grad_scale(f), d_val, d_grad);
+  PI_LAUNCH(k_eval_points, div_up(m, 128), 128, 0, s, g, pview(f), d_pts, order.p,
+            ordered ? cnt.p + nc : nullptr, m, f->iso, grad_scale(f), d_val, d_grad);
 }
 
 // GetPIdxList: counts, then lists (particle indices through IndexList).

@@ -5,6 +5,7 @@
 #include <atomic>
 #include <cstdint>
 #include <mutex>
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -17,6 +18,11 @@ struct pi_ctx;
 namespace pisurf {
 
 void ctx_account(pi_ctx* c, long long delta);
+
+// No device memory, or none left in the context's budget.
+struct NoMem : std::runtime_error {
+  using std::runtime_error::runtime_error;
+};
 
 // Stream-ordered device buffer (cudaMallocAsync from the device's pool on the
 // context stream), counted against the context budget.

@@ -3,12 +3,15 @@ cell, all beyond the grid's reach on one side or on any, on the last cells that
 still reach the grid, and a few or half of the points among such ones.  Values and gradients are
 those of small calls, which take the points as they come, bit for bit (the sign of
 a zero gradient too)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from particleisosurface_gb300 import _native as N
 from particleisosurface_gb300 import build as B
 from particleisosurface_gb300 import synth
+from test_gpu_kept_eviction import Pool
 
 pytestmark = pytest.mark.gpu
 
@@ -63,3 +66,27 @@ def test_values_are_those_of_small_calls(frame, kind, m):
     assert np.array_equal(val.view(np.uint32), f.eval(p).view(np.uint32))
     if kind not in ("corner", "around"):
         assert (val != np.float32(f.info()["iso_value"])).any()
+
+
+def test_without_device_memory_for_the_ordering(frame):
+    """Scattered points whose own arrays fit the device's memory and the ordering's
+    do not are evaluated as they come."""
+    fr, f = frame
+    m = 16_000_000
+    rng = np.random.default_rng(m)
+    p = (fr.xyz[rng.integers(0, fr.n, 4000)] + rng.normal(0, fr.radius, (4000, 3))).astype(np.float32)
+    want = f.eval(p)
+    p = np.tile(p, (m // 4000, 1))
+    assert np.array_equal(f.eval(p[:40000]), np.tile(want, 10))
+    pool = Pool()
+    assert pool.cu.cuCtxSynchronize() == 0 and pool.cu.cuMemPoolTrimTo(pool.pool, C.c_size_t(0)) == 0
+    free, total = C.c_size_t(), C.c_size_t()
+    assert pool.cu.cuMemGetInfo_v2(C.byref(free), C.byref(total)) == 0
+    block = C.c_uint64()
+    # 16 bytes a point for its coordinates and value, 12 for its place
+    assert pool.cu.cuMemAlloc_v2(C.byref(block), C.c_size_t(free.value - 16 * m - (96 << 20))) == 0
+    try:
+        took = pool.taken_by(lambda: np.testing.assert_array_equal(f.eval(p), np.tile(want, m // 4000)))
+    finally:
+        assert pool.cu.cuMemFree_v2(block) == 0
+    assert 16 * m <= took < 28 * m
