@@ -392,13 +392,17 @@ void stage_hashgrid(pi_frame* f) {
   PI_LAUNCH(k_bbox, blocks, 256, 0, s, f->xyz.p, n, f->misc.p);
   unsigned* const h = reinterpret_cast<unsigned*>(f->ctx->hpin + kPinReadOffset);
   PI_CUDA(cudaMemcpyAsync(h, f->misc.p, sizeof(unsigned) * 8, cudaMemcpyDeviceToHost, s));
-  // the buffers that do not depend on the box, while it is worked out
-  f->key.alloc(f->ctx, s, n);
-  f->sidx.alloc(f->ctx, s, n);
-  f->u32a.alloc(f->ctx, s, n);
-  f->u32b.alloc(f->ctx, s, n);
-  f->u32c.alloc(f->ctx, s, n / kSmallCell + 1);  // a listed cell holds more than kSmallCell
-  f->pos.alloc(f->ctx, s, n);
+  // the buffers that do not depend on the box, while it is worked out (under a
+  // budget after it, which refuses positions that are not finite whatever is left)
+  auto buffers = [&]() {
+    f->key.alloc(f->ctx, s, n);
+    f->sidx.alloc(f->ctx, s, n);
+    f->u32a.alloc(f->ctx, s, n);
+    f->u32b.alloc(f->ctx, s, n);
+    f->u32c.alloc(f->ctx, s, n / kSmallCell + 1);  // a listed cell holds more than kSmallCell
+    f->pos.alloc(f->ctx, s, n);
+  };
+  if (!f->ctx->budget) buffers();
   PI_CUDA(cudaStreamSynchronize(s));
   if (h[6]) throw std::invalid_argument("non-finite particle coordinate");
   float bb[6];
@@ -419,6 +423,7 @@ void stage_hashgrid(pi_frame* f) {
   // FindStartEnd stores keys in an int (src/hash_grid.cpp:105).
   g.cellNum = grid_cell_counts(g.bounding, cell, (1LL << 31) - 2, nn);
   g.nx = nn[0], g.ny = nn[1], g.nz = nn[2];
+  if (f->ctx->budget) buffers();
   f->tmp.alloc(f->ctx, s, scan_tmp_ints(g.cellNum + 1));
   f->off.alloc(f->ctx, s, g.cellNum + 1);
   // misc[7]: particles outside the grid, misc[8], misc[9]: cells above kSmallCell

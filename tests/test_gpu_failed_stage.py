@@ -48,6 +48,24 @@ def test_info_after_two_failed_attempts():
     c.close()
 
 
+@pytest.mark.parametrize("value,code", [(np.nan, N.PI_ERR_INVALID), (np.inf, N.PI_ERR_INVALID), (1e9, N.PI_ERR_LIMIT)])
+def test_refusals_do_not_depend_on_the_memory_left(value, code):
+    """Positions that are not finite, or too far apart for the grid, are refused as
+    such under a budget that the particles alone take."""
+    B.build()
+    fr = synth.small_blob(n=20000, seed=3)
+    xyz = fr.xyz.copy()
+    xyz[7, 1] = value
+    for budget in (12 * fr.n + 4096, 0):
+        c = N.Context(0, budget_bytes=budget)
+        f = N.Frame(c, N.default_params(fr.radius)).upload(xyz)
+        with pytest.raises(N.PiError) as e:
+            f.hashgrid()
+        assert e.value.code == code
+        f.close()
+        c.close()
+
+
 def _state(call):
     with pytest.raises(N.PiError) as e:
         call()
