@@ -1100,7 +1100,6 @@ static_assert(kTopDepth + 5 <= kPinTopWords, "the level starts fit their pinned 
 struct TopArgs {
   LevelArgs la;  // grid, particles, expand, iso
   int D;         // deepest level
-  int spawn;     // k_top_nodes also writes the children of level D's INTERNAL nodes
   float cx, cy, cz, half;  // root
   int size;                // the root's edge in lattice units
   unsigned* flags;         // kTopWords: non-empty paths, a bit each
@@ -1265,24 +1264,6 @@ __global__ void __launch_bounds__(kTopThreads) k_top_nodes(TopArgs t) {
   t.nd_org[at] = org;
   if (d < t.D) return;
   t.rank[at - begin[d]] = rank(d, id);
-  if (!t.spawn || !in) return;
-  const float hc = c.w / 2;
-  const int hs = org.w >> 1;
-  for (int k = 0; k < 8; ++k) {
-    const float4 cc = make_float4(__fadd_rn(c.x, (k & 1) ? hc : -hc), __fadd_rn(c.y, (k & 2) ? hc : -hc),
-                                  __fadd_rn(c.z, (k & 4) ? hc : -hc), hc);
-    t.nd_c[kids + k] = cc;
-    t.nd_v[kids + k] = make_float4(cc.x, cc.y, cc.z, 0.f);
-    t.nd_id[kids + k] = (uint64_t)id * 8ull + (uint64_t)k;
-    t.nd_parent[kids + k] = (int)at;
-    t.nd_child[kids + k] = -1;
-    t.nd_type[kids + k] = T_UNCERTAIN;
-    t.nd_depth[kids + k] = (int8_t)(d + 1);
-    t.nd_sc[kids + k] = 0;
-    t.nd_curv[kids + k] = 0.f;
-    t.nd_org[kids + k] =
-        make_int4(org.x + ((k & 1) ? hs : 0), org.y + ((k & 2) ? hs : 0), org.z + ((k & 4) ? hs : 0), hs);
-  }
 }
 
 __global__ void k_root(float cx, float cy, float cz, float h, int size, float4* nd_c, float4* nd_v,
@@ -1789,11 +1770,10 @@ void stage_octree(pi_frame* f) {
   }
   f->nNodes = 0;
   f->levelBegin.clear();
-  // coarse levels written by k_top_nodes: 0 .. D, and the children of level D
-  // when it is not the last one above D_min
+  // coarse levels written by k_top_nodes: 0 .. D (37449 nodes at most)
   const int D = std::min(f->dmin - 1, kTopDepth);
-  const bool top_spawn = D < f->dmin - 1;
-  ensure_nodes(f, std::max(1 << 16, D >= 0 ? top_base(D + 1 + (top_spawn ? 1 : 0)) : 0));
+  static_assert(top_base(kTopDepth + 1) <= 1 << 16, "room for the coarse levels");
+  ensure_nodes(f, 1 << 16);
   if (!f->ev[kLevelEvent]) PI_CUDA(cudaEventCreateWithFlags(&f->ev[kLevelEvent], cudaEventDisableTiming));
   const GridHost& gh = f->g;
   GridView g{gh.bounding[0], gh.bounding[2], gh.bounding[4], gh.cell, gh.nx, gh.ny, gh.nz, f->off.p};
@@ -1843,7 +1823,6 @@ void stage_octree(pi_frame* f) {
     long long* const lvh = reinterpret_cast<long long*>(ctx->hpin + kPinTopOffset);  // stored by the kernel
     TopArgs ta{LevelArgs{g, f->pos.p, f->nrm.p, f->P.radius * f->P.smooth_factor, f->iso, f->P.radius, 0, 0, 1, P},
                D,
-               top_spawn ? 1 : 0,
                f->rootC[0],
                f->rootC[1],
                f->rootC[2],
@@ -1871,11 +1850,17 @@ void stage_octree(pi_frame* f) {
     lb = lvh[D], le = lvh[D + 1];
     f->nNodes = le;
     const long long newn = 8 * lvh[D + 3];
-    if (newn > 0 && !top_spawn) {
+    if (newn > 0) {
       ensure_nodes(f, le + newn);
-      spawn_scan(LevelArgs{g, f->pos.p, f->nrm.p, f->P.radius * f->P.smooth_factor, f->iso, f->P.radius, lb, le, 1, P},
-                 D, flag.p);
-      known = true;
+      known = D + 1 >= f->dmin;
+      if (known)
+        spawn_scan(
+            LevelArgs{g, f->pos.p, f->nrm.p, f->P.radius * f->P.smooth_factor, f->iso, f->P.radius, lb, le, 1, P}, D,
+            flag.p);
+      else
+        PI_LAUNCH(k_spawn, div_up(le - lb, 256), 256, 0, s, lb, le, le, flag.p, f->nd_type.p, D + 1, f->nd_c.p,
+                  f->nd_v.p, f->nd_id.p, f->nd_parent.p, f->nd_child.p, f->nd_type.p, f->nd_depth.p, f->nd_sc.p,
+                  f->nd_curv.p, f->nd_org.p);
     }
     lb = le;
     le += newn;
