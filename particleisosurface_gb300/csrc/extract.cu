@@ -97,18 +97,26 @@ struct WordBits {
   }
 };
 
-// Interior corners of each leaf, key (x << 2B) | (y << B) | z, B = D_max + 1;
-// boundary corners, and those of nodes that are no leaves, get the all-ones key.
-__global__ void k_corner_keys(const int* __restrict__ nd_child, long long nn, const int4* __restrict__ nd_org,
+// Interior corners of the leaves, key (x << 2B) | (y << B) | z, B = D_max + 1.  A
+// thread per point of a family's 3 x 3 x 3 lattice (27 keys for eight leaves'
+// 64 corners); boundary points, and those that are no leaf's corner, get the
+// all-ones key.
+__global__ void k_corner_keys(const int* __restrict__ nd_child, long long nf, const int4* __restrict__ nd_org,
                               int full, int B, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
   launch_wait();
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nn * 8) return;
-  const int4 o = nd_org[t >> 3];
-  const int k = (int)(t & 7);
-  const int x = o.x + ((k & 1) ? o.w : 0), y = o.y + ((k & 2) ? o.w : 0), z = o.z + ((k & 4) ? o.w : 0);
+  if (t >= nf * 27) return;
+  const long long first = 8 * (t / 27) + 1;  // the family's first node
+  const int p = (int)(t % 27), ix = p % 3, iy = p / 3 % 3, iz = p / 9;
+  const int4 o = nd_org[first];
+  const int x = o.x + ix * o.w, y = o.y + iy * o.w, z = o.z + iz * o.w;
+  bool leaf = false;  // of the children around the point
+  for (int k = 0; k < 8; ++k) {
+    const int dx = ix - (k & 1), dy = iy - ((k >> 1) & 1), dz = iz - (k >> 2);
+    if ((unsigned)dx < 2u && (unsigned)dy < 2u && (unsigned)dz < 2u) leaf = leaf || nd_child[first + k] < 0;
+  }
   uint64_t key;
-  if (nd_child[t >> 3] < 0 && x > 0 && x < full && y > 0 && y < full && z > 0 && z < full)
+  if (leaf && x > 0 && x < full && y > 0 && y < full && z > 0 && z < full)
     key = ((uint64_t)x << (2 * B)) | ((uint64_t)y << B) | (uint64_t)z;
   else
     key = (1ull << (3 * B)) - 1ull;
@@ -786,7 +794,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     PI_LAUNCH(k_bitmap_keys, div_up(nw, 256), 256, 0, s, bits.p, nw, cnt.p, bb, dense ? nullptr : blist.p, B,
               uverts.p);
   } else {
-    const long long nk = nn * 8;
+    const long long nk = nf * 27;
     const uint64_t invalid = (1ull << (3 * B)) - 1ull;
     DBuf<uint64_t> keys, keys2;
     DBuf<uint32_t> vals, vals2;
@@ -794,7 +802,7 @@ static void extract_topology(pi_frame* f, cudaStream_t s, const CountReader& rd)
     keys2.alloc(c, s, nk);
     vals.alloc(c, s, nk);
     vals2.alloc(c, s, nk);
-    PI_LAUNCH(k_corner_keys, div_up(nk, 256), 256, 0, s, f->nd_child.p, nn, f->nd_org.p, full, B, keys.p, vals.p);
+    PI_LAUNCH(k_corner_keys, div_up(nk, 256), 256, 0, s, f->nd_child.p, nf, f->nd_org.p, full, B, keys.p, vals.p);
     DBuf<int> rtmp;
     rtmp.alloc(c, s, radix_tmp_ints(nk));
     uint64_t *kp = keys.p, *ka = keys2.p;
