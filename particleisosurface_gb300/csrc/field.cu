@@ -50,6 +50,13 @@ struct GradSums {
   }
 };
 
+// A normal and its length, whose rounding is written out: the compiler's choice of
+// which product to fuse moved with the code around it, and the lengths' last bits,
+// and the node curvatures', with it.
+__device__ __forceinline__ float4 with_length(float x, float y, float z) {
+  return make_float4(x, y, z, sqrtf(fmaf(z, z, fmaf(y, y, __fmul_rn(x, x)))));
+}
+
 // |d| < R / 2: |A d| < 1 needs it.
 __device__ __forceinline__ bool grad_reach(const float4* xm, float qx, float qy, float qz) {
   const float4 x = __ldg(xm);
@@ -92,7 +99,7 @@ __global__ void __launch_bounds__(128, 12) k_normals(GridView g, PartView P, lon
   grad_sum<L>(g, P, p.x, p.y, p.z, t < n && !splash, sub, sum);
   if (L > 1 && (sub != 0 || t >= n || splash)) return;
   const float gx = sum.x.s * gscale, gy = sum.y.s * gscale, gz = sum.z.s * gscale;
-  nrm[t] = make_float4(gx, gy, gz, sqrtf(gx * gx + gy * gy + gz * gz));
+  nrm[t] = with_length(gx, gy, gz);
 }
 
 // field_sum and grad_sum at q in one walk: both need u = A_j d of the same
@@ -259,7 +266,7 @@ __global__ void __launch_bounds__(128) k_vr_normals(const MultiGridView* __restr
   grad_sum_vr<L>(*mg, P, p.x, p.y, p.z, t < n, sub, sum);
   if (L > 1 && (sub != 0 || t >= n)) return;
   const float gx = sum.x.s, gy = sum.y.s, gz = sum.z.s;
-  nrm[t] = make_float4(gx, gy, gz, sqrtf(gx * gx + gy * gy + gz * gz));
+  nrm[t] = with_length(gx, gy, gz);
 }
 
 __global__ void k_vr_eval_points(const MultiGridView* __restrict__ mg, PartView P, const float* __restrict__ pts,
