@@ -3,11 +3,11 @@
 // :465-512), pass 2 weighted covariance of neighbour centres and its
 // eigen-decomposition into the anisotropy matrix G (compute_G_Yus, :585-654).
 //
-// One thread per particle in cell order, so a warp's particles share most of
-// their 27-cell candidates and the candidate loads hit L1.  Distances that
-// decide neighbour membership (d^2 < (4r)^2) are rounded exactly as the
-// reference rounds them (no fused multiply-add, x0 + (x1 + x2) order), so the
-// neighbour sets match; the sums are compensated FP32.
+// One thread per particle in cell order (four on small frames, particle_lanes),
+// so a warp's particles share most of their 27-cell candidates and the candidate
+// loads hit L1.  Distances that decide neighbour membership (d^2 < (4r)^2) are
+// rounded exactly as the reference rounds them (no fused multiply-add, x0 + (x1
+// + x2) order), so the neighbour sets match; the sums are compensated FP32.
 //
 // The covariance is symmetric positive definite (Influnce2 * I is added), so
 // the reference's JacobiSVD has U = V and G = V diag(s / w) V^T is a spectral

@@ -37,7 +37,6 @@ struct CudaError : std::runtime_error {
     }                                                                                   \
   } while (0)
 
-// Launch wrapper: counts the launch and checks the launch error.
 // Programmatic stream serialization: a kernel is brought up while the one before
 // it on the stream drains, and every kernel begins with launch_wait(), where it
 // waits until that one is complete and its writes are visible, before it touches
@@ -64,6 +63,7 @@ inline void launch_kernel(void (*kernel)(KA...), dim3 grid, dim3 block, size_t s
   PI_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KA>(std::forward<A>(args))...));
 }
 
+// Launch wrapper: counts the launch and checks the launch error.
 #define PI_LAUNCH(kernel, grid, block, smem, stream, ...)                              \
   do {                                                                                 \
     if ((grid) > 0) {                                                                  \
@@ -142,7 +142,5 @@ void radix_sort_u32(uint32_t** keys, uint32_t** vals, uint32_t** keys_alt, uint3
 void radix_sort_u64(uint64_t** keys, uint32_t** vals, uint64_t** keys_alt, uint32_t** vals_alt,
                     long long n, int bits, int* tmp, cudaStream_t s);
 
-// iota: v[i] = i
-void iota_u32(uint32_t* v, long long n, cudaStream_t s);
 
 }  // namespace pisurf

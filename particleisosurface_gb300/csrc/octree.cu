@@ -1975,23 +1975,23 @@ void stage_octree(pi_frame* f) {
           qef_level(f, lb, le, depth, parts, p);
         }
       } else {
-      const int pg = dense ? PG_CHUNK : PG_THREAD;
-      prof_begin(ctx, s, pg);
-      if (dense)
-        dense_eval(f, cfg, qa, qn, nb, order.p, qcnt.p, ucnt, chunks.p, qcnt.p + nb + 1, 0, qval.p, f->dcount.p);
-      else
-        PI_LAUNCH(k_q_eval_thread, (int)std::min<long long>((long long)ctx->smCount * 8, div_up(qn, kEvalThreads)),
-                  kEvalThreads, 0, s, qa, list, ucum.p + nb, qcnt.p + nb + 2, f->nd_c.p, f->nd_v.p, qval.p, f->dcount.p);
-      prof_end(ctx, s, pg);
-      if (known || leaf_level)  // no node needs a particle scan
-        PI_LAUNCH(k_classify_thread, div_up(nl, kClassifyNodes), kClassifyThreads, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
-                  f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p, (const int*)nullptr,
-                  (const int*)nullptr, 0, 0);
-      else
-        PI_LAUNCH(k_classify, div_up(nl, wpb), 32 * wpb, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
-                  f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, known ? 1 : 0, f->dcount.p,
-                  (const float*)nullptr);
-      if (f->P.qef) qef_level(f, lb, le, depth);
+        const int pg = dense ? PG_CHUNK : PG_THREAD;
+        prof_begin(ctx, s, pg);
+        if (dense)
+          dense_eval(f, cfg, qa, qn, nb, order.p, qcnt.p, ucnt, chunks.p, qcnt.p + nb + 1, 0, qval.p, f->dcount.p);
+        else
+          PI_LAUNCH(k_q_eval_thread, (int)std::min<long long>((long long)ctx->smCount * 8, div_up(qn, kEvalThreads)),
+                    kEvalThreads, 0, s, qa, list, ucum.p + nb, qcnt.p + nb + 2, f->nd_c.p, f->nd_v.p, qval.p, f->dcount.p);
+        prof_end(ctx, s, pg);
+        if (known || leaf_level)  // no node needs a particle scan
+          PI_LAUNCH(k_classify_thread, div_up(nl, kClassifyNodes), kClassifyThreads, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
+                    f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, f->dcount.p, (const int*)nullptr,
+                    (const int*)nullptr, 0, 0);
+        else
+          PI_LAUNCH(k_classify, div_up(nl, wpb), 32 * wpb, 0, s, la, qval.p, rep.p, f->nd_c.p, f->nd_v.p,
+                    f->nd_type.p, f->nd_sc.p, f->nd_curv.p, f->nd_samp.p, f->P.qef, 0, f->dcount.p,
+                    (const float*)nullptr);
+        if (f->P.qef) qef_level(f, lb, le, depth);
       }
     }
     if (last) {

@@ -578,39 +578,39 @@ __global__ void __launch_bounds__(128) k_qef_accept(QefArgs a, const int* __rest
     const int entry = lane < 8 && t0 + lane < count ? list[t0 + lane] : 0;
     unsigned todo = __ballot_sync(0xffffffffu, entry < 0);
     for (; todo; todo &= todo - 1u) {
-    const long long node = a.lb + (__shfl_sync(0xffffffffu, entry, __ffs(todo) - 1) & ~kAccepted);
-    const float4 c = nd_c[node];
-    float4 v = nd_v[node];
-    const float h = c.w;
-    const float cellsize = 2.0f * h;
-    const float step = cellsize / 2;
-    float term = 0.f;
-    {
-      const int i = min(lane, 26);
-      const float mn[3] = {__fsub_rn(c.x, h), __fsub_rn(c.y, h), __fsub_rn(c.z, h)};
-      const float mx[3] = {__fadd_rn(c.x, h), __fadd_rn(c.y, h), __fadd_rn(c.z, h)};
-      const float* sv = nd_samp + node * 27;
-      const int x = i % 3, y = (i / 3) % 3, z = i / 9;
-      const float px = __fadd_rn(__fmul_rn(1.0f - x * 0.5f, mn[0]), __fmul_rn(x * 0.5f, mx[0]));
-      const float py = __fadd_rn(__fmul_rn(1.0f - y * 0.5f, mn[1]), __fmul_rn(y * 0.5f, mx[1]));
-      const float pz = __fadd_rn(__fmul_rn(1.0f - z * 0.5f, mn[2]), __fmul_rn(z * 0.5f, mx[2]));
-      auto fdf = [&](int d, int stride) {
-        if (d == 0) return (sv[i] - sv[i + stride]) / step;
-        if (d == 2) return (sv[i - stride] - sv[i]) / step;
-        return (sv[i - stride] - sv[i + stride]) / (step * 2);
-      };
-      const float gx = fdf(x, 1), gy = fdf(y, 3), gz = fdf(z, 9);
-      const float d = gx * (v.x - px) + gy * (v.y - py) + gz * (v.z - pz) - v.w;
-      term = d * d / (1.0f + gx * gx + gy * gy + gz * gz);
-    }
-    float err = 0.0f;
-    for (int i = 0; i < 27; ++i) err = __fadd_rn(err, __shfl_sync(0xffffffffu, term, i));
-    v.w = a.iso - field_sum_warp(a.g, a.P, v.x, v.y, v.z);
-    // leaf by size keeps the zeroing (no SingleEval follows it)
-    const bool leaf_by_size = cellsize - a.radius < kAbove1em8;
-    if (leaf_by_size && err / cellsize < 0.0001f) v.w = 0.0f;
-    if (lane == 0) nd_v[node] = v;
-    ++done;
+      const long long node = a.lb + (__shfl_sync(0xffffffffu, entry, __ffs(todo) - 1) & ~kAccepted);
+      const float4 c = nd_c[node];
+      float4 v = nd_v[node];
+      const float h = c.w;
+      const float cellsize = 2.0f * h;
+      const float step = cellsize / 2;
+      float term = 0.f;
+      {
+        const int i = min(lane, 26);
+        const float mn[3] = {__fsub_rn(c.x, h), __fsub_rn(c.y, h), __fsub_rn(c.z, h)};
+        const float mx[3] = {__fadd_rn(c.x, h), __fadd_rn(c.y, h), __fadd_rn(c.z, h)};
+        const float* sv = nd_samp + node * 27;
+        const int x = i % 3, y = (i / 3) % 3, z = i / 9;
+        const float px = __fadd_rn(__fmul_rn(1.0f - x * 0.5f, mn[0]), __fmul_rn(x * 0.5f, mx[0]));
+        const float py = __fadd_rn(__fmul_rn(1.0f - y * 0.5f, mn[1]), __fmul_rn(y * 0.5f, mx[1]));
+        const float pz = __fadd_rn(__fmul_rn(1.0f - z * 0.5f, mn[2]), __fmul_rn(z * 0.5f, mx[2]));
+        auto fdf = [&](int d, int stride) {
+          if (d == 0) return (sv[i] - sv[i + stride]) / step;
+          if (d == 2) return (sv[i - stride] - sv[i]) / step;
+          return (sv[i - stride] - sv[i + stride]) / (step * 2);
+        };
+        const float gx = fdf(x, 1), gy = fdf(y, 3), gz = fdf(z, 9);
+        const float d = gx * (v.x - px) + gy * (v.y - py) + gz * (v.z - pz) - v.w;
+        term = d * d / (1.0f + gx * gx + gy * gy + gz * gz);
+      }
+      float err = 0.0f;
+      for (int i = 0; i < 27; ++i) err = __fadd_rn(err, __shfl_sync(0xffffffffu, term, i));
+      v.w = a.iso - field_sum_warp(a.g, a.P, v.x, v.y, v.z);
+      // leaf by size keeps the zeroing (no SingleEval follows it)
+      const bool leaf_by_size = cellsize - a.radius < kAbove1em8;
+      if (leaf_by_size && err / cellsize < 0.0001f) v.w = 0.0f;
+      if (lane == 0) nd_v[node] = v;
+      ++done;
     }
   }
   if (lane == 0) {

@@ -1,9 +1,10 @@
 // Exclusive scan and stable LSD radix sort.
 //
-// Used to order particles into hash cells (a stable sort by cell key keeps
-// particle-index order inside a cell), to build the dense cell offset table,
-// to compact octree frontiers and to deduplicate dual-grid vertices, mesh
-// vertices and triangles.
+// The scan builds the cell offset tables, ranks the octree's INTERNAL nodes and
+// numbers the extraction's vertices and triangles.  The radix sort orders
+// particles by (grid, cell) where radii differ and in the build that allocates
+// nothing (grid.cu's counting sort does the others), and the leaves' corners
+// above D_max 14.
 //
 // Scan: scan.cuh.
 // Radix sort: 8-bit digits; per pass a per-tile digit histogram, an exclusive
@@ -119,15 +120,6 @@ void radix_sort_u32(uint32_t** keys, uint32_t** vals, uint32_t** kalt, uint32_t*
 void radix_sort_u64(uint64_t** keys, uint32_t** vals, uint64_t** kalt, uint32_t** valt, long long n,
                     int bits, int* tmp, cudaStream_t s) {
   radix_sort<uint64_t>(keys, vals, kalt, valt, n, bits, tmp, s);
-}
-
-__global__ void k_iota(uint32_t* v, long long n) {
-  launch_wait();
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) v[i] = (uint32_t)i;
-}
-void iota_u32(uint32_t* v, long long n, cudaStream_t s) {
-  PI_LAUNCH(k_iota, div_up(n, 256), 256, 0, s, v, n);
 }
 
 }  // namespace pisurf
