@@ -31,7 +31,8 @@ extern "C" {
 #define PI_ERR_CUDA (-2)    /* CUDA runtime error (message in pi_last_error) */
 #define PI_ERR_NOMEM (-3)   /* device memory budget of the context exceeded */
 #define PI_ERR_STATE (-4)   /* stage called before the stages it depends on */
-#define PI_ERR_LIMIT (-5)   /* size limit: >= 2^31 hash cells, octree depth > 20, ... */
+#define PI_ERR_LIMIT (-5)   /* size limit: >= 2^31 hash cells (grown by 2 on each side, for the octree), octree depth > 20,
+                               an octree level of more than 76M sampled nodes, ... */
 
 typedef struct pi_ctx pi_ctx;
 typedef struct pi_frame pi_frame;
