@@ -77,6 +77,9 @@ static void upload_tables(int device) {
   }
   PI_CUDA(cudaMemcpyToSymbol(d_case, cs, sizeof(cs)));
   PI_CUDA(cudaMemcpyToSymbol(d_edges, edges, sizeof(edges)));
+  // a copy from pageable memory may return before it has arrived, and the contexts'
+  // streams do not wait for the default one
+  PI_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
   if (device >= 0 && device < 128) done[device] = true;
 }
 
